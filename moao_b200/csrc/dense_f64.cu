@@ -380,18 +380,12 @@ moao_status launch_gemm(const KParams& p, int cfg, cudaStream_t s) {
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Leaf kernel of the blocked factorisation (leaf_factor_inverse, one CTA).
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 1) potrf_inv_leaf_kernel(double* A, long lda,
-                                                                    double* Linv, long ldi, int n,
-                                                                    long col0, int* info) {
+__global__ void __launch_bounds__(LEAF_THREADS, 1)
+    potrf_inv_leaf_kernel(double* A, long lda, double* Linv, long ldi, int n, long col0,
+                          int* info) {
   extern __shared__ __align__(16) double leaf_smem[];
-  leaf_factor_inverse<THREADS>(A, lda, Linv, ldi, n, col0, info, leaf_smem);
+  leaf_factor_inverse(A, lda, Linv, ldi, n, col0, info, leaf_smem);
 }
-
-// The leaf CTA has 1,024 threads (two or three triangle elements each): 54 us
-// per 64 x 64 block against 66 us with 512 and 91 us with 256 threads (B200,
-// CUDA events over the leaves of an nmeas 15,936 FP64 build).
-constexpr int kLeafThreads = 1024;
 
 __global__ void copy_kernel(const double* __restrict__ src, long lds, double* __restrict__ dst,
                             long ldd, long m, long n) {
@@ -467,9 +461,8 @@ moao_status potrf_inv_leaf(double* A, long lda, double* Linv, long ldi, int n, l
   if (n > LEAF) return set_error(MOAO_ERR_BAD_ARG, "potrf leaf: n > 64");
   static std::atomic<unsigned long long> configured{0};
   const int smem = LEAF_SMEM_BYTES;
-  MOAO_CUDA_TRY(set_smem_limit(potrf_inv_leaf_kernel<kLeafThreads>, smem, configured));
-  potrf_inv_leaf_kernel<kLeafThreads><<<1, kLeafThreads, smem, s>>>(A, lda, Linv, ldi, n, col0,
-                                                                    d_info);
+  MOAO_CUDA_TRY(set_smem_limit(potrf_inv_leaf_kernel, smem, configured));
+  potrf_inv_leaf_kernel<<<1, LEAF_THREADS, smem, s>>>(A, lda, Linv, ldi, n, col0, d_info);
   if (launches) ++*launches;
   MOAO_CUDA_TRY(cudaGetLastError());
   return MOAO_OK;

@@ -55,6 +55,7 @@ namespace {
 constexpr int T = 64;               // tile edge
 constexpr int TLD = T + 4;          // shared-memory leading dimension (conflict-free fragments)
 constexpr int NTHREADS = 256;       // 8 warps: 4 along m (16 rows) x 2 along n (32 columns)
+static_assert(NTHREADS == LEAF_THREADS, "the leaf runs on the whole CTA");
 constexpr int TILE_SMEM = T * TLD * 8;
 // P, Q and (for an update) the old value of the tile written: 102 KB, two CTAs per SM
 constexpr int SMEM_BYTES = 3 * TILE_SMEM > LEAF_SMEM_BYTES ? 3 * TILE_SMEM : LEAF_SMEM_BYTES;
@@ -293,7 +294,7 @@ __global__ void __launch_bounds__(NTHREADS, 2)
     if (stop) break;
     switch (type) {
       case kPotrf:
-        leaf_factor_inverse<NTHREADS>(At(k, k), I.lda, I.Linv + (size_t)k * T * T, T, tn(k), (long)k * T,
+        leaf_factor_inverse(At(k, k), I.lda, I.Linv + (size_t)k * T * T, T, tn(k), (long)k * T,
                             I.info, smem);
         break;
       case kTrsm:

@@ -41,6 +41,15 @@ moao_status moao_debug_residual(moao_ctx* ctx, int scheme, long m, long n, const
  * sums, and the slice products run instead). Host only. */
 int moao_debug_crt_moduli(int ns, long K);
 
+/* An FP64 product by int8 residue products (device pointers, context stream),
+ * whatever its size: form 0: C = alpha A B^T + beta C (A M x K, B N x K; lower = 1
+ * writes only C(r, c) with r >= c, M = N), form 1: C = alpha A B + beta C (B K x N),
+ * form 2: C = A S with S the symmetric K x K matrix in B's lower triangle (N = K,
+ * alpha and beta not used). All column-major; K < 131,072. */
+moao_status moao_debug_crt64(moao_ctx* ctx, int form, int lower, long M, long N, long K,
+                             double alpha, const double* A, long lda, const double* B, long ldb,
+                             double beta, double* C, long ldc);
+
 #ifdef __cplusplus
 }
 #endif

@@ -66,6 +66,10 @@ struct moao_ctx {
   moao::DevBuf mx_rid, mx_y, mx_y2, mx_zu, mx_sinv, mx_exps, mx_dsl;
   // mixed Cee/Cvv chain: int8 slices of Ctm's rows (then of E's), their exponents
   moao::DevBuf cx_qc, cx_ec;
+  // FP64 products by residues (crt_f64.cu): operands' residues and row maxima,
+  // the product's residues, the guard flags
+  moao::DevBuf cf_a, cf_b, cf_ma, cf_mb, cf_k, cf_z, cf_flag;
+  bool crt_f64 = true;  // off where nothing may be allocated (stream capture, no-alloc calls)
   long mx_factored_n = -1;  // size of the factorisation held in mx_* (reuse across targets)
   // Block-constant offsets of Cmm known to the caller (moao_ctx_set_offsets):
   // the mixed path factors Cmm minus them and adds them back exactly.
@@ -138,7 +142,7 @@ struct moao_ctx {
     return {&ws_w,  &ws_dinv, &ws_info, &ws_tmp, &ws_host_t, &ws_corner, &mx_a32, &mx_lr,  &mx_lc,    &mx_t32,
             &mx_w1, &mx_w2,   &mx_x,    &mx_r64, &mx_e64, &mx_qa,  &mx_qb,    &mx_ea,
             &mx_fb, &mx_colmax, &mx_norm, &mx_rid, &mx_y, &mx_y2, &mx_zu, &mx_sinv, &mx_exps,
-            &mx_dsl, &cx_qc, &cx_ec};
+            &mx_dsl, &cx_qc, &cx_ec, &cf_a, &cf_b, &cf_ma, &cf_mb, &cf_k, &cf_z, &cf_flag};
   }
   // Device bytes held by the workspaces and the geometry caches.
   size_t bytes_held() {

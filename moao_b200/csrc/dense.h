@@ -21,6 +21,7 @@ struct GemmArgs {
   long ldb = 0;
   bool transB = false;
   TriMode triB = TRI_FULL;
+  long tri_off = 0;           // column index of B's first column (triB != TRI_FULL)
   double* C = nullptr;        // M x N, column-major, ldc
   long ldc = 0;
   bool lowerC = false;        // write only C(i, j) with i >= j (SYRK / SYR2K)
@@ -32,6 +33,11 @@ constexpr int kGemmConfigs = 4;
 
 // C = alpha * A * op(B) + beta * C in FP64 on the DMMA tensor-core path.
 moao_status gemm_f64(const GemmArgs& g, cudaStream_t s, long long* launches);
+
+// The same product on the tiles [tile0, tile0 + tiles) of a 128 x 256-tile walk
+// over C (tile_walk.cuh), only when *flag_a or *flag_b (device) is nonzero.
+moao_status gemm_f64_guarded(const GemmArgs& g, long tile0, long tiles, const int* flag_a,
+                             const int* flag_b, cudaStream_t s, long long* launches);
 
 // Factor the n x n (n <= 64) diagonal block A (lower triangle read) in place:
 // A <- L (lower; the upper triangle is left untouched) and Linv <- L^-1 (lower,

@@ -17,6 +17,7 @@
 
 #include "dense.h"
 #include "leaf_f64.cuh"
+#include "tile_walk.cuh"
 
 namespace moao {
 namespace {
@@ -99,6 +100,7 @@ struct KParams {
   double* C;
   long ldc;
   int triB;
+  long tri_off;
   // tile order (set by the launcher): bands of group_m row tiles; inside a band
   // the column tiles in turn, the band's row tiles fastest
   int tiles_m, tiles_n, group_m;
@@ -162,25 +164,22 @@ __device__ __forceinline__ void load_k_tile(double* s, const double* g, long ld,
   }
 }
 
+// The tile of C at (m0, n0), by all threads of the CTA.
 template <class TL, bool TRANSB, bool LOWERC, int VEC, bool MMA16>
-__global__ void __launch_bounds__(TL::NTHREADS) gemm_f64_kernel(const KParams p) {
+__device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const long m0,
+                                          const long n0) {
   constexpr int BM = TL::BM, BN = TL::BN, NTHREADS = TL::NTHREADS, MF = TL::MF;
   constexpr int BK = TL::BK, STAGES = TL::STAGES;
   constexpr int LDA_S = TL::LDA_S, LDB_S = TL::LDB_S, LDBT_S = TL::LDBT_S;
   constexpr int A_STAGE = TL::A_STAGE, B_STAGE = TL::B_STAGE;
-  extern __shared__ __align__(16) double smem[];
   double* As = smem;
   double* Bs = smem + STAGES * A_STAGE;
-
-  long m0 = 0, n0 = 0;
-  if (!band_tile<BM, BN, LOWERC>(p, blockIdx.x, &m0, &n0)) return;
-  if (LOWERC && m0 + BM <= n0) return;  // tile strictly above the diagonal
 
   // K range (tile aligned); a triangular B limits it.
   long kb = 0, ke = p.K;
   if (p.triB != 0) {
-    if (!TRANSB) kb = n0;                      // B(k, n) with k >= n
-    else ke = min(p.K, n0 + BN);               // B(n, k) with n >= k
+    if (!TRANSB) kb = n0 + p.tri_off;          // B(k, n) with k >= n
+    else ke = min(p.K, n0 + p.tri_off + BN);   // B(n, k) with n >= k
   }
   kb = (kb / BK) * BK;
   const int ntiles = (ke > kb) ? (int)((ke - kb + BK - 1) / BK) : 0;
@@ -221,11 +220,12 @@ __global__ void __launch_bounds__(TL::NTHREADS) gemm_f64_kernel(const KParams p)
       // Zero the entries of the stored B outside its lower (or strictly lower)
       // triangle when this slice crosses the diagonal.
       const long k0 = kb + (long)t * BK;
-      const bool crosses = TRANSB ? (k0 + BK - 1 >= n0) : (k0 <= n0 + BN - 1);
+      const long d0 = n0 + p.tri_off;
+      const bool crosses = TRANSB ? (k0 + BK - 1 >= d0) : (k0 <= d0 + BN - 1);
       if (crosses) {
         for (int e = threadIdx.x; e < BK * BN; e += NTHREADS) {
           const int kk = e / BN, nn = e % BN;
-          const long gk = k0 + kk, gn = n0 + nn;
+          const long gk = k0 + kk, gn = d0 + nn;
           // stored row / column of this element
           const long row = TRANSB ? gn : gk, col = TRANSB ? gk : gn;
           const bool keep = (p.triB == 1) ? (row >= col) : (row > col);
@@ -323,6 +323,35 @@ __global__ void __launch_bounds__(TL::NTHREADS) gemm_f64_kernel(const KParams p)
   }
 }
 
+template <class TL, bool TRANSB, bool LOWERC, int VEC, bool MMA16>
+__global__ void __launch_bounds__(TL::NTHREADS) gemm_f64_kernel(const KParams p) {
+  extern __shared__ __align__(16) double smem[];
+  long m0 = 0, n0 = 0;
+  if (!band_tile<TL::BM, TL::BN, LOWERC>(p, blockIdx.x, &m0, &n0)) return;
+  if (LOWERC && m0 + TL::BM <= n0) return;  // tile strictly above the diagonal
+  gemm_tile<TL, TRANSB, LOWERC, VEC, MMA16>(p, smem, m0, n0);
+}
+
+// The tiles [tile0, tile0 + tiles) of a tensor-core product's walk over C, when
+// one of its two guard flags is raised; otherwise the few CTAs leave at once.
+template <class TL, bool TRANSB, bool LOWERC, int VEC>
+__global__ void __launch_bounds__(TL::NTHREADS)
+    gemm_f64_guard_kernel(const KParams p, const __grid_constant__ TileWalk walk, int tile0,
+                          int tiles, const int* flag_a, const int* flag_b) {
+  extern __shared__ __align__(16) double smem[];
+  if (*flag_a == 0 && *flag_b == 0) return;
+  constexpr int PER = kWalkTileN / TL::BN;  // columns of this kernel's tiles in one of the walk's
+  static_assert(TL::BM == 128, "the walk's tiles are 128 rows");
+  for (int v = blockIdx.x; v < tiles * PER; v += gridDim.x) {
+    int mt, nt;
+    decode_tile(walk, tile0 + v / PER, &mt, &nt);
+    const long m0 = (long)mt * TL::BM, n0 = (long)nt * kWalkTileN + (v % PER) * TL::BN;
+    if (m0 >= p.M || n0 >= p.N || (LOWERC && m0 + TL::BM <= n0)) continue;
+    gemm_tile<TL, TRANSB, LOWERC, VEC, true>(p, smem, m0, n0);
+    __syncthreads();  // the C tile in shared memory is stored before the next ring fill
+  }
+}
+
 // FP64 MMA shape: m16n8k16 unless MOAO_GEMM_MMA=k4 selects m8n8k4.
 bool use_mma16() {
   static const bool v = [] {
@@ -375,6 +404,25 @@ moao_status launch_gemm(const KParams& p, int cfg, cudaStream_t s) {
   }
   return use_mma16() ? launch_gemm_t<TileL, TRANSB, LOWERC, VEC, true>(p, s)
                      : launch_gemm_t<TileL, TRANSB, LOWERC, VEC, false>(p, s);
+}
+
+KParams params_of(const GemmArgs& g) {
+  KParams p{g.M, g.N, g.K, g.alpha, g.beta, g.A, g.lda, g.B, g.ldb, g.C, g.ldc, (int)g.triB,
+            g.tri_off};
+  if (g.K == 0) p.alpha = 0.0;  // C = beta C
+  return p;
+}
+
+template <bool TRANSB, bool LOWERC, int VEC>
+moao_status launch_guard(const KParams& p, const TileWalk& w, long tile0, long tiles,
+                         const int* flag_a, const int* flag_b, cudaStream_t s) {
+  using TL = TileL32x2;
+  static std::atomic<unsigned long long> configured{0};
+  auto kern = gemm_f64_guard_kernel<TL, TRANSB, LOWERC, VEC>;
+  MOAO_CUDA_TRY(set_smem_limit(kern, (int)TL::SMEM_BYTES, configured));
+  kern<<<2 * 148, TL::NTHREADS, TL::SMEM_BYTES, s>>>(p, w, (int)tile0, (int)tiles, flag_a, flag_b);
+  MOAO_CUDA_TRY(cudaGetLastError());
+  return MOAO_OK;
 }
 
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -437,10 +485,7 @@ moao_status gemm_f64(const GemmArgs& g, cudaStream_t s, long long* launches) {
   if (g.lda < std::max(1L, g.M) || g.ldc < std::max(1L, g.M) ||
       g.ldb < std::max(1L, g.transB ? g.N : g.K))
     return set_error(MOAO_ERR_BAD_ARG, "gemm: leading dimension too small");
-  KParams p{g.M, g.N, g.K, g.alpha, g.beta, g.A, g.lda, g.B, g.ldb, g.C, g.ldc, (int)g.triB};
-  if (g.K == 0) {  // C = beta C
-    p.alpha = 0.0;
-  }
+  KParams p = params_of(g);
   const bool v2 = aligned16(g.A) && aligned16(g.B) && (g.lda % 2 == 0) && (g.ldb % 2 == 0);
   moao_status st;
   const int c = g.cfg;
@@ -450,6 +495,29 @@ moao_status gemm_f64(const GemmArgs& g, cudaStream_t s, long long* launches) {
   } else {
     if (g.transB) st = g.lowerC ? launch_gemm<true, true, 1>(p, c, s) : launch_gemm<true, false, 1>(p, c, s);
     else st = g.lowerC ? launch_gemm<false, true, 1>(p, c, s) : launch_gemm<false, false, 1>(p, c, s);
+  }
+  if (st == MOAO_OK && launches) ++*launches;
+  return st;
+}
+
+moao_status gemm_f64_guarded(const GemmArgs& g, long tile0, long tiles, const int* flag_a,
+                             const int* flag_b, cudaStream_t s, long long* launches) {
+  if (g.M <= 0 || g.N <= 0 || tiles <= 0) return MOAO_OK;
+  TileWalk w{};
+  fill_walk(&w, g.M, g.N, g.lowerC ? 1 : 0, 0, 128);
+  const KParams p = params_of(g);
+  const bool v2 = aligned16(g.A) && aligned16(g.B) && (g.lda % 2 == 0) && (g.ldb % 2 == 0);
+  moao_status st;
+  if (g.lowerC) {
+    if (!g.transB) return set_error(MOAO_ERR_UNSUPPORTED, "guarded gemm: lower C without a transposed B");
+    st = v2 ? launch_guard<true, true, 2>(p, w, tile0, tiles, flag_a, flag_b, s)
+            : launch_guard<true, true, 1>(p, w, tile0, tiles, flag_a, flag_b, s);
+  } else if (g.transB) {
+    st = v2 ? launch_guard<true, false, 2>(p, w, tile0, tiles, flag_a, flag_b, s)
+            : launch_guard<true, false, 1>(p, w, tile0, tiles, flag_a, flag_b, s);
+  } else {
+    st = v2 ? launch_guard<false, false, 2>(p, w, tile0, tiles, flag_a, flag_b, s)
+            : launch_guard<false, false, 1>(p, w, tile0, tiles, flag_a, flag_b, s);
   }
   if (st == MOAO_OK && launches) ++*launches;
   return st;

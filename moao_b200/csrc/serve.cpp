@@ -37,6 +37,7 @@
 #include <vector>
 
 #include "context.h"
+#include "crt_f64.h"
 #include "moao_b200.h"
 
 namespace moao {
@@ -122,6 +123,7 @@ size_t footprint(const moao_server* s, const System& sys, const moao_request& r)
     f += 2 * bytes_of(n, nb);
   }
   const bool cvv = (r.Cvv || r.psf) && a > 0;
+  if (r.prec != MOAO_PREC_MIXED) f += crt64_bytes(n, m, nb, cvv ? a : 0);
   if (cvv) f += 2 * bytes_of(m, m) + bytes_of(a, a) + 3 * bytes_of(a, m) + bytes_of(m, n);
   if (r.psf && sys.has_psf)
     f += bytes_of(sys.psf_n, sys.psf_n) * 7 + sizeof(int) * 2 * (size_t)sys.idx.size();

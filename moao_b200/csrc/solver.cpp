@@ -12,6 +12,7 @@
 #include <cstring>
 
 #include "context.h"
+#include "crt_f64.h"
 #include "dense.h"
 
 namespace moao {
@@ -32,6 +33,33 @@ moao_status gemm(moao_ctx* ctx, long M, long N, long K, double alpha, const doub
   if (tri != TRI_FULL) fl *= 0.5;
   KernelTimer kt(ctx, "gemm_f64", fl);
   return gemm_f64(g, ctx->stream, &ctx->launches);
+}
+
+// The same product by int8 residue products where those are faster (crt_f64.cu);
+// the FP64 tensor cores where not, or where their buffers do not fit.
+moao_status gemm_long(moao_ctx* ctx, long M, long N, long K, double alpha, const double* A,
+                      long lda, const double* B, long ldb, bool transB, double beta, double* C,
+                      long ldc, bool lowerC = false, const CrtBalance* bal = nullptr) {
+  if (crt64_pays(ctx, M, N, K, lowerC)) {
+    GemmArgs g;
+    g.M = M; g.N = N; g.K = K; g.alpha = alpha; g.beta = beta;
+    g.A = A; g.lda = lda; g.B = B; g.ldb = ldb; g.transB = transB;
+    g.C = C; g.ldc = ldc; g.lowerC = lowerC;
+    const moao_status st = crt64_gemm(ctx, g, bal);
+    if (st != MOAO_ERR_OOM) return st;
+  }
+  return gemm(ctx, M, N, K, alpha, A, lda, B, ldb, transB, beta, C, ldc, lowerC);
+}
+
+// C (M x n) = A (M x n) S, S the symmetric n x n matrix in the lower triangle of B.
+moao_status symm_right(moao_ctx* ctx, long M, long n, const double* A, long lda, const double* B,
+                       long ldb, double* C, long ldc) {
+  if (crt64_pays(ctx, M, n, n, false)) {
+    const moao_status st = crt64_symm(ctx, M, n, A, lda, B, ldb, C, ldc);
+    if (st != MOAO_ERR_OOM) return st;
+  }
+  MOAO_TRY(gemm(ctx, M, n, n, 1.0, A, lda, B, ldb, false, 0.0, C, ldc, false, TRI_LOWER));
+  return gemm(ctx, M, n, n, 1.0, A, lda, B, ldb, true, 1.0, C, ldc, false, TRI_STRICT_LOWER);
 }
 
 // Factor the nb x nb diagonal block A (lda) and write its inverse into D (ldd).
@@ -77,11 +105,13 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
     if (rest <= 0) break;
     double* P = A + (k0 + kb) + k0 * lda;
     // panel: P <- P L_kk^-T
-    MOAO_TRY(gemm(ctx, rest, kb, kb, 1.0, P, lda, Dk, n, true, 0.0, W, rest));
+    // (column k of P goes with the variable whose pivot is 1 / Dk(k, k))
+    const CrtBalance piv{Dk, n + 1, 0, 1};
+    MOAO_TRY(gemm_long(ctx, rest, kb, kb, 1.0, P, lda, Dk, n, true, 0.0, W, rest, false, &piv));
     MOAO_TRY(copy_matrix(W, rest, P, lda, rest, kb, ctx->stream));
     // trailing: A22 -= P P^T on the lower tiles
     double* A22 = A + (k0 + kb) + (k0 + kb) * lda;
-    MOAO_TRY(gemm(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A22, lda, true));
+    MOAO_TRY(gemm_long(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A22, lda, true));
   }
   return MOAO_OK;
 }
@@ -95,11 +125,12 @@ moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, co
   for (long k0 = 0; k0 < n; k0 += nb) {
     const long kb = std::min(nb, n - k0);
     double* Bk = B + k0 * ldb;
-    MOAO_TRY(gemm(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, true, 0.0, W, m));
+    const CrtBalance piv{dinv + k0, n + 1, 0, 1};
+    MOAO_TRY(gemm_long(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, true, 0.0, W, m, false, &piv));
     MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream));
     const long rest = n - k0 - kb;
     if (rest > 0)
-      MOAO_TRY(gemm(ctx, m, rest, kb, -1.0, Bk, ldb, L + (k0 + kb) + k0 * ldl, ldl, true, 1.0,
+      MOAO_TRY(gemm_long(ctx, m, rest, kb, -1.0, Bk, ldb, L + (k0 + kb) + k0 * ldl, ldl, true, 1.0,
                     B + (k0 + kb) * ldb, ldb));
   }
   // Backward: R L = X.
@@ -107,10 +138,12 @@ moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, co
   for (long b = nblk - 1; b >= 0; --b) {
     const long k0 = b * nb, kb = std::min(nb, n - k0);
     double* Bk = B + k0 * ldb;
-    MOAO_TRY(gemm(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, false, 0.0, W, m));
+    MOAO_TRY(gemm_long(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, false, 0.0, W, m));
     MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream));
-    if (k0 > 0)
-      MOAO_TRY(gemm(ctx, m, k0, kb, -1.0, Bk, ldb, L + k0, ldl, false, 1.0, B, ldb));
+    if (k0 > 0) {
+      const CrtBalance piv{L + k0 + k0 * ldl, ldl + 1, 0, 1};  // R(:, k) goes with L(k, :)
+      MOAO_TRY(gemm_long(ctx, m, k0, kb, -1.0, Bk, ldb, L + k0, ldl, false, 1.0, B, ldb, false, &piv));
+    }
   }
   return MOAO_OK;
 }
@@ -261,25 +294,25 @@ moao_status moao_cee_cvv_prec(moao_ctx* ctx, long nmeas, long nmeasts, long nact
     return cee_cvv_mixed(ctx, nmeas, nmeasts, nact, Cmm, ldCmm, Cpp, ldCpp, Cpm, ldCpm, R, ldR, Dx,
                          ldDx, Cee, ldCee, Cvv, ldCvv, Tmp, ldTmp);
   const long nm = nmeas, nt = nmeasts;
+  // the measurements' variances: Ctm and R Cmm scale with them, R with their inverse
+  const CrtBalance var{Cmm, ldCmm + 1, 1, -1}, var_r{Cmm, ldCmm + 1, 1, 1};
   // (1) Cpp <- Cpp - Cpm R^T - R Cpm^T  (syr2k, lower)
-  MOAO_TRY(gemm(ctx, nt, nt, nm, -1.0, Cpm, ldCpm, R, ldR, true, 1.0, Cpp, ldCpp, true));
-  MOAO_TRY(gemm(ctx, nt, nt, nm, -1.0, R, ldR, Cpm, ldCpm, true, 1.0, Cpp, ldCpp, true));
+  MOAO_TRY(gemm_long(ctx, nt, nt, nm, -1.0, Cpm, ldCpm, R, ldR, true, 1.0, Cpp, ldCpp, true, &var));
+  MOAO_TRY(gemm_long(ctx, nt, nt, nm, -1.0, R, ldR, Cpm, ldCpm, true, 1.0, Cpp, ldCpp, true, &var_r));
   // (2) Cpm <- R Cmm  (symm right, Cmm lower-stored)
-  MOAO_TRY(gemm(ctx, nt, nm, nm, 1.0, R, ldR, Cmm, ldCmm, false, 0.0, Cpm, ldCpm, false,
-                TRI_LOWER));
-  MOAO_TRY(gemm(ctx, nt, nm, nm, 1.0, R, ldR, Cmm, ldCmm, true, 1.0, Cpm, ldCpm, false,
-                TRI_STRICT_LOWER));
+  MOAO_TRY(symm_right(ctx, nt, nm, R, ldR, Cmm, ldCmm, Cpm, ldCpm));
   // (3)-(6) Cee <- sym(tril(Cpp))
   MOAO_TRY(sym_from_lower(Cpp, ldCpp, Cee, ldCee, nt, ctx->stream, &ctx->launches));
   // (7) Cee += Cpm R^T
-  MOAO_TRY(gemm(ctx, nt, nt, nm, 1.0, Cpm, ldCpm, R, ldR, true, 1.0, Cee, ldCee));
+  MOAO_TRY(gemm_long(ctx, nt, nt, nm, 1.0, Cpm, ldCpm, R, ldR, true, 1.0, Cee, ldCee, false, &var));
   // (8) Tmp <- Dx sym(tril(Cee))
-  MOAO_TRY(gemm(ctx, nact, nt, nt, 1.0, Dx, ldDx, Cee, ldCee, false, 0.0, Tmp, ldTmp, false,
-                TRI_LOWER));
-  MOAO_TRY(gemm(ctx, nact, nt, nt, 1.0, Dx, ldDx, Cee, ldCee, true, 1.0, Tmp, ldTmp, false,
-                TRI_STRICT_LOWER));
+  MOAO_TRY(symm_right(ctx, nact, nt, Dx, ldDx, Cee, ldCee, Tmp, ldTmp));
   // (9) Cvv <- Tmp Dx^T
-  MOAO_TRY(gemm(ctx, nact, nact, nt, 1.0, Tmp, ldTmp, Dx, ldDx, true, 0.0, Cvv, ldCvv));
+  {
+    const CrtBalance err{Cee, ldCee + 1, 1, -1};  // Tmp(:, k) scales with Cee(k, k)
+    MOAO_TRY(gemm_long(ctx, nact, nact, nt, 1.0, Tmp, ldTmp, Dx, ldDx, true, 0.0, Cvv, ldCvv, false,
+                       &err));
+  }
   return MOAO_OK;
 }
 

@@ -32,12 +32,13 @@
 
 #include "tc_gemm.h"
 #include "context.h"
+#include "tile_walk.cuh"
 #include "moao_b200_debug.h"
 
 namespace moao {
 namespace {
 
-constexpr int TBM = 128, TBN = 256;      // accumulator of one CTA: TMEM lanes x columns
+constexpr int TBM = 128, TBN = kWalkTileN;  // accumulator of one CTA: TMEM lanes x columns
 constexpr int BOX_ROWS = 128;            // rows of one TMA box (A and B operands alike)
 constexpr int KBYTES = 128;              // bytes of K per stage row (one 128B swizzle atom)
 constexpr int A_TILE = TBM * KBYTES;     // 16 KB
@@ -48,8 +49,6 @@ constexpr int ACC_COLS = TBN;            // fp32 / int32 columns of one accumula
 constexpr int TMEM_COLS = 2 * ACC_COLS;  // double-buffered accumulator
 constexpr int STAGE_C = 32 * 32 * 4;     // per epilogue warp: one 32x32 FP32 chunk for TMA
 constexpr unsigned long long kSpinLimit = 1ull << 28;  // default polls of a bounded wait
-constexpr int kBandRows = 2048;          // rows of C per band of the tile order
-constexpr int kMaxBands = 64;
 
 // PAIR = 0: one CTA computes a 128 x 256 tile of C.
 // PAIR = 1: a cluster of two CTAs computes a 256 x 256 tile with M = 256 MMAs
@@ -71,7 +70,7 @@ struct TcCfg {
   static_assert(2 * STAGES + 5 <= 31, "barrier area");
 };
 
-struct __align__(64) TcParams {
+struct __align__(64) TcParams : TileWalk {
   CUtensorMap mapA[kTcMaxMaps];
   CUtensorMap mapB[kTcMaxMaps];
   CUtensorMap mapC;        // FP32 C (rows inner) for the TMA reduce-add epilogue
@@ -80,8 +79,6 @@ struct __align__(64) TcParams {
   int nseg;
   int M, N;
   int a_row0, b_row0;      // row coordinate of C(0,0) in the A / B tensors
-  int lower;               // 1: only C(r, c) with r + diag_off >= c
-  int diag_off;
   int kind;                // TcKind
   int epi;                 // TcEpilogue
   float alpha, beta;
@@ -90,12 +87,12 @@ struct __align__(64) TcParams {
   const int* erow;         // INT8: per-row exponent of A (length M, indexed by r)
   const int* ecol;         // INT8: per-column exponent of B (length N)
   int shift;
-  int modulus;             // kTcEpiMod8
-  int tile_m;              // rows of C per tile (128, or 256 for CTA pairs)
-  int tiles_m, tiles_n;
-  int total_tiles;         // tiles that intersect the written part of C
-  int band;                // row tiles per band of the tile order
-  int band_start[kMaxBands + 1];  // tiles before each band
+  // kTcEpiMod8 / kTcEpiModZ: products per tile, and per product the modulus m,
+  // floor(2^32 / m) and the smallest multiple of m that is at least 2^31
+  int nmod;
+  unsigned md[kTcMaxMaps], md_inv[kTcMaxMaps], md_bias[kTcMaxMaps];
+  int tile0;               // first tile of the launch
+  int items;               // tiles of the launch times nmod
   int* err;
   unsigned long long spin_limit;  // polls of a role's bounded wait before it gives up
 };
@@ -272,49 +269,14 @@ constexpr uint32_t idesc_of(int dfmt, int abfmt, int m) {
          (uint32_t)((TBN >> 3) << 17) | (uint32_t)((m >> 4) << 24);
 }
 
-// First row tile of column tile nt that reaches the written (lower) part.
-__device__ __forceinline__ int first_mt(const TcParams& p, int nt) {
-  if (!p.lower) return 0;
-  const int num = nt * TBN - p.diag_off - (p.tile_m - 1);
-  return num <= 0 ? 0 : (num + p.tile_m - 1) / p.tile_m;
-}
-
-// v-th tile of the walk over the tiles that are written. The row tiles are
-// taken in bands of p.band (about 2,048 rows); a band is walked column by
-// column and each column down the band's rows. A wave of the persistent grid
-// then covers a block of roughly 2,048 rows by 2,300 columns of C, whose A rows
-// and B rows stay in L2 while its tiles run (a column-major walk over all rows
-// streams every A row through L2 in every wave).
-__device__ __forceinline__ void decode_tile(const TcParams& p, int v, int* mt, int* nt) {
-  int b = 0;
-  while (b + 1 < kMaxBands && p.band_start[b + 1] <= v && b + 1 < (p.tiles_m + p.band - 1) / p.band)
-    ++b;
-  v -= p.band_start[b];
-  const int r0 = b * p.band, r1 = min(r0 + p.band, p.tiles_m), h = r1 - r0;
-  // columns whose first written row tile is at or above r0 hold all h tiles of the band
-  int full = p.tiles_n;
-  if (p.lower) {
-    const int num = r0 * p.tile_m + p.diag_off + p.tile_m - 1;
-    full = num < 0 ? 0 : min(p.tiles_n, num / TBN + 1);
-  }
-  if (v < full * h) {
-    *nt = v / h;
-    *mt = r0 + v % h;
-    return;
-  }
-  v -= full * h;
-  for (int c = full; c < p.tiles_n; ++c) {
-    const int f = max(r0, first_mt(p, c));
-    const int cnt = max(0, r1 - f);
-    if (v < cnt || c == p.tiles_n - 1) {
-      *nt = c;
-      *mt = f + v;
-      return;
-    }
-    v -= cnt;
-  }
-  *nt = p.tiles_n - 1;
-  *mt = r0;
+// acc mod m in [0, m) for the k-th modulus: acc + bias is non-negative and
+// congruent, its quotient by multiplication with floor(2^32 / m) is at most one
+// too small, and one conditional subtraction (the smaller of t and t - m as
+// unsigned) finishes. |acc| < 2^31.
+__device__ __forceinline__ unsigned mod_of(const TcParams& p, int k, uint32_t acc) {
+  const unsigned v = acc + p.md_bias[k];
+  const unsigned t = v - __umulhi(v, p.md_inv[k]) * p.md[k];
+  return min(t, t - p.md[k]);
 }
 
 // Persistent warp-specialised kernel: warp 0 TMA producer, warp 1 MMA issuer,
@@ -385,9 +347,10 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
     const uint32_t full0 = PAIR ? cluster_addr(smem_u32(full_bar), 0) : 0;
     int it = 0;
     bool ok = true;
-    for (int v = group; v < p.total_tiles && ok; v += ngroups) {
+    for (int v = group; v < p.items && ok; v += ngroups) {
       int mt, nt;
-      decode_tile(p, v, &mt, &nt);
+      decode_tile(p, p.tile0 + v / p.nmod, &mt, &nt);
+      const int mod = v % p.nmod;  // the product: its operands are A[mod], B[mod]
       const int m0 = mt * Cfg::TILE_M + (int)crank * TBM;
       const int n0 = nt * TBN + (int)crank * Cfg::B_ROWS;
       for (int s = 0; s < p.nseg && ok; ++s) {
@@ -405,13 +368,13 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
           if (PAIR) {
             if (crank == 0) mbar_expect_tx(&full_bar[st], 2 * STAGE_BYTES);
             const uint32_t fb = full0 + (uint32_t)(st * 8);
-            tma_load_2d_pair(sa, &p.mapA[sg.a], xa, p.a_row0 + m0, fb);
-            tma_load_2d_pair(sb, &p.mapB[sg.b], xb, p.b_row0 + n0, fb);
+            tma_load_2d_pair(sa, &p.mapA[sg.a + mod], xa, p.a_row0 + m0, fb);
+            tma_load_2d_pair(sb, &p.mapB[sg.b + mod], xb, p.b_row0 + n0, fb);
           } else {
             mbar_expect_tx(&full_bar[st], STAGE_BYTES);
-            tma_load_2d(sa, &p.mapA[sg.a], xa, p.a_row0 + m0, &full_bar[st]);
-            tma_load_2d(sb, &p.mapB[sg.b], xb, p.b_row0 + n0, &full_bar[st]);
-            tma_load_2d(sb + BOX_BYTES, &p.mapB[sg.b], xb, p.b_row0 + n0 + BOX_ROWS, &full_bar[st]);
+            tma_load_2d(sa, &p.mapA[sg.a + mod], xa, p.a_row0 + m0, &full_bar[st]);
+            tma_load_2d(sb, &p.mapB[sg.b + mod], xb, p.b_row0 + n0, &full_bar[st]);
+            tma_load_2d(sb + BOX_BYTES, &p.mapB[sg.b + mod], xb, p.b_row0 + n0 + BOX_ROWS, &full_bar[st]);
           }
         }
       }
@@ -434,7 +397,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
                                                   : idesc_of(2, 1, Cfg::TILE_M));
       int it = 0, tc = 0;
       bool ok = true;
-      for (int v = group; v < p.total_tiles && ok; v += ngroups, ++tc) {
+      for (int v = group; v < p.items && ok; v += ngroups, ++tc) {
         const int buf = tc & 1;
         const uint32_t use = tc >> 1;
         if (use > 0 && !mbar_wait(&tempty_bar[buf], (use - 1) & 1, p.err, 4, p.spin_limit)) break;
@@ -482,9 +445,9 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
     const int half = (warp - 4) >> 2;
     const uint32_t tempty0 = PAIR ? cluster_addr(smem_u32(tempty_bar), 0) : 0;
     int tc = 0;
-    for (int v = group; v < p.total_tiles; v += ngroups, ++tc) {
+    for (int v = group; v < p.items; v += ngroups, ++tc) {
       int mt, nt;
-      decode_tile(p, v, &mt, &nt);
+      decode_tile(p, p.tile0 + v / p.nmod, &mt, &nt);
       const int m0 = mt * Cfg::TILE_M + (int)crank * TBM, n0 = nt * TBN;
       const int buf = tc & 1;
       // every lane waits; the warp leaves together if any lane gave up
@@ -526,7 +489,21 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
           __syncwarp();
         }
-        if (r < p.M) {
+        if (p.epi == kTcEpiModZ) {
+          // 32 columns of this row modulo the product's modulus: two 16-byte records
+          const int mod = v % p.nmod;
+          uint32_t w[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            w[j] = __byte_perm(
+                __byte_perm(mod_of(p, mod, v32[4 * j]), mod_of(p, mod, v32[4 * j + 1]), 0x0040),
+                __byte_perm(mod_of(p, mod, v32[4 * j + 2]), mod_of(p, mod, v32[4 * j + 3]), 0x0040),
+                0x5410);
+          uint4* z = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.C) + (size_t)v * kTcZTile) +
+                     (c0 >> 4) * TBM + q * 32 + lane;
+          z[0] = make_uint4(w[0], w[1], w[2], w[3]);
+          z[TBM] = make_uint4(w[4], w[5], w[6], w[7]);
+        } else if (r < p.M) {
           // Mask of the chunk's columns that this row writes.
           uint32_t mask = 0;
 #pragma unroll
@@ -568,13 +545,9 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
           } else if (p.epi == kTcEpiMod8) {
             // the exact int32 sum reduced modulo p.modulus, one byte per element
             uint8_t* dst = static_cast<uint8_t*>(p.C) + (size_t)(n0 + c0) * p.ldc + r;
-            const int md = p.modulus;
 #pragma unroll
             for (int j = 0; j < 32; ++j)
-              if (mask >> j & 1u) {
-                const int t = (int)v32[j] % md;
-                dst[(size_t)j * p.ldc] = (uint8_t)(t < 0 ? t + md : t);
-              }
+              if (mask >> j & 1u) dst[(size_t)j * p.ldc] = (uint8_t)mod_of(p, 0, v32[j]);
           } else {
             double* dst = static_cast<double*>(p.C) + (size_t)(n0 + c0) * p.ldc + r;
             const int er = p.erow[r] + p.shift;
@@ -625,6 +598,150 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
   }
 }
 
+// ---- reconstruction of the kTcEpiModZ products
+//
+// P from its residues z_i (i < 16) by the fractional form of the Chinese
+// remainder theorem: with c_i = (M / m_i)^-1 mod m_i, P / M = sum z_i c_i / m_i
+// modulo 1. The weights c_i / m_i are kept to 80 bits (ten bytes), so ten sums of
+// 16 byte-by-byte products (four dp4a each) and their carries give P / M to
+// 2^-69, which is 2^-57 of a P of 2^114 (the size of a product of 1,024 terms
+// whose operands' rms is an eighth of their largest). Mixed-radix (Garner)
+// reconstruction takes 120 dependent steps per element instead.
+constexpr int kFracBytes = 10;
+struct FracWeights {
+  uint32_t w[kFracBytes][kCrt64Moduli / 4];  // byte b (0 lowest) of moduli 4 g .. 4 g + 3
+};
+constexpr int modinv64(int a, int m) {
+  int t = 0, nt = 1, r = m, nr = a % m;
+  while (nr != 0) {
+    const int q = r / nr, t2 = t - q * nt, r2 = r - q * nr;
+    t = nt;
+    nt = t2;
+    r = nr;
+    nr = r2;
+  }
+  return t < 0 ? t + m : t;
+}
+constexpr FracWeights frac_weights() {
+  FracWeights f{};
+  for (int i = 0; i < kCrt64Moduli; ++i) {
+    const int m = kCrt64Mod[i];
+    int prod = 1;  // M / m_i mod m_i
+    for (int j = 0; j < kCrt64Moduli; ++j)
+      if (j != i) prod = prod * (kCrt64Mod[j] % m) % m;
+    int rem = modinv64(prod, m);
+    for (int b = kFracBytes - 1; b >= 0; --b) {  // long division of c_i by m_i, byte by byte
+      rem *= 256;
+      f.w[b][i / 4] |= (uint32_t)(rem / m) << (8 * (i % 4));
+      rem %= m;
+    }
+  }
+  return f;
+}
+__constant__ FracWeights c_frac = frac_weights();
+
+// M as the sum of two doubles: the product of the first eight moduli is below
+// 2^64 = 2^8 times an odd 56-bit number, so it is split exactly into 32-bit parts.
+struct ModProduct {
+  double hi, lo;
+};
+constexpr ModProduct mod_product() {
+  unsigned __int128 v = 1;
+  for (int i = 0; i < kCrt64Moduli; ++i) v *= (unsigned)kCrt64Mod[i];  // < 2^126
+  const double hi = (double)v;
+  const unsigned __int128 back = (unsigned __int128)hi;
+  const double lo = back > v ? -(double)(back - v) : (double)(v - back);
+  return {hi, lo};
+}
+
+__device__ __forceinline__ uint32_t dp4a_u(uint32_t a, uint32_t b, uint32_t c) {
+  return __dp4a(a, b, c);
+}
+
+// e of a row whose largest biased exponent is b: |x| < 2^e
+__device__ __forceinline__ int exp_of_row(int b) { return b >= 0 ? b - 1022 : 0; }
+// value of 2^e (|e| <= 1022)
+__device__ __forceinline__ double exp2i(int e) {
+  return __hiloint2double((e + 1023) << 20, 0);
+}
+
+// A block takes one 16-column group of a tile per 128 threads: a thread owns a
+// row of it, so the 16 planes are read as 16-byte records and C by coalesced
+// columns. Bound by issue (40 dp4a and about as many integer operations per
+// element), with the planes' 16 bytes per element next.
+constexpr int kCombThreads = 256;
+__global__ void __launch_bounds__(kCombThreads)
+    modz_combine_kernel(const __grid_constant__ TileWalk walk, int tile0, const uint8_t* __restrict__ Z,
+                        int M, int N, int bits, const int* __restrict__ ea,
+                        const int* __restrict__ eb, double alpha, double beta,
+                        double* __restrict__ C, long long ldc, const int* __restrict__ skip_a, const int* __restrict__ skip_b) {
+  if (*skip_a || *skip_b) return;
+  int mt, nt;
+  decode_tile(walk, tile0 + (int)blockIdx.x, &mt, &nt);
+  const int row = threadIdx.x & (TBM - 1);
+  const int grp = blockIdx.y * (kCombThreads / TBM) + threadIdx.x / TBM;
+  const int r = mt * TBM + row, c0 = nt * TBN + grp * 16;
+  if (r >= M || c0 >= N || (walk.lower && r < c0)) return;
+  const uint4* z = reinterpret_cast<const uint4*>(Z + (size_t)blockIdx.x * kCrt64Moduli * kTcZTile) +
+                   grp * TBM + row;
+  uint4 pl[kCrt64Moduli];
+#pragma unroll
+  for (int i = 0; i < kCrt64Moduli; ++i) pl[i] = __ldcs(z + i * (kTcZTile / 16));
+  constexpr ModProduct mp = mod_product();
+  const double er = exp2i(exp_of_row(ea[r]) - bits);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    double old[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + 4 * q + j;
+      old[j] = (beta != 0.0 && c < N && !(walk.lower && r < c)) ? C[(size_t)c * ldc + r] : 0.0;
+    }
+    // residues of column j: four words of four moduli (byte transposes of 4 x 4)
+    uint32_t zz[4][4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      uint32_t w[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint4 v = pl[4 * g + i];
+        w[i] = q == 0 ? v.x : (q == 1 ? v.y : (q == 2 ? v.z : v.w));
+      }
+      const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
+      const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
+      zz[0][g] = __byte_perm(a, b, 0x5410);
+      zz[1][g] = __byte_perm(a, b, 0x7632);
+      zz[2][g] = __byte_perm(c, d, 0x5410);
+      zz[3][g] = __byte_perm(c, d, 0x7632);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = c0 + 4 * q + j;
+      if (c >= N || (walk.lower && r < c)) continue;
+      uint32_t p[kFracBytes];  // each below 2^20
+#pragma unroll
+      for (int b = 0; b < kFracBytes; ++b) {
+        uint32_t t = 0;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) t = dp4a_u(zz[j][g], c_frac.w[b][g], t);
+        p[b] = t;
+      }
+      // the sum modulo 2^80: low 16 bits, then the signed 64-bit fraction above them
+      const uint32_t low = p[0] + (p[1] << 8);
+      const unsigned long long mid = (unsigned long long)(p[2] + (p[3] << 8) + (low >> 16)) +
+                                     ((unsigned long long)p[4] << 16) +
+                                     ((unsigned long long)p[5] << 24);
+      const uint32_t top = p[6] + (p[7] << 8) + (p[8] << 16) + (p[9] << 24);
+      const long long frac = (long long)(mid + ((unsigned long long)top << 32));
+      const double f = (double)frac + (double)(low & 0xffffu) * (1.0 / 65536.0);
+      // P 2^-(bits) = f M 2^-64 2^-(bits): M's 2^-64 folded into the exponents
+      const double v = fma(f, mp.hi * 0x1p-64, f * (mp.lo * 0x1p-64));
+      const double s = (v * er) * exp2i(exp_of_row(eb[c]) - bits);
+      C[(size_t)c * ldc + r] = beta != 0.0 ? fma(alpha, s, beta * old[j]) : alpha * s;
+    }
+  }
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
   static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
   static std::once_flag once;
@@ -640,6 +757,11 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 
 }  // namespace
+
+long tc_tile_count(long M, long N, bool lower) {
+  TileWalk w{};
+  return M > 0 && N > 0 ? fill_walk(&w, M, N, lower ? 1 : 0, 0, TBM) : 0;
+}
 
 moao_status make_tc_map(TcTensor* t, const void* base, int kind, long long rows, long long kcols,
                         long long row_stride_elems, int box_rows) {
@@ -684,6 +806,9 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
     return set_error(MOAO_ERR_BAD_ARG, "tc_gemm: fp32 epilogue needs bf16 or fp16 operands");
   if (g.epi == kTcEpiMod8 && (g.kind != kTcI8 || g.modulus < 2 || g.modulus > 256))
     return set_error(MOAO_ERR_BAD_ARG, "tc_gemm: modular epilogue needs int8 and a modulus <= 256");
+  if (g.epi == kTcEpiModZ &&
+      (g.kind != kTcI8 || g.nmod < 1 || g.nmod > g.nA || g.nmod > g.nB || !g.moduli || g.nseg != 1))
+    return set_error(MOAO_ERR_BAD_ARG, "tc_gemm: modular products need int8 operands per modulus");
   if (g.epi == kTcEpiF32 && (!g.erow) != (!g.ecol))
     return set_error(MOAO_ERR_BAD_ARG, "tc_gemm: row and column exponents go together");
   TcParams p;
@@ -712,8 +837,6 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
   p.N = (int)g.N;
   p.a_row0 = g.a_row0;
   p.b_row0 = g.b_row0;
-  p.lower = g.lower;
-  p.diag_off = g.diag_off;
   p.kind = g.kind;
   p.epi = g.epi;
   p.alpha = g.alpha;
@@ -723,33 +846,31 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
   p.erow = g.erow;
   p.ecol = g.ecol;
   p.shift = g.shift;
-  p.modulus = g.modulus;
   p.err = g.err;
   p.spin_limit = g.spin_limit > 0 ? g.spin_limit : kSpinLimit;
   // Pairs of CTAs (256-row tiles) when asked for and C has more than one
   // 128-row tile; a grid capped below four CTAs keeps single CTAs.
-  const bool pair = g.pair && g.M > TBM && (g.max_ctas <= 0 || g.max_ctas >= 4);
-  p.tile_m = pair ? TcCfg<1>::TILE_M : TcCfg<0>::TILE_M;
-  p.tiles_m = (int)((g.M + p.tile_m - 1) / p.tile_m);
-  p.tiles_n = (int)((g.N + TBN - 1) / TBN);
-  p.band = std::max(kBandRows / p.tile_m, (p.tiles_m + kMaxBands - 1) / kMaxBands);
-  const int nbands = (p.tiles_m + p.band - 1) / p.band;
-  long total = 0;
-  for (int b = 0; b < nbands; ++b) {
-    p.band_start[b] = (int)total;
-    const long r0 = (long)b * p.band, r1 = std::min<long>(r0 + p.band, p.tiles_m);
-    for (int nt = 0; nt < p.tiles_n; ++nt) {
-      long first = 0;
-      if (g.lower) {
-        const long num = (long)nt * TBN - g.diag_off - (p.tile_m - 1);
-        first = num <= 0 ? 0 : (num + p.tile_m - 1) / p.tile_m;
-      }
-      total += std::max(0L, r1 - std::max(r0, first));
+  const bool modz = g.epi == kTcEpiModZ;
+  const bool pair = !modz && g.pair && g.M > TBM && (g.max_ctas <= 0 || g.max_ctas >= 4);
+  const long total = fill_walk(&p, g.M, g.N, g.lower, g.diag_off, pair ? TcCfg<1>::TILE_M
+                                                                       : TcCfg<0>::TILE_M);
+  if (total == 0) return MOAO_OK;
+  p.nmod = 1;
+  if (modz || g.epi == kTcEpiMod8) {
+    p.nmod = modz ? g.nmod : 1;
+    for (int i = 0; i < p.nmod; ++i) {
+      const unsigned m = (unsigned)(modz ? g.moduli[i] : g.modulus);
+      p.md[i] = m;
+      p.md_inv[i] = (unsigned)((1ull << 32) / m);
+      p.md_bias[i] = (unsigned)(((1ull << 31) + m - 1) / m * m);
     }
   }
-  for (int b = nbands; b <= kMaxBands; ++b) p.band_start[b] = (int)total;
-  if (total == 0) return MOAO_OK;
-  p.total_tiles = (int)total;
+  p.tile0 = modz ? (int)g.tile0 : 0;
+  const long run = modz && g.tiles > 0 ? std::min(g.tiles, total - g.tile0) : total - p.tile0;
+  if (run <= 0) return MOAO_OK;
+  if (run * p.nmod > 0x7fffffffL) return set_error(MOAO_ERR_BAD_ARG, "tc_gemm: too many tiles");
+  const long items = run * p.nmod;
+  p.items = (int)items;
   // C += alpha * acc (beta 1) through TMA reductions when C's layout allows a
   // tensor map: 16-byte aligned base and row stride.
   p.c_tma = 0;
@@ -778,7 +899,7 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
     static std::atomic<unsigned long long> configured{0};
     MOAO_CUDA_TRY(set_smem_limit(tc_gemm_kernel<0>, (int)TcCfg<0>::SMEM, configured));
     const long ctas =
-        std::min<long>(total, g.max_ctas > 0 ? std::min(g.max_ctas, num_sms) : num_sms);
+        std::min<long>(items, g.max_ctas > 0 ? std::min(g.max_ctas, num_sms) : num_sms);
     tc_gemm_kernel<0><<<(unsigned)ctas, THREADS, TcCfg<0>::SMEM, s>>>(p);
   } else {
     static std::atomic<unsigned long long> configured{0};
@@ -807,10 +928,24 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
       if (dev < 64) resident[dev].store(groups);
     }
     if (g.max_ctas > 0) groups = std::min(groups, g.max_ctas / 2);
-    groups = (int)std::min<long>(groups, total);
+    groups = (int)std::min<long>(groups, items);
     cfg.gridDim = dim3((unsigned)(2 * groups));
     MOAO_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_gemm_kernel<1>, p));
   }
+  if (launches) ++*launches;
+  MOAO_CUDA_TRY(cudaGetLastError());
+  return MOAO_OK;
+}
+
+moao_status tc_modz_combine(const TcModz& z, cudaStream_t s, long long* launches) {
+  TileWalk w{};
+  const long total = fill_walk(&w, z.M, z.N, z.lower, 0, TBM);
+  const long run = z.tiles > 0 ? std::min(z.tiles, total - z.tile0) : total - z.tile0;
+  if (run <= 0) return MOAO_OK;
+  const dim3 grid((unsigned)run, TBN / 16 / (kCombThreads / TBM));
+  modz_combine_kernel<<<grid, kCombThreads, 0, s>>>(w, (int)z.tile0, z.Z, (int)z.M, (int)z.N, z.bits,
+                                                    z.ea, z.eb, z.alpha, z.beta, z.C, z.ldc,
+                                                    z.skip_a, z.skip_b);
   if (launches) ++*launches;
   MOAO_CUDA_TRY(cudaGetLastError());
   return MOAO_OK;
@@ -825,7 +960,7 @@ extern "C" moao_status moao_debug_tc_gemm(moao_ctx* ctx, int kind, long M, long 
                                           const int* ecol, int shift, int lower) {
   using namespace moao;
   if (!ctx || !A || !B || !C || !pa || !pb || kind < 0 || kind > 2 || na < 1 ||
-      na > kTcMaxMaps || nb < 1 || nb > kTcMaxMaps || npairs < 1 || npairs > kTcMaxSegs ||
+      na > 6 || nb < 1 || nb > 6 || npairs < 1 || npairs > kTcMaxSegs ||
       ldc < M || lda < K || ldb < K)
     return set_error(MOAO_ERR_BAD_ARG, "debug_tc_gemm: bad arguments");
   std::lock_guard<std::mutex> lk(ctx->mu);

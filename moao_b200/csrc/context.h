@@ -69,6 +69,7 @@ struct moao_ctx {
   // FP64 products by residues (crt_f64.cu): operands' residues and row maxima,
   // the product's residues, the guard flags
   moao::DevBuf cf_a, cf_b, cf_ma, cf_mb, cf_k, cf_z, cf_flag;
+  bool chained = true;  // chained launches of the small FP64 kernels (off under stream capture)
   bool crt_f64 = true;  // off where nothing may be allocated (stream capture, no-alloc calls)
   long mx_factored_n = -1;  // size of the factorisation held in mx_* (reuse across targets)
   // Block-constant offsets of Cmm known to the caller (moao_ctx_set_offsets):
@@ -184,6 +185,8 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
 moao_status gemm(moao_ctx* ctx, long M, long N, long K, double alpha, const double* A, long lda,
                  const double* B, long ldb, bool transB, double beta, double* C, long ldc,
                  bool lowerC = false, TriMode tri = TRI_FULL);
+// Creates the context's side stream and lookahead events on first use.
+moao_status ensure_lookahead(moao_ctx* ctx);
 // Factor the nb x nb diagonal block A in place (FP64) and write its inverse into D.
 moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long ldd, long nb,
                             long col0, int* d_info, double* W);

@@ -400,6 +400,10 @@ static long chunk_tiles(long total) {
   return std::min<long>(total, (long)(kZBytes / (kNM * kTcZTile)));
 }
 
+moao_status crt64_reserve(moao_ctx* ctx, long M, long N, bool lower) {
+  return ctx->cf_z.ensure((size_t)chunk_tiles(tc_tile_count(M, N, lower)) * kNM * kTcZTile);
+}
+
 moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const CrtOperand& B, long b0,
                           const GemmArgs* fp64, int n, int max_ctas) {
   const GemmArgs& f = fp64[0];

@@ -50,6 +50,9 @@ struct CrtBalance {
   int half, sign;
 };
 
+// Sizes the product's residue buffer for M x N (crt64_product does so itself).
+moao_status crt64_reserve(moao_ctx* ctx, long M, long N, bool lower);
+
 // g (triB: full) by residue products, operands included.
 moao_status crt64_gemm(moao_ctx* ctx, const GemmArgs& g, const CrtBalance* bal);
 // C (M x n) = A (M x n) S, S the symmetric n x n matrix in the lower triangle of B.

@@ -25,6 +25,7 @@ struct GemmArgs {
   double* C = nullptr;        // M x N, column-major, ldc
   long ldc = 0;
   bool lowerC = false;        // write only C(i, j) with i >= j (SYRK / SYR2K)
+  bool chained = false;       // may start beside its predecessor in the stream (dense_f64.cu)
   int cfg = 1;                // tile configuration of the large products (128x64 CTA tiles;
                               // 0: K 16 per stage, 4 stages; 1: K 32, 2 stages (default);
                               // 2: K 32, 3 stages; 3: K 16, 6 stages)
@@ -44,13 +45,15 @@ moao_status gemm_f64_guarded(const GemmArgs& g, long tile0, long tiles, const in
 // zeros above the diagonal, ldi). On a non-positive pivot the 1-based global
 // column (col0 + local column + 1) is stored in *d_info if it is still 0.
 moao_status potrf_inv_leaf(double* A, long lda, double* Linv, long ldi, int n, long col0,
-                           int* d_info, cudaStream_t s, long long* launches);
+                           int* d_info, bool chained, cudaStream_t s, long long* launches);
 
 // Elementwise helpers (column-major).
 moao_status copy_matrix(const double* src, long lds, double* dst, long ldd, long m, long n,
                         cudaStream_t s);
-moao_status fill_matrix(double* A, long lda, long m, long n, double v, cudaStream_t s,
-                        long long* launches);
+// dst (m x n) = src and the zm x zn block at z = 0, in one launch.
+moao_status copy_zero(const double* src, long lds, double* dst, long ldd, long m, long n, double* z,
+                      long ldz, long zm, long zn, bool chained, cudaStream_t s,
+                      long long* launches);
 // Cee <- sym(tril(Cpp)): the net effect of laset('U',0,0) + lacpy('L') +
 // geadd('T') + scal(diag, 0.5) in lapack/compute/cee_cvv.cpp:73-92.
 moao_status sym_from_lower(const double* Cpp, long ldp, double* Cee, long lde, long n,

@@ -34,12 +34,13 @@ constexpr int PAD_K = 4;   // doubles of padding on k-contiguous rows
 // diagonal-block recursion). BK (K per pipeline stage, a multiple of 16) and
 // STAGES (the cp.async ring) are the other dimensions a configuration sets
 // (GemmArgs::cfg, chosen per context: moao_ctx_set_gemm_tile / the autotuner).
-template <int BM_, int BN_, int WM_, int BK_ = 16, int STAGES_ = 4>
+template <int BM_, int BN_, int WM_, int BK_ = 16, int STAGES_ = 4, int WN_ = 32>
 struct Tile {
-  static constexpr int BM = BM_, BN = BN_, WM = WM_, BK = BK_, STAGES = STAGES_;
-  static constexpr int WARPS_M = BM / WM, WARPS_N = BN / 32;
+  static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, BK = BK_, STAGES = STAGES_;
+  static constexpr int WARPS_M = BM / WM, WARPS_N = BN / WN;
   static constexpr int NTHREADS = 32 * WARPS_M * WARPS_N;
   static constexpr int MF = WM / 8;             // 8-row fragments per warp
+  static constexpr int NF = WN / 8;             // 8-column fragments per warp
   static constexpr int LDA_S = BM + PAD_MN;     // As[k][m]
   static constexpr int LDB_S = BN + PAD_MN;     // Bs[k][n]   (transB)
   static constexpr int LDBT_S = BK + PAD_K;     // Bs[n][k]   (!transB)
@@ -49,6 +50,10 @@ struct Tile {
 };
 using TileL = Tile<128, 64, 32>;
 using TileS = Tile<64, 64, 32>;
+// 32 x 32 tiles for the products of a handful of 64 x 64 ones: an SM does a
+// 64 x 64 x K tile in 64 K cycles (its FP64 rate is 64 multiply-adds a cycle), so
+// few large tiles leave a product of the diagonal-block recursion to a few SMs.
+using TileXS = Tile<32, 32, 16, 32, 3, 16>;
 // alternative large-product configurations (GemmArgs::cfg 1..3)
 using TileL32x2 = Tile<128, 64, 32, 32, 2>;   // 102 KB: two CTAs per SM, two k16 steps per barrier
 using TileL32x3 = Tile<128, 64, 32, 32, 3>;   // 154 KB: one CTA per SM
@@ -105,6 +110,35 @@ struct KParams {
   // the column tiles in turn, the band's row tiles fastest
   int tiles_m, tiles_n, group_m;
 };
+
+// Chained launches (programmatic dependent launch): a kernel launched with
+// launch_chained may start while its predecessor in the stream still runs; it lets
+// its own successor start as early, and waits here until the predecessor has
+// finished and its writes are visible. Every thread of a chained kernel calls this
+// before it touches memory, so completion orders along the chain as in a plain
+// stream. Without the launch attribute both instructions do nothing. A diagonal
+// block of 1,024 columns is a chain of about 90 short launches; with the 32 x 32
+// tiles, an nmeas 640 FP64 reconstructor takes 507 us instead of 952.
+__device__ __forceinline__ void chain_wait() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+template <typename... P, typename... A>
+cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
+                           cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
 
 // Tile v of the launch in band order. Consecutive CTAs share one column strip
 // of B and the band's row strips of A stay in L2 while the band sweeps the
@@ -168,7 +202,7 @@ __device__ __forceinline__ void load_k_tile(double* s, const double* g, long ld,
 template <class TL, bool TRANSB, bool LOWERC, int VEC, bool MMA16>
 __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const long m0,
                                           const long n0) {
-  constexpr int BM = TL::BM, BN = TL::BN, NTHREADS = TL::NTHREADS, MF = TL::MF;
+  constexpr int BM = TL::BM, BN = TL::BN, NTHREADS = TL::NTHREADS, MF = TL::MF, NF = TL::NF;
   constexpr int BK = TL::BK, STAGES = TL::STAGES;
   constexpr int LDA_S = TL::LDA_S, LDB_S = TL::LDB_S, LDBT_S = TL::LDBT_S;
   constexpr int A_STAGE = TL::A_STAGE, B_STAGE = TL::B_STAGE;
@@ -185,16 +219,16 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
   const int ntiles = (ke > kb) ? (int)((ke - kb + BK - 1) / BK) : 0;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int wm = (warp % TL::WARPS_M) * TL::WM, wn = (warp / TL::WARPS_M) * 32;
+  const int wm = (warp % TL::WARPS_M) * TL::WM, wn = (warp / TL::WARPS_M) * TL::WN;
   const int gid = lane >> 2, tig = lane & 3;
 
-  // acc[i][j][h]: k4 layout = MF m-frags of 8 rows x 4 n-frags x 2;
-  // k16 layout = MF/2 m-frags of 16 rows x 4 n-frags x 4.
-  double acc[MF][4][2];
+  // acc[i][j][h]: k4 layout = MF m-frags of 8 rows x NF n-frags x 2;
+  // k16 layout = MF/2 m-frags of 16 rows x NF n-frags x 4.
+  double acc[MF][NF][2];
 #pragma unroll
   for (int i = 0; i < MF; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int j = 0; j < NF; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
 
   auto issue = [&](int stage, int t) {
     const long k0 = kb + (long)t * BK;
@@ -245,9 +279,9 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
     if (MMA16) {
 #pragma unroll
       for (int k16 = 0; k16 < BK; k16 += 16) {
-        double bf[4][4];
+        double bf[NF][4];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
+        for (int j = 0; j < NF; ++j)
 #pragma unroll
           for (int r = 0; r < 4; ++r) {
             const int k = k16 + r * 4 + tig, n = wn + j * 8 + gid;
@@ -260,7 +294,7 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
           for (int r = 0; r < 8; ++r)
             af[r] = as[(k16 + (r >> 1) * 4 + tig) * LDA_S + wm + i * 16 + gid + 8 * (r & 1)];
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
+          for (int j = 0; j < NF; ++j)
             dmma16(acc[2 * i][j][0], acc[2 * i][j][1], acc[2 * i + 1][j][0], acc[2 * i + 1][j][1],
                    af, bf[j]);
         }
@@ -268,18 +302,18 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
     } else {
 #pragma unroll
       for (int k4 = 0; k4 < BK; k4 += 4) {
-        double a[MF], b[4];
+        double a[MF], b[NF];
 #pragma unroll
         for (int i = 0; i < MF; ++i) a[i] = as[(k4 + tig) * LDA_S + wm + i * 8 + gid];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < NF; ++j) {
           if (TRANSB) b[j] = bs[(k4 + tig) * LDB_S + wn + j * 8 + gid];
           else b[j] = bs[(wn + j * 8 + gid) * LDBT_S + k4 + tig];
         }
 #pragma unroll
         for (int i = 0; i < MF; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+          for (int j = 0; j < NF; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
       }
     }
   }
@@ -307,7 +341,7 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
   for (int i = 0; i < MF; ++i) {
     const int rr = MMA16 ? wm + (i >> 1) * 16 + (i & 1) * 8 + gid : wm + i * 8 + gid;
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int j = 0; j < NF; ++j)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int cc = wn + j * 8 + 2 * tig + h;
@@ -326,6 +360,7 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
 template <class TL, bool TRANSB, bool LOWERC, int VEC, bool MMA16>
 __global__ void __launch_bounds__(TL::NTHREADS) gemm_f64_kernel(const KParams p) {
   extern __shared__ __align__(16) double smem[];
+  chain_wait();
   long m0 = 0, n0 = 0;
   if (!band_tile<TL::BM, TL::BN, LOWERC>(p, blockIdx.x, &m0, &n0)) return;
   if (LOWERC && m0 + TL::BM <= n0) return;  // tile strictly above the diagonal
@@ -362,7 +397,7 @@ bool use_mma16() {
 }
 
 template <class TL, bool TRANSB, bool LOWERC, int VEC, bool MMA16>
-moao_status launch_gemm_t(const KParams& p, cudaStream_t s) {
+moao_status launch_gemm_t(const KParams& p, bool chained, cudaStream_t s) {
   static std::atomic<unsigned long long> configured{0};
   auto kern = gemm_f64_kernel<TL, TRANSB, LOWERC, VEC, MMA16>;
   MOAO_CUDA_TRY(set_smem_limit(kern, (int)TL::SMEM_BYTES, configured));
@@ -379,8 +414,8 @@ moao_status launch_gemm_t(const KParams& p, cudaStream_t s) {
   }
   if (total <= 0) return MOAO_OK;
   if (total > 0x7fffffffL) return set_error(MOAO_ERR_BAD_ARG, "gemm: too many tiles");
-  kern<<<(unsigned)total, TL::NTHREADS, TL::SMEM_BYTES, s>>>(q);
-  MOAO_CUDA_TRY(cudaGetLastError());
+  MOAO_CUDA_TRY(launch_chained(chained, kern, dim3((unsigned)total), dim3(TL::NTHREADS),
+                               TL::SMEM_BYTES, s, q));
   return MOAO_OK;
 }
 
@@ -391,19 +426,29 @@ bool small_tiles(const KParams& p) {
   return tiles < 2 * 148;
 }
 
+// Products of at most 74 tiles of 64 x 64 (half the SMs) take 32 x 32 ones: up to two
+// per SM. The small products of an nmeas 640 reconstructor: 19.8 -> 11.9 us a launch
+// on average, of an nmeas 12,032 one's diagonal blocks 18.3 -> 11.6 (B200, CUDA events
+// around each launch).
+bool tiny_tiles(const KParams& p, bool lower) {
+  const long tiles = ((p.M + 63) / 64) * ((p.N + 63) / 64);
+  return (lower ? (tiles + 1) / 2 : tiles) <= 74;
+}
+
 template <bool TRANSB, bool LOWERC, int VEC>
-moao_status launch_gemm(const KParams& p, int cfg, cudaStream_t s) {
+moao_status launch_gemm(const KParams& p, int cfg, bool ch, cudaStream_t s) {
+  if (use_mma16() && tiny_tiles(p, LOWERC)) return launch_gemm_t<TileXS, TRANSB, LOWERC, VEC, true>(p, ch, s);
   if (small_tiles(p))
-    return use_mma16() ? launch_gemm_t<TileS, TRANSB, LOWERC, VEC, true>(p, s)
-                       : launch_gemm_t<TileS, TRANSB, LOWERC, VEC, false>(p, s);
+    return use_mma16() ? launch_gemm_t<TileS, TRANSB, LOWERC, VEC, true>(p, ch, s)
+                       : launch_gemm_t<TileS, TRANSB, LOWERC, VEC, false>(p, ch, s);
   switch (cfg) {
-    case 1: return launch_gemm_t<TileL32x2, TRANSB, LOWERC, VEC, true>(p, s);
-    case 2: return launch_gemm_t<TileL32x3, TRANSB, LOWERC, VEC, true>(p, s);
-    case 3: return launch_gemm_t<TileL16x6, TRANSB, LOWERC, VEC, true>(p, s);
+    case 1: return launch_gemm_t<TileL32x2, TRANSB, LOWERC, VEC, true>(p, ch, s);
+    case 2: return launch_gemm_t<TileL32x3, TRANSB, LOWERC, VEC, true>(p, ch, s);
+    case 3: return launch_gemm_t<TileL16x6, TRANSB, LOWERC, VEC, true>(p, ch, s);
     default: break;
   }
-  return use_mma16() ? launch_gemm_t<TileL, TRANSB, LOWERC, VEC, true>(p, s)
-                     : launch_gemm_t<TileL, TRANSB, LOWERC, VEC, false>(p, s);
+  return use_mma16() ? launch_gemm_t<TileL, TRANSB, LOWERC, VEC, true>(p, ch, s)
+                     : launch_gemm_t<TileL, TRANSB, LOWERC, VEC, false>(p, ch, s);
 }
 
 KParams params_of(const GemmArgs& g) {
@@ -432,26 +477,19 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1)
     potrf_inv_leaf_kernel(double* A, long lda, double* Linv, long ldi, int n, long col0,
                           int* info) {
   extern __shared__ __align__(16) double leaf_smem[];
+  chain_wait();
   leaf_factor_inverse(A, lda, Linv, ldi, n, col0, info, leaf_smem);
 }
 
-__global__ void copy_kernel(const double* __restrict__ src, long lds, double* __restrict__ dst,
-                            long ldd, long m, long n) {
-  const long total = m * n;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
-       e += (long)gridDim.x * blockDim.x) {
-    const long i = e % m, j = e / m;
-    dst[j * ldd + i] = src[j * lds + i];
-  }
-}
-
-__global__ void fill_kernel(double* A, long lda, long m, long n, double v) {
-  const long total = m * n;
-  for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total;
-       e += (long)gridDim.x * blockDim.x) {
-    const long i = e % m, j = e / m;
-    A[j * lda + i] = v;
-  }
+// dst (m x n) = src, and the zn x zm block at z (null: none) = 0: the factor's block
+// into place and the zeros above the diagonal of its inverse.
+__global__ void copy_zero_kernel(const double* __restrict__ src, long lds, double* __restrict__ dst,
+                                 long ldd, long m, long n, double* __restrict__ z, long ldz,
+                                 long zm, long zn) {
+  chain_wait();
+  const long step = (long)gridDim.x * blockDim.x, e0 = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  for (long e = e0; e < m * n; e += step) dst[(e / m) * ldd + e % m] = src[(e / m) * lds + e % m];
+  for (long e = e0; e < zm * zn; e += step) z[(e / zm) * ldz + e % zm] = 0.0;
 }
 
 // Cee(i, j) = Cpp(max(i,j), min(i,j)); the diagonal goes through 2d * 0.5
@@ -490,11 +528,11 @@ moao_status gemm_f64(const GemmArgs& g, cudaStream_t s, long long* launches) {
   moao_status st;
   const int c = g.cfg;
   if (v2) {
-    if (g.transB) st = g.lowerC ? launch_gemm<true, true, 2>(p, c, s) : launch_gemm<true, false, 2>(p, c, s);
-    else st = g.lowerC ? launch_gemm<false, true, 2>(p, c, s) : launch_gemm<false, false, 2>(p, c, s);
+    if (g.transB) st = g.lowerC ? launch_gemm<true, true, 2>(p, c, g.chained, s) : launch_gemm<true, false, 2>(p, c, g.chained, s);
+    else st = g.lowerC ? launch_gemm<false, true, 2>(p, c, g.chained, s) : launch_gemm<false, false, 2>(p, c, g.chained, s);
   } else {
-    if (g.transB) st = g.lowerC ? launch_gemm<true, true, 1>(p, c, s) : launch_gemm<true, false, 1>(p, c, s);
-    else st = g.lowerC ? launch_gemm<false, true, 1>(p, c, s) : launch_gemm<false, false, 1>(p, c, s);
+    if (g.transB) st = g.lowerC ? launch_gemm<true, true, 1>(p, c, g.chained, s) : launch_gemm<true, false, 1>(p, c, g.chained, s);
+    else st = g.lowerC ? launch_gemm<false, true, 1>(p, c, g.chained, s) : launch_gemm<false, false, 1>(p, c, g.chained, s);
   }
   if (st == MOAO_OK && launches) ++*launches;
   return st;
@@ -524,15 +562,15 @@ moao_status gemm_f64_guarded(const GemmArgs& g, long tile0, long tiles, const in
 }
 
 moao_status potrf_inv_leaf(double* A, long lda, double* Linv, long ldi, int n, long col0,
-                           int* d_info, cudaStream_t s, long long* launches) {
+                           int* d_info, bool chained, cudaStream_t s, long long* launches) {
   if (n <= 0) return MOAO_OK;
   if (n > LEAF) return set_error(MOAO_ERR_BAD_ARG, "potrf leaf: n > 64");
   static std::atomic<unsigned long long> configured{0};
   const int smem = LEAF_SMEM_BYTES;
   MOAO_CUDA_TRY(set_smem_limit(potrf_inv_leaf_kernel, smem, configured));
-  potrf_inv_leaf_kernel<<<1, LEAF_THREADS, smem, s>>>(A, lda, Linv, ldi, n, col0, d_info);
+  MOAO_CUDA_TRY(launch_chained(chained, potrf_inv_leaf_kernel, dim3(1), dim3(LEAF_THREADS), (size_t)smem,
+                               s, A, lda, Linv, ldi, n, col0, d_info));
   if (launches) ++*launches;
-  MOAO_CUDA_TRY(cudaGetLastError());
   return MOAO_OK;
 }
 
@@ -544,12 +582,14 @@ moao_status copy_matrix(const double* src, long lds, double* dst, long ldd, long
   return MOAO_OK;
 }
 
-moao_status fill_matrix(double* A, long lda, long m, long n, double v, cudaStream_t s,
-                        long long* launches) {
-  if (m <= 0 || n <= 0) return MOAO_OK;
-  fill_kernel<<<grid_for(m * n), 256, 0, s>>>(A, lda, m, n, v);
+moao_status copy_zero(const double* src, long lds, double* dst, long ldd, long m, long n, double* z,
+                      long ldz, long zm, long zn, bool chained, cudaStream_t s,
+                      long long* launches) {
+  const long total = std::max(m * n, zm * zn);
+  if (total <= 0) return MOAO_OK;
+  MOAO_CUDA_TRY(launch_chained(chained, copy_zero_kernel, dim3(grid_for(total)), dim3(256), 0, s, src, lds,
+                               dst, ldd, m, n, z, ldz, zm, zn));
   if (launches) ++*launches;
-  MOAO_CUDA_TRY(cudaGetLastError());
   return MOAO_OK;
 }
 

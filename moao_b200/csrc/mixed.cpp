@@ -567,13 +567,7 @@ moao_status reconstructor_mixed(moao_ctx* ctx, long n, long m, double* Cmm, long
     // panel's columns, that panel's diagonal block is factored on the side stream
     // while the rest of the update leaves ctx->lookahead_sms SMs to it.
     const bool ahead = ctx->lookahead_sms > 0 && !graph;
-    if (ahead && !ctx->aux) {
-      int lo = 0, hi = 0;
-      MOAO_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
-      MOAO_CUDA_TRY(cudaStreamCreateWithPriority(&ctx->aux, cudaStreamNonBlocking, hi));
-      for (auto& e : ctx->la_ev)
-        MOAO_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    }
+    if (ahead) MOAO_TRY(ensure_lookahead(ctx));
     int nsm = 148;
     MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     MOAO_TRY(diag_block(0, std::min(nb, n), s));

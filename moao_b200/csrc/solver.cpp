@@ -27,6 +27,7 @@ moao_status gemm(moao_ctx* ctx, long M, long N, long K, double alpha, const doub
   g.A = A; g.lda = lda; g.B = B; g.ldb = ldb; g.transB = transB; g.triB = tri;
   g.C = C; g.ldc = ldc; g.lowerC = lowerC;
   g.cfg = ctx->gemm_cfg;
+  g.chained = ctx->chained;
   // algorithmic flops: 2MNK, halved when only a triangle of C or of B counts
   double fl = 2.0 * M * N * K;
   if (lowerC) fl = (double)M * N * K + (double)std::min(M, N) * K;
@@ -62,13 +63,24 @@ moao_status symm_right(moao_ctx* ctx, long M, long n, const double* A, long lda,
   return gemm(ctx, M, n, n, 1.0, A, lda, B, ldb, true, 1.0, C, ldc, false, TRI_STRICT_LOWER);
 }
 
+// The side stream and events of the lookahead (created on first use).
+moao_status ensure_lookahead(moao_ctx* ctx) {
+  if (ctx->aux) return MOAO_OK;
+  int lo = 0, hi = 0;
+  MOAO_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&lo, &hi));
+  MOAO_CUDA_TRY(cudaStreamCreateWithPriority(&ctx->aux, cudaStreamNonBlocking, hi));
+  for (auto& e : ctx->la_ev) MOAO_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  return MOAO_OK;
+}
+
 // Factor the nb x nb diagonal block A (lda) and write its inverse into D (ldd).
 // W is scratch of at least nb*nb/4 doubles... (nb/2 x nb/2 + margin).
 moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long ldd, long nb,
                             long col0, int* d_info, double* W) {
   if (nb <= kLeaf) {
     KernelTimer kt(ctx, "potrf_leaf", (double)nb * nb * nb * (1.0 / 3 + 1.0 / 3));
-    return potrf_inv_leaf(A, lda, D, ldd, (int)nb, col0, d_info, ctx->stream, &ctx->launches);
+    return potrf_inv_leaf(A, lda, D, ldd, (int)nb, col0, d_info, ctx->chained, ctx->stream,
+                          &ctx->launches);
   }
   const long n1 = kLeaf * ((nb + 2 * kLeaf - 1) / (2 * kLeaf));
   const long n2 = nb - n1;
@@ -79,16 +91,51 @@ moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long 
   double* D21 = D + n1;
   double* D22 = D + n1 + n1 * ldd;
   MOAO_TRY(potrf_inv_block(ctx, A11, lda, D11, ldd, n1, col0, d_info, W));
-  // L21 = A21 L11^-T
+  // L21 = A21 L11^-T ; D12 = 0
   MOAO_TRY(gemm(ctx, n2, n1, n1, 1.0, A21, lda, D11, ldd, true, 0.0, W, n2));
-  MOAO_TRY(copy_matrix(W, n2, A21, lda, n2, n1, ctx->stream));
+  MOAO_TRY(copy_zero(W, n2, A21, lda, n2, n1, D + n1 * ldd, ldd, n1, n2, ctx->chained, ctx->stream,
+                     &ctx->launches));
   // A22 -= L21 L21^T (lower)
   MOAO_TRY(gemm(ctx, n2, n2, n1, -1.0, A21, lda, A21, lda, true, 1.0, A22, lda, true));
   MOAO_TRY(potrf_inv_block(ctx, A22, lda, D22, ldd, n2, col0 + n1, d_info, W));
-  // D21 = -D22 L21 D11 ; D12 = 0
+  // D21 = -D22 L21 D11
   MOAO_TRY(gemm(ctx, n2, n1, n1, 1.0, A21, lda, D11, ldd, false, 0.0, W, n2));
   MOAO_TRY(gemm(ctx, n2, n1, n2, -1.0, D22, ldd, W, n2, false, 0.0, D21, ldd));
-  MOAO_TRY(fill_matrix(D + n1 * ldd, ldd, n1, n2, 0.0, ctx->stream, &ctx->launches));
+  return MOAO_OK;
+}
+
+// A22 (rest x rest, lower) -= P P^T by residue products with one panel of lookahead:
+// the update reaches the next panel's columns first, whose diagonal block
+// (next_block, on the side stream) is then factored beside the rest of the update,
+// which leaves it the context's lookahead SMs (nmeas 29,120: 270 -> 252 ms; not beside
+// the FP64 tensor cores' update, whose CTAs hold their SMs for up to 70 us while the
+// block's ~90 launches wait for one). MOAO_ERR_OOM: nothing was done.
+template <class F>
+moao_status trailing_ahead(moao_ctx* ctx, const double* P, long lda, long rest, long kb, long kb1,
+                           double* A22, F next_block) {
+  MOAO_TRY(ensure_lookahead(ctx));
+  CrtOperand op;
+  MOAO_TRY(crt64_begin(ctx));
+  MOAO_TRY(crt64_operand(ctx, P, lda, rest, kb, &op));
+  MOAO_TRY(crt64_reserve(ctx, rest, rest, true));
+  cudaStream_t s = ctx->stream;
+  GemmArgs g;
+  g.M = rest; g.N = kb1; g.K = kb; g.alpha = -1.0; g.beta = 1.0;
+  g.A = P; g.lda = lda;
+  g.B = P; g.ldb = lda; g.transB = true;
+  g.C = A22; g.ldc = lda; g.lowerC = true;
+  MOAO_TRY(crt64_product(ctx, op, 0, op, 0, &g, 1));
+  MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[0], s));
+  MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->la_ev[0], 0));
+  MOAO_TRY(next_block(ctx->aux));
+  MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[1], ctx->aux));
+  g.M = g.N = rest - kb1;
+  g.A = g.B = P + kb1;
+  g.C = A22 + kb1 + kb1 * lda;
+  int nsm = 148;
+  MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+  MOAO_TRY(crt64_product(ctx, op, kb1, op, kb1, &g, 1, std::max(1, nsm - ctx->lookahead_sms)));
+  MOAO_CUDA_TRY(cudaStreamWaitEvent(s, ctx->la_ev[1], 0));
   return MOAO_OK;
 }
 
@@ -96,11 +143,10 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
   const long nb = ctx->nb;
   MOAO_TRY(ctx->ws_w.ensure(sizeof(double) * (size_t)std::max(n, 1L) * nb));
   double* W = ctx->ws_w.as<double>();
+  MOAO_TRY(potrf_inv_block(ctx, A, lda, dinv, n, std::min(nb, n), 0, d_info, W));
   for (long k0 = 0; k0 < n; k0 += nb) {
     const long kb = std::min(nb, n - k0);
-    double* Akk = A + k0 + k0 * lda;
     double* Dk = dinv + k0;  // rows k0.., ld n
-    MOAO_TRY(potrf_inv_block(ctx, Akk, lda, Dk, n, kb, k0, d_info, W));
     const long rest = n - k0 - kb;
     if (rest <= 0) break;
     double* P = A + (k0 + kb) + k0 * lda;
@@ -109,9 +155,25 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
     const CrtBalance piv{Dk, n + 1, 0, 1};
     MOAO_TRY(gemm_long(ctx, rest, kb, kb, 1.0, P, lda, Dk, n, true, 0.0, W, rest, false, &piv));
     MOAO_TRY(copy_matrix(W, rest, P, lda, rest, kb, ctx->stream));
-    // trailing: A22 -= P P^T on the lower tiles
-    double* A22 = A + (k0 + kb) + (k0 + kb) * lda;
-    MOAO_TRY(gemm_long(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A22, lda, true));
+    // trailing: A22 -= P P^T on the lower tiles, then the next diagonal block
+    const long k1 = k0 + kb, kb1 = std::min(nb, rest), r2 = rest - kb1;
+    double* A22 = A + k1 + k1 * lda;
+    bool done = false;
+    if (ctx->lookahead_sms > 0 && r2 > 0 && crt64_pays(ctx, r2, r2, kb, true)) {
+      const moao_status st = trailing_ahead(ctx, P, lda, rest, kb, kb1, A22, [&](cudaStream_t s) {
+        cudaStream_t keep = ctx->stream;
+        ctx->stream = s;
+        const moao_status r = potrf_inv_block(ctx, A22, lda, dinv + k1, n, kb1, k1, d_info, W);
+        ctx->stream = keep;
+        return r;
+      });
+      if (st != MOAO_OK && st != MOAO_ERR_OOM) return st;
+      done = st == MOAO_OK;
+    }
+    if (!done) {
+      MOAO_TRY(gemm_long(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A22, lda, true));
+      MOAO_TRY(potrf_inv_block(ctx, A22, lda, dinv + k1, n, kb1, k1, d_info, W));
+    }
   }
   return MOAO_OK;
 }

@@ -18,9 +18,10 @@
 // rounded additions per element on the FP64 tensor cores.
 //
 // Measured (B200, against the FP64 tensor cores at 28-31 TF/s): the FP64
-// reconstructor at nmeas 29,120 563 -> 270 ms, its Cee/Cvv chain 253 -> 107 ms (107
-// TF/s in the int8 products alone: 1.8 Pop/s); error against an FP64 library's
-// result 1.4e-11 -> 1.2e-11 and 8.2e-12 -> 3.3e-12.
+// reconstructor at nmeas 29,120 563 -> 238 ms (lookahead included), its Cee/Cvv chain
+// 253 -> 84 ms; the int8 products alone run at 1.7 Pop/s over K = 1,024 and 2.1 over
+// K = 29,120. Error against an FP64 library's result 1.5e-11 -> 1.3e-11 and 1.1e-11 ->
+// 4.4e-12.
 //
 // Guard: a NaN, an infinity or a magnitude outside 2^-900 .. 2^900 in an operand
 // (found with the row exponents) or a tensor-core wait that ran out raises a flag on
@@ -39,7 +40,10 @@ namespace {
 
 constexpr int kNM = kCrt64Moduli;
 constexpr int kMaxBits = 57;
-constexpr size_t kZBytes = (size_t)1 << 30;        // residues of the product held at once
+// Tiles of the product held at once (2 GB of residues). Running the combine step of
+// one part beside the products of the next (a second stream, parts of 128 to 1,024
+// tiles) was slower at every size: the products lose what the overlap gains.
+constexpr long kPartTiles = 4096;
 constexpr long kMaxChunks = 4096;
 constexpr size_t kOperandBytes = (size_t)6 << 30;  // residues of one operand held at once
 
@@ -90,9 +94,16 @@ __global__ void exps_over_cols_kernel(const double* __restrict__ A, long lda, lo
   const long c0 = blockIdx.y * 256L + threadIdx.y * 32L;
   if (r >= nr) return;
   ExpMax st;
-#pragma unroll 8
-  for (int c = 0; c < 32; ++c)
-    if (c0 + c < nc) st.add(A[(c0 + c) * lda + r], off ? sign * off[c0 + c] : 0);
+  const int lim = (int)min(32L, nc - c0);
+  const double* a = A + c0 * lda + r;
+#pragma unroll
+  for (int h = 0; h < 32; h += 16) {
+    double v[16];  // all in flight before the first is used
+#pragma unroll
+    for (int c = 0; c < 16; ++c) v[c] = h + c < lim ? a[(h + c) * lda] : 0.0;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) st.add(v[c], off && h + c < lim ? sign * off[c0 + h + c] : 0);
+  }
   st.check(flag);
   st.store(out + r);
 }
@@ -106,10 +117,19 @@ __global__ void exps_over_rows_kernel(const double* __restrict__ A, long lda, lo
   if (c >= nc) return;
   const long r0 = blockIdx.y * 1024L;
   ExpMax st;
-#pragma unroll 8
-  for (int q = 0; q < 32; ++q) {
-    const long r = r0 + q * 32 + threadIdx.x;
-    if (r < nr) st.add(A[c * lda + r], off ? sign * off[r] : 0);
+#pragma unroll
+  for (int h = 0; h < 32; h += 16) {
+    double v[16];
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const long r = r0 + (h + q) * 32 + threadIdx.x;
+      v[q] = r < nr ? A[c * lda + r] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 16; ++q) {
+      const long r = r0 + (h + q) * 32 + threadIdx.x;
+      st.add(v[q], off && r < nr ? sign * off[r] : 0);
+    }
   }
   st.check(flag);
   st.m = __reduce_max_sync(0xffffffffu, st.m);
@@ -164,16 +184,15 @@ __global__ void check_rows_kernel(const int* __restrict__ e, long rows, int* fla
 
 // ---- residues of 57-bit integers
 // X + 2^58 is a non-negative 59-bit integer; its bytes times 256^k mod m_i (two
-// dp4a of unsigned bytes by signed weights) give |r| < 2^19 congruent to X, whose
-// distance to the nearest multiple of m_i comes from FP32 arithmetic that is
-// exact here: r and m_i q are integers below 2^24, and r / m_i is at least
-// 1 / (2 m_i) from a half-integer for odd m_i, far above the quotient's error.
+// dp4a of unsigned bytes by signed weights) and a multiple of m_i give 0 <= r < 2^20
+// congruent to X. The quotient floor((r + h) / m), h = (m - 1) / 2, is the high word of
+// a product with ceil(2^32 / m): it is too large by less than 2^-12, below 1 / m, so
+// the floor is right and r - m q is the centred residue.
 struct ByteWeights {
   int lo[kNM], hi[kNM];  // signed bytes 256^k mod m_i, k = 0..3 and 4..7
-  int bias[kNM];         // -(2^58 mod m_i), on top of the float magic constant
-  float inv[kNM], neg[kNM];
+  int bias[kNM];         // -(2^58 mod m_i) plus a multiple of m_i above 2^18
+  int inv[kNM], half[kNM], neg[kNM];
 };
-constexpr int kMagicBits = 0x4B400000;  // bits of 1.5 * 2^23
 constexpr ByteWeights byte_weights() {
   ByteWeights b{};
   for (int i = 0; i < kNM; ++i) {
@@ -191,9 +210,10 @@ constexpr ByteWeights byte_weights() {
     b.hi[i] = (int)w[1];
     long long t = 1;
     for (int k = 0; k < 58; ++k) t = t * 2 % m;
-    b.bias[i] = kMagicBits - (int)t;
-    b.inv[i] = 1.0f / (float)m;
-    b.neg[i] = -(float)m;
+    b.bias[i] = (262144 + m - 1) / m * m + m - (int)t;
+    b.inv[i] = (int)(((1ll << 32) + m - 1) / m);
+    b.half[i] = (m - 1) / 2;
+    b.neg[i] = -m;
   }
   return b;
 }
@@ -207,7 +227,6 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, int b, int c) {
 
 // The residues of four integers, one word (byte q = residue of x[q]) per modulus.
 __device__ __forceinline__ void residue_words(const long long (&x)[4], uint32_t (&w)[kNM]) {
-  constexpr float kMagic = 12582912.0f;
   uint32_t lo[4], hi[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
@@ -223,11 +242,8 @@ __device__ __forceinline__ void residue_words(const long long (&x)[4], uint32_t 
       if (i == 0) {
         b[q] = lo[q];  // modulo 256: the low byte
       } else {
-        const float f =
-            __int_as_float(dp4a_us(lo[q], c_bw.lo[i], dp4a_us(hi[q], c_bw.hi[i], c_bw.bias[i]))) -
-            kMagic;
-        const float k = fmaf(f, c_bw.inv[i], kMagic) - kMagic;
-        b[q] = (uint32_t)__float_as_int(fmaf(c_bw.neg[i], k, f) + kMagic);
+        const int r = dp4a_us(lo[q], c_bw.lo[i], dp4a_us(hi[q], c_bw.hi[i], c_bw.bias[i]));
+        b[q] = (uint32_t)(r + c_bw.neg[i] * __mulhi(r + c_bw.half[i], c_bw.inv[i]));
       }
     }
     w[i] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
@@ -282,6 +298,10 @@ long round128(long x) { return (x + 127) / 128 * 128; }
 
 }  // namespace
 
+static size_t z_bytes(long tiles) {
+  return (size_t)std::min(tiles, kPartTiles) * kNM * kTcZTile;
+}
+
 bool crt64_pays(const moao_ctx* ctx, long M, long N, long K, bool lower) {
   // Below K = 1,024 the combine step (an element of C at a time) costs about what the
   // FP64 product does: at K = 512 35 ps an element on the FP64 tensor cores, 8 + 7 ps
@@ -305,7 +325,7 @@ size_t crt64_bytes(long n, long m, long nb, long nact) {
     const size_t row = (size_t)round128(K) * kNM;
     qa = std::max(qa, std::min(kOperandBytes, row * (size_t)M));
     qb = std::max(qb, std::min(kOperandBytes / share, row * (size_t)N));
-    z = std::max(z, std::min(kZBytes, (size_t)tc_tile_count(M, N, lower) * kNM * kTcZTile));
+    z = std::max(z, z_bytes(tc_tile_count(M, N, lower)));
     small = std::max(small, sizeof(int) * (size_t)(M + N + K + kMaxChunks + 1));
   };
   const long rest = n - nb;
@@ -396,12 +416,8 @@ static moao_status make_balance(moao_ctx* ctx, const CrtBalance* bal, long K, co
   return MOAO_OK;
 }
 
-static long chunk_tiles(long total) {
-  return std::min<long>(total, (long)(kZBytes / (kNM * kTcZTile)));
-}
-
 moao_status crt64_reserve(moao_ctx* ctx, long M, long N, bool lower) {
-  return ctx->cf_z.ensure((size_t)chunk_tiles(tc_tile_count(M, N, lower)) * kNM * kTcZTile);
+  return ctx->cf_z.ensure(z_bytes(tc_tile_count(M, N, lower)));
 }
 
 moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const CrtOperand& B, long b0,
@@ -434,28 +450,27 @@ moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const Crt
   g.lower = f.lowerC ? 1 : 0;
   g.max_ctas = max_ctas;
   const long total = tc_tile_count(M, N, f.lowerC);
-  const long chunk = chunk_tiles(total);
-  const long chunks = (total + chunk - 1) / chunk;
-  if (chunks > kMaxChunks) return set_error(MOAO_ERR_UNSUPPORTED, "crt64: product too large");
-  MOAO_TRY(ctx->cf_z.ensure((size_t)chunk * kNM * kTcZTile));
-  MOAO_CUDA_TRY(cudaMemsetAsync(flag + 1, 0, sizeof(int) * (size_t)chunks, s));
+  const long part = kPartTiles, parts = (total + part - 1) / part;
+  if (parts > kMaxChunks) return set_error(MOAO_ERR_UNSUPPORTED, "crt64: product too large");
+  MOAO_TRY(ctx->cf_z.ensure(z_bytes(total)));
+  MOAO_CUDA_TRY(cudaMemsetAsync(flag + 1, 0, sizeof(int) * (size_t)parts, s));
   g.C = ctx->cf_z.p;
   TcModz z;
-  z.Z = ctx->cf_z.as<uint8_t>();
   z.M = M;
   z.N = N;
   z.lower = g.lower;
   z.bits = bits_for(A.K);
   z.ea = A.erow + a0;
   z.eb = B.erow + b0;
+  z.Z = ctx->cf_z.as<uint8_t>();
   z.alpha = f.alpha;
   z.beta = f.beta;
   z.C = f.C;
   z.ldc = f.ldc;
   z.skip_a = flag;
-  for (long c = 0; c < chunks; ++c) {
-    g.tile0 = z.tile0 = c * chunk;
-    g.tiles = z.tiles = std::min(chunk, total - c * chunk);
+  for (long c = 0; c < parts; ++c) {
+    g.tile0 = z.tile0 = c * part;
+    g.tiles = z.tiles = std::min(part, total - c * part);
     g.err = flag + 1 + c;
     z.skip_b = g.err;
     {

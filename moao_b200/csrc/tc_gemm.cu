@@ -56,6 +56,8 @@ constexpr unsigned long long kSpinLimit = 1ull << 28;  // default polls of a bou
 // its shared memory and 128 rows of the accumulator in its TMEM; the first CTA
 // of the pair issues the MMAs for both. Per SM a stage then carries 32 KB of
 // operands instead of 48 KB for the same tensor work.
+constexpr int epi_warps(int modz) { return modz ? 16 : EPI_WARPS; }
+
 template <int PAIR>
 struct TcCfg {
   static constexpr int B_ROWS = PAIR ? TBN / 2 : TBN;  // B rows held by one CTA
@@ -91,6 +93,8 @@ struct __align__(64) TcParams : TileWalk {
   // floor(2^32 / m) and the smallest multiple of m that is at least 2^31
   int nmod;
   unsigned md[kTcMaxMaps], md_inv[kTcMaxMaps], md_bias[kTcMaxMaps];
+  int md_inv38[kTcMaxMaps];  // ceil(2^38 / m), used where md_short
+  int md_short;              // K < 2^16 and every m > 128
   int tile0;               // first tile of the launch
   int items;               // tiles of the launch times nmod
   int* err;
@@ -279,6 +283,30 @@ __device__ __forceinline__ unsigned mod_of(const TcParams& p, int k, uint32_t ac
   return min(t, t - p.md[k]);
 }
 
+// A byte congruent to acc modulo m, in [0, m], for |acc| < 2^30 (K < 2^16) and
+// 129 <= m <= 256: inv = ceil(2^38 / m), so the floor of acc inv / 2^38 is the quotient
+// or, for a negative multiple of m, one less (the byte is then m, not 0; m = 256 is
+// exact).
+__device__ __forceinline__ uint32_t mod_byte(uint32_t acc, int inv, int m) {
+  return acc - (uint32_t)((__mulhi((int)acc, inv) >> 6) * m);
+}
+
+// Item v of a launch: the tile and the product (modulus) it computes. Blocks of
+// as many tiles as there are CTAs (groups) take their moduli in turn, so that all of
+// them read the same plane of the operands at a time (moduli fastest, the 148 CTAs
+// read 16 planes for 9 tiles: 1.78 against 2.43 Pop/s at M = N = 5,888, K = 16,384).
+__device__ __forceinline__ void decode_item(const TcParams& p, int v, int groups, int* tile, int* mod) {
+  if (p.nmod == 1) {
+    *tile = v;
+    *mod = 0;
+    return;
+  }
+  const int tiles = p.items / p.nmod, blk = v / (groups * p.nmod), first = blk * groups;
+  const int size = min(groups, tiles - first), w = v - first * p.nmod;
+  *mod = w / size;
+  *tile = first + w % size;
+}
+
 // Persistent warp-specialised kernel: warp 0 TMA producer, warp 1 MMA issuer,
 // warp 2 TMEM allocator, warps 4.. epilogue. The accumulator is double-buffered
 // in TMEM so the epilogue of one tile overlaps the main loop of the next. With
@@ -286,9 +314,14 @@ __device__ __forceinline__ unsigned mod_of(const TcParams& p, int k, uint32_t ac
 // of the operands (the bytes counted on the first CTA's barrier), the first
 // CTA's issuer runs the MMAs and its commits reach both CTAs, and both
 // epilogues drain their own TMEM and report to the first CTA.
-template <int PAIR>
-__global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_constant__ TcParams p) {
+// MODZ: the kTcEpiModZ epilogue alone, on 16 warps: at K = 1,024 a tile's MMAs take
+// ~5,900 cycles, in which 8 warps do not reduce its 32,768 sums.
+template <int PAIR, int MODZ>
+__global__ void __launch_bounds__((4 + epi_warps(MODZ)) * 32, 1)
+    tc_gemm_kernel(const __grid_constant__ TcParams p) {
   using Cfg = TcCfg<PAIR>;
+  constexpr int EW = epi_warps(MODZ);
+  constexpr int CW = TBN / (EW / 4);  // columns per epilogue warp
   constexpr int STAGES = Cfg::STAGES, STAGE_BYTES = Cfg::STAGE_BYTES;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
@@ -316,7 +349,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull_bar[b], 1);
-      mbar_init(&tempty_bar[b], PAIR ? 2 * EPI_WARPS : EPI_WARPS);
+      mbar_init(&tempty_bar[b], PAIR ? 2 * EW : EW);
     }
     mbar_init(drain_bar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -348,9 +381,9 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
     int it = 0;
     bool ok = true;
     for (int v = group; v < p.items && ok; v += ngroups) {
-      int mt, nt;
-      decode_tile(p, p.tile0 + v / p.nmod, &mt, &nt);
-      const int mod = v % p.nmod;  // the product: its operands are A[mod], B[mod]
+      int mt, nt, tl, mod;
+      decode_item(p, v, ngroups, &tl, &mod);  // the product's operands are A[mod], B[mod]
+      decode_tile(p, p.tile0 + tl, &mt, &nt);
       const int m0 = mt * Cfg::TILE_M + (int)crank * TBM;
       const int n0 = nt * TBN + (int)crank * Cfg::B_ROWS;
       for (int s = 0; s < p.nseg && ok; ++s) {
@@ -446,8 +479,9 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
     const uint32_t tempty0 = PAIR ? cluster_addr(smem_u32(tempty_bar), 0) : 0;
     int tc = 0;
     for (int v = group; v < p.items; v += ngroups, ++tc) {
-      int mt, nt;
-      decode_tile(p, p.tile0 + v / p.nmod, &mt, &nt);
+      int mt, nt, tl, mod;
+      decode_item(p, v, ngroups, &tl, &mod);
+      decode_tile(p, p.tile0 + tl, &mt, &nt);
       const int m0 = mt * Cfg::TILE_M + (int)crank * TBM, n0 = nt * TBN;
       const int buf = tc & 1;
       // every lane waits; the warp leaves together if any lane gave up
@@ -460,8 +494,8 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
       const bool live =
           __shfl_sync(0xffffffffu, (int)(kblocks > 0 && !*(volatile int*)p.err), 0) != 0;
       float* wscale = col_scale + (warp - 4) * 32;
-      for (int c0 = half * (TBN / 2); c0 < (half + 1) * (TBN / 2) && live; c0 += 32) {
-        if (p.epi == kTcEpiF32 && p.erow) {
+      for (int c0 = half * CW; c0 < (half + 1) * CW && live; c0 += 32) {
+        if (!MODZ && p.epi == kTcEpiF32 && p.erow) {
           // one coalesced load of the chunk's column exponents, shared by the warp
           const int c = n0 + c0 + lane;
           const int e = c < p.N ? p.ecol[c] : 0;
@@ -484,25 +518,31 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
               "=r"(v32[31])
             : "r"(taddr));
         asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        if (p.c_tma) {
+        if (!MODZ && p.c_tma) {
           // the previous chunk's reduction must have read the staging buffer
           if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");
           __syncwarp();
         }
-        if (p.epi == kTcEpiModZ) {
-          // 32 columns of this row modulo the product's modulus: two 16-byte records
-          const int mod = v % p.nmod;
+        if (MODZ) {
+          // 32 columns of this row modulo the product's modulus: four 8-byte records
+          const int zi = tl * p.nmod + mod;
           uint32_t w[8];
+          if (p.md_short) {
+            const int inv = p.md_inv38[mod], m = (int)p.md[mod];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v32[j] = mod_byte(v32[j], inv, m);
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v32[j] = mod_of(p, mod, v32[j]);
+          }
 #pragma unroll
           for (int j = 0; j < 8; ++j)
-            w[j] = __byte_perm(
-                __byte_perm(mod_of(p, mod, v32[4 * j]), mod_of(p, mod, v32[4 * j + 1]), 0x0040),
-                __byte_perm(mod_of(p, mod, v32[4 * j + 2]), mod_of(p, mod, v32[4 * j + 3]), 0x0040),
-                0x5410);
-          uint4* z = reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.C) + (size_t)v * kTcZTile) +
-                     (c0 >> 4) * TBM + q * 32 + lane;
-          z[0] = make_uint4(w[0], w[1], w[2], w[3]);
-          z[TBM] = make_uint4(w[4], w[5], w[6], w[7]);
+            w[j] = __byte_perm(__byte_perm(v32[4 * j], v32[4 * j + 1], 0x0040),
+                               __byte_perm(v32[4 * j + 2], v32[4 * j + 3], 0x0040), 0x5410);
+          uint2* z = reinterpret_cast<uint2*>(static_cast<uint8_t*>(p.C) + (size_t)zi * kTcZTile) +
+                     (c0 >> 3) * TBM + q * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) z[j * TBM] = make_uint2(w[2 * j], w[2 * j + 1]);
         } else if (r < p.M) {
           // Mask of the chunk's columns that this row writes.
           uint32_t mask = 0;
@@ -566,7 +606,7 @@ __global__ void __launch_bounds__(THREADS, 1) tc_gemm_kernel(const __grid_consta
                     old[j] + (double)p.alpha * ldexp((double)(int)v32[j], er + ec[j]);
           }
         }
-        if (p.c_tma) {
+        if (!MODZ && p.c_tma) {
           // make the staged chunk visible to the TMA unit, then one lane adds it to C
           asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
           __syncwarp();
@@ -665,12 +705,12 @@ __device__ __forceinline__ double exp2i(int e) {
   return __hiloint2double((e + 1023) << 20, 0);
 }
 
-// A block takes one 16-column group of a tile per 128 threads: a thread owns a
-// row of it, so the 16 planes are read as 16-byte records and C by coalesced
-// columns. Bound by issue (40 dp4a and about as many integer operations per
-// element), with the planes' 16 bytes per element next.
-constexpr int kCombThreads = 256;
-__global__ void __launch_bounds__(kCombThreads)
+// A block takes one 8-column group of a tile: a thread owns a row of it, so the 16
+// planes are read as 8-byte records and C by coalesced columns. Bound by issue (40
+// dp4a and about as many integer operations per element), with the planes' 16 bytes
+// per element next.
+constexpr int kCombThreads = 128;
+__global__ void __launch_bounds__(kCombThreads, 6)
     modz_combine_kernel(const __grid_constant__ TileWalk walk, int tile0, const uint8_t* __restrict__ Z,
                         int M, int N, int bits, const int* __restrict__ ea,
                         const int* __restrict__ eb, double alpha, double beta,
@@ -678,19 +718,18 @@ __global__ void __launch_bounds__(kCombThreads)
   if (*skip_a || *skip_b) return;
   int mt, nt;
   decode_tile(walk, tile0 + (int)blockIdx.x, &mt, &nt);
-  const int row = threadIdx.x & (TBM - 1);
-  const int grp = blockIdx.y * (kCombThreads / TBM) + threadIdx.x / TBM;
-  const int r = mt * TBM + row, c0 = nt * TBN + grp * 16;
+  const int row = threadIdx.x, grp = blockIdx.y;
+  const int r = mt * TBM + row, c0 = nt * TBN + grp * 8;
   if (r >= M || c0 >= N || (walk.lower && r < c0)) return;
-  const uint4* z = reinterpret_cast<const uint4*>(Z + (size_t)blockIdx.x * kCrt64Moduli * kTcZTile) +
+  const uint2* z = reinterpret_cast<const uint2*>(Z + (size_t)blockIdx.x * kCrt64Moduli * kTcZTile) +
                    grp * TBM + row;
-  uint4 pl[kCrt64Moduli];
+  uint2 pl[kCrt64Moduli];
 #pragma unroll
-  for (int i = 0; i < kCrt64Moduli; ++i) pl[i] = __ldcs(z + i * (kTcZTile / 16));
+  for (int i = 0; i < kCrt64Moduli; ++i) pl[i] = __ldcs(z + i * (kTcZTile / 8));
   constexpr ModProduct mp = mod_product();
   const double er = exp2i(exp_of_row(ea[r]) - bits);
 #pragma unroll
-  for (int q = 0; q < 4; ++q) {
+  for (int q = 0; q < 2; ++q) {
     double old[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -704,8 +743,7 @@ __global__ void __launch_bounds__(kCombThreads)
       uint32_t w[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint4 v = pl[4 * g + i];
-        w[i] = q == 0 ? v.x : (q == 1 ? v.y : (q == 2 ? v.z : v.w));
+        w[i] = q == 0 ? pl[4 * g + i].x : pl[4 * g + i].y;
       }
       const uint32_t a = __byte_perm(w[0], w[1], 0x5140), b = __byte_perm(w[2], w[3], 0x5140);
       const uint32_t c = __byte_perm(w[0], w[1], 0x7362), d = __byte_perm(w[2], w[3], 0x7362);
@@ -858,11 +896,14 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
   p.nmod = 1;
   if (modz || g.epi == kTcEpiMod8) {
     p.nmod = modz ? g.nmod : 1;
+    p.md_short = modz && (long)g.seg[0].nk * kstep < (1L << 16);
     for (int i = 0; i < p.nmod; ++i) {
       const unsigned m = (unsigned)(modz ? g.moduli[i] : g.modulus);
       p.md[i] = m;
       p.md_inv[i] = (unsigned)((1ull << 32) / m);
       p.md_bias[i] = (unsigned)(((1ull << 31) + m - 1) / m * m);
+      p.md_inv38[i] = m > 128 ? (int)(((1ull << 38) + m - 1) / m) : 0;
+      if (m <= 128) p.md_short = 0;
     }
   }
   p.tile0 = modz ? (int)g.tile0 : 0;
@@ -897,13 +938,19 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
   }
   if (!pair) {
     static std::atomic<unsigned long long> configured{0};
-    MOAO_CUDA_TRY(set_smem_limit(tc_gemm_kernel<0>, (int)TcCfg<0>::SMEM, configured));
+    MOAO_CUDA_TRY(set_smem_limit(tc_gemm_kernel<0, 0>, (int)TcCfg<0>::SMEM, configured));
     const long ctas =
         std::min<long>(items, g.max_ctas > 0 ? std::min(g.max_ctas, num_sms) : num_sms);
-    tc_gemm_kernel<0><<<(unsigned)ctas, THREADS, TcCfg<0>::SMEM, s>>>(p);
+    if (modz) {
+      static std::atomic<unsigned long long> configured_z{0};
+      MOAO_CUDA_TRY(set_smem_limit(tc_gemm_kernel<0, 1>, (int)TcCfg<0>::SMEM, configured_z));
+      tc_gemm_kernel<0, 1><<<(unsigned)ctas, (4 + epi_warps(1)) * 32, TcCfg<0>::SMEM, s>>>(p);
+    } else {
+      tc_gemm_kernel<0, 0><<<(unsigned)ctas, THREADS, TcCfg<0>::SMEM, s>>>(p);
+    }
   } else {
     static std::atomic<unsigned long long> configured{0};
-    MOAO_CUDA_TRY(set_smem_limit(tc_gemm_kernel<1>, (int)TcCfg<1>::SMEM, configured));
+    MOAO_CUDA_TRY(set_smem_limit(tc_gemm_kernel<1, 0>, (int)TcCfg<1>::SMEM, configured));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -923,14 +970,14 @@ moao_status tc_gemm(const TcGemm& g, cudaStream_t s, long long* launches) {
     int groups = dev < 64 ? resident[dev].load() : 0;
     if (groups <= 0) {
       cfg.gridDim = dim3((unsigned)(num_sms & ~1));
-      MOAO_CUDA_TRY(cudaOccupancyMaxActiveClusters(&groups, tc_gemm_kernel<1>, &cfg));
+      MOAO_CUDA_TRY(cudaOccupancyMaxActiveClusters(&groups, tc_gemm_kernel<1, 0>, &cfg));
       if (groups <= 0) groups = num_sms / 2;
       if (dev < 64) resident[dev].store(groups);
     }
     if (g.max_ctas > 0) groups = std::min(groups, g.max_ctas / 2);
     groups = (int)std::min<long>(groups, items);
     cfg.gridDim = dim3((unsigned)(2 * groups));
-    MOAO_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_gemm_kernel<1>, p));
+    MOAO_CUDA_TRY(cudaLaunchKernelEx(&cfg, tc_gemm_kernel<1, 0>, p));
   }
   if (launches) ++*launches;
   MOAO_CUDA_TRY(cudaGetLastError());
@@ -942,7 +989,7 @@ moao_status tc_modz_combine(const TcModz& z, cudaStream_t s, long long* launches
   const long total = fill_walk(&w, z.M, z.N, z.lower, 0, TBM);
   const long run = z.tiles > 0 ? std::min(z.tiles, total - z.tile0) : total - z.tile0;
   if (run <= 0) return MOAO_OK;
-  const dim3 grid((unsigned)run, TBN / 16 / (kCombThreads / TBM));
+  const dim3 grid((unsigned)run, TBN / 8);
   modz_combine_kernel<<<grid, kCombThreads, 0, s>>>(w, (int)z.tile0, z.Z, (int)z.M, (int)z.N, z.bits,
                                                     z.ea, z.eb, z.alpha, z.beta, z.C, z.ldc,
                                                     z.skip_a, z.skip_b);

@@ -26,8 +26,8 @@ enum TcEpilogue { kTcEpiF32 = 0, kTcEpiF64Scaled = 1, kTcEpiMod8 = 2, kTcEpiModZ
 // kTcEpiMod8 (int8 operands): C (uint8, column-major) = acc mod modulus, in [0, modulus).
 // kTcEpiModZ (int8 operands): nmod products in one launch, the i-th A[i] B[i]^T
 // modulo moduli[i], into 128 x 256-tile blocks for tc_modz_combine: tile t of the
-// launch holds nmod planes of 32 KB, each 16 groups of 16 columns, a group one
-// 16-byte record per row.
+// launch holds nmod planes of 32 KB, each 32 groups of 8 columns, a group one
+// 8-byte record per row.
 constexpr long kTcZTile = 128 * 256;  // bytes per tile and modulus
 
 // A K-major operand: rows x kcols elements, row stride in elements.

@@ -15,6 +15,7 @@
 #include <cstdint>
 #include <cstdlib>
 
+#include "chain.cuh"
 #include "dense.h"
 #include "leaf_f64.cuh"
 #include "tile_walk.cuh"
@@ -110,35 +111,6 @@ struct KParams {
   // the column tiles in turn, the band's row tiles fastest
   int tiles_m, tiles_n, group_m;
 };
-
-// Chained launches (programmatic dependent launch): a kernel launched with
-// launch_chained may start while its predecessor in the stream still runs; it lets
-// its own successor start as early, and waits here until the predecessor has
-// finished and its writes are visible. Every thread of a chained kernel calls this
-// before it touches memory, so completion orders along the chain as in a plain
-// stream. Without the launch attribute both instructions do nothing. A diagonal
-// block of 1,024 columns is a chain of about 90 short launches; with the 32 x 32
-// tiles, an nmeas 640 FP64 reconstructor takes 507 us instead of 952.
-__device__ __forceinline__ void chain_wait() {
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  asm volatile("griddepcontrol.wait;\n" ::: "memory");
-}
-
-template <typename... P, typename... A>
-cudaError_t launch_chained(bool chained, void (*kern)(P...), dim3 grid, dim3 block, size_t smem,
-                           cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = chained ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
-}
 
 // Tile v of the launch in band order. Consecutive CTAs share one column strip
 // of B and the band's row strips of A stay in L2 while the band sweeps the

@@ -1,12 +1,12 @@
 // 2-D complex FFT (FP64) as row transforms, a transpose, row transforms and a
-// transpose back. A row transform is one CTA of N/2 threads: the row is read
-// into shared memory in bit-reversed order, then log2(N) radix-2
-// decimation-in-time stages run with one butterfly per thread and a barrier
-// between stages (Cooley-Tukey). Twiddles come from a table computed on the
-// host in long double, so every factor is the correctly rounded double of
-// exp(-2 pi i k / N). The transposes move 32 x 32 tiles through shared memory
-// so that reads and writes are both coalesced.
+// transpose back. A row transform is one CTA (fft_row.cuh): the row is read into
+// shared memory in bit-reversed order, then log2(N) radix-2 decimation-in-time stages
+// run, three at a time in registers (Cooley-Tukey). Twiddles come from a table
+// computed on the host in long double, so every factor is the correctly rounded
+// double of exp(-2 pi i k / N). The transposes move 32 x 32 tiles through shared
+// memory so that reads and writes are both coalesced.
 #include "fft.h"
+#include "fft_row.cuh"
 
 #include <cmath>
 #include <vector>
@@ -14,28 +14,13 @@
 namespace moao {
 namespace {
 
-__device__ __forceinline__ unsigned bitrev(unsigned v, int bits) { return __brev(v) >> (32 - bits); }
-
 __global__ void fft_rows_kernel(Cplx* __restrict__ data, int N, int logN,
                                 const Cplx* __restrict__ tw, int dir) {
   extern __shared__ Cplx row[];
   Cplx* g = data + (long)blockIdx.x * N;
-  for (int c = threadIdx.x; c < N; c += blockDim.x) row[bitrev((unsigned)c, logN)] = g[c];
-  __syncthreads();
-  const int t = threadIdx.x;  // one butterfly per thread and stage (N / 2 threads)
-  for (int s = 0; s < logN; ++s) {
-    const int half = 1 << s;
-    const int pos = t & (half - 1);
-    const int i0 = ((t >> s) << (s + 1)) + pos, i1 = i0 + half;
-    Cplx w = tw[pos << (logN - 1 - s)];
-    if (dir > 0) w.y = -w.y;
-    const Cplx u = row[i0], v = row[i1];
-    const Cplx vw = {v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x};
-    row[i0] = {u.x + vw.x, u.y + vw.y};
-    row[i1] = {u.x - vw.x, u.y - vw.y};
-    __syncthreads();
-  }
-  for (int c = threadIdx.x; c < N; c += blockDim.x) g[c] = row[c];
+  for (int c = threadIdx.x; c < N; c += blockDim.x) row[fft_place(c, logN)] = g[c];
+  fft_row(row, logN, tw, dir);
+  for (int c = threadIdx.x; c < N; c += blockDim.x) g[c] = row[fft_at(c)];
 }
 
 // dst[c * N + r] = src[r * N + c]
@@ -87,11 +72,12 @@ void fft2d_free(Fft2d* f) {
 moao_status fft2d(const Fft2d& f, Cplx* data, int dir, cudaStream_t s, long long* launches) {
   const int N = (int)f.N;
   if (N < 2 || !f.tw || !f.tmp) return set_error(MOAO_ERR_BAD_ARG, "fft2d: no plan");
-  const size_t smem = sizeof(Cplx) * N;
+  const size_t smem = fft_smem(N);
+  const int threads = fft_threads(N);
   const dim3 tgrid((N + 31) / 32, (N + 31) / 32), tblock(32, 8);
-  fft_rows_kernel<<<N, N / 2, smem, s>>>(data, N, f.logN, f.tw, dir);
+  fft_rows_kernel<<<N, threads, smem, s>>>(data, N, f.logN, f.tw, dir);
   transpose_kernel<<<tgrid, tblock, 0, s>>>(data, f.tmp, N);
-  fft_rows_kernel<<<N, N / 2, smem, s>>>(f.tmp, N, f.logN, f.tw, dir);
+  fft_rows_kernel<<<N, threads, smem, s>>>(f.tmp, N, f.logN, f.tw, dir);
   transpose_kernel<<<tgrid, tblock, 0, s>>>(f.tmp, data, N);
   if (launches) *launches += 4;
   MOAO_CUDA_TRY(cudaGetLastError());

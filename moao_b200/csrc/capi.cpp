@@ -180,6 +180,15 @@ moao_status device_geometry(moao_ctx* ctx, const moao_tomo* tp, const DevGeometr
   g.u = d + ou; g.v = d + ov; g.X = d + oX; g.Y = d + oY;
   g.noiseLGSxx = d + oxx; g.noiseLGSyy = d + oyy; g.noiseLGSxy = d + oxy;
   g.noiseNGS = d + ongs; g.layer = d + olay;
+  if (!ctx->dphi.p) {  // once per context
+    MOAO_TRY(ctx->dphi.ensure(sizeof(DphiRow) * kDphiRows));
+    cudaError_t st = cudaMemcpyAsync(ctx->dphi.p, dphi_table(), sizeof(DphiRow) * kDphiRows,
+                                     cudaMemcpyHostToDevice, ctx->stream);
+    if (st == cudaSuccess) st = cudaStreamSynchronize(ctx->stream);
+    if (st != cudaSuccess) ctx->dphi.release();
+    MOAO_CUDA_TRY(st);
+  }
+  g.dphi = ctx->dphi.as<DphiRow>();
   {
     KernelTimer kt(ctx, "matcov_table", (double)ntab / 4);
     MOAO_TRY(build_toeplitz_tables(g, ctx->stream, &ctx->launches));
@@ -393,6 +402,7 @@ void moao_ctx_destroy(moao_ctx* c) {
   cudaStreamSynchronize(c->stream);
   for (auto& kv : c->geom) kv.second.buf.release();
   for (moao::DevBuf* b : c->workspaces()) b->release();
+  c->dphi.release();
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   for (auto& p : c->pending) {
@@ -648,7 +658,7 @@ moao_status moao_matcov_tile(moao_ctx* ctx, const moao_tomo* t, double* d_data, 
   if (type_mat == 1 && xoffset == yoffset && nrows == ncols) elems = 0.5 * nrows * (nrows + 1.0);
   KernelTimer kt(ctx, "matcov", elems);
   return launch_matcov(*g, d_data, nrows, ncols, xoffset, yoffset, lda, type_mat, ctx->stream,
-                       &ctx->launches);
+                       &ctx->launches, ctx->chained);
 }
 
 namespace {

@@ -56,6 +56,7 @@ struct moao_ctx {
   bool graph_mode = false;  // mixed path under stream capture: no host waits or reads
   std::mutex mu;
   std::map<const moao_tomo*, moao::GeomEntry> geom;
+  moao::DevBuf dphi;  // structure-function table (dphi_table), uploaded once
   moao::DevBuf ws_w, ws_dinv, ws_info, ws_tmp, ws_host_t, ws_corner;
   // mixed-precision workspace
   moao::DevBuf mx_a32, mx_lr, mx_lc, mx_t32, mx_w1, mx_w2, mx_x, mx_r64, mx_e64, mx_qa, mx_qb,

@@ -15,15 +15,18 @@
 // four covariances. When the two WFS have the same subaperture size on a layer
 // (every NGS/NGS and equal-altitude LGS/LGS pair) the 16 stencil points of the
 // block collapse to 9 distinct DPHI evaluations. Per-layer constants
-// (2 pi / L0, k1 L0^(5/3), 0.5 kk cn2) are hoisted to shared memory. The
-// kernel is bound by FP64 pipe throughput (cbrt / exp / an 11-term polynomial
-// per DPHI), not by HBM: each 8-byte store costs ~10^3 FP64 operations.
+// (2 pi / L0, k1 L0^(5/3), 0.5 kk cn2) are hoisted to shared memory. Pairs of equal
+// projection gather from tables over grid offsets, edge-aligned ones share their
+// points in matcov_edge_kernel, and f itself comes from a table of polynomials
+// (dphi_v): its 40 to 55 FP64 operations bounded the direct form, reads of the
+// table bound this one.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
+#include "chain.cuh"
 #include "moao_internal.h"
 
 namespace moao {
@@ -129,8 +132,82 @@ __device__ __forceinline__ double dphi_unit_s_inl(double s) {
 
 __device__ __noinline__ double dphi_unit_s(double s) { return dphi_unit_s_inl(s); }
 
-__device__ __forceinline__ double D(double x, double y, double tpl) {
-  return dphi_unit_s((tpl * tpl) * (x * x + y * y));
+// The same function of v = s / Xlim^2 from the table: kDphiSub intervals per octave
+// from v's leading bits (the two forms of f meet at v = 1, an interval's edge), then
+// a polynomial of degree 8 in the distance y from the interval's middle, against ~40
+// FP64 operations of the series and ~55 of the asymptotic form with exp. The
+// polynomials interpolate f, evaluated in 80-bit arithmetic, at Chebyshev nodes: an
+// interval's half width is at most v / 32 and f's nearest singularity is v = 0, so the
+// truncation is below 92^-9 of f. The terms y^5 and up are at most 3e-10 of f, so
+// their FP32 coefficients and evaluation are good to 2e-17 of it. Outside the table
+// (separations of a few centimetres, or where f is within 2e-16 of its limit) the
+// direct form.
+//
+// What bounds it is shared-memory reads: 56 bytes a value. The table is held in
+// copies, one per lane of a load's phase (8 lanes of 16 bytes, 16 of 8), each in banks
+// of its own, so that lanes on different rows never conflict: 14 wavefronts a warp.
+// One copy (degree 5, 64 intervals per octave, 48 bytes a value) took 21 in conflicts
+// and 7.2 against 5.5 ms for the Ctm of nmeas 15,936; in L1 7.4 ms.
+constexpr int kTab01 = 0, kTab23 = kTab01 + kDphiRows * 8 * 16, kTabF = kTab23 + kDphiRows * 8 * 16,
+              kTab4 = kTabF + kDphiRows * 8 * 16, kTabBytes = kTab4 + kDphiRows * 16 * 8;
+
+template <int THREADS>
+__device__ __forceinline__ void dphi_fill(char* tab, const DphiRow* __restrict__ rows) {
+  constexpr int PER = kDphiRows * 16 / THREADS;
+  static_assert(PER * THREADS == kDphiRows * 16, "copies per thread");
+  DphiRow r[PER];  // every row's loads in flight together
+#pragma unroll
+  for (int u = 0; u < PER; ++u) r[u] = rows[(threadIdx.x + u * THREADS) >> 4];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int q = threadIdx.x + u * THREADS, k = q >> 4, p = q & 15;
+    reinterpret_cast<double*>(tab + kTab4)[q] = r[u].c[4];
+    if (p < 8) {
+      reinterpret_cast<double2*>(tab + kTab01)[k * 8 + p] = make_double2(r[u].c[0], r[u].c[1]);
+      reinterpret_cast<double2*>(tab + kTab23)[k * 8 + p] = make_double2(r[u].c[2], r[u].c[3]);
+    } else {
+      reinterpret_cast<float4*>(tab + kTabF)[k * 8 + p - 8] =
+          make_float4(r[u].f[0], r[u].f[1], r[u].f[2], r[u].f[3]);
+    }
+  }
+}
+
+__device__ __noinline__ double dphi_outside(double v) { return dphi_unit_s_inl(v * kXlim2); }
+
+__device__ __forceinline__ double dphi_v(const char* tab, double v) {
+  const int hi = __double2hiint(v), lane = threadIdx.x & 31;
+  const unsigned k = (unsigned)((hi >> 16) - ((1023 + kDphiLo) << 4));
+  if (k >= (unsigned)kDphiRows) return dphi_outside(v);
+  const double y = v - __hiloint2double((hi & 0xffff0000) | 0x8000, 0);
+  const char* t = tab + (k * 8 + (lane & 7)) * 16;
+  const float4 f = *reinterpret_cast<const float4*>(t + kTabF);
+  const double2 c0 = *reinterpret_cast<const double2*>(t + kTab01);
+  const double2 c2 = *reinterpret_cast<const double2*>(t + kTab23);
+  const double c4 = *reinterpret_cast<const double*>(tab + kTab4 + (k * 16 + (lane & 15)) * 8);
+  const float yf = (float)y;
+  const float ph = fmaf(fmaf(fmaf(f.w, yf, f.z), yf, f.y), yf, f.x);
+  double p = fma((double)ph, y, c4);
+  p = fma(p, y, c2.y);
+  p = fma(p, y, c2.x);
+  p = fma(p, y, c0.y);
+  return fma(p, y, c0.x);
+}
+
+// The same from the rows in global memory (the per-pair and table kernels; not
+// inlined, so that their 9 or 16 points per layer share one body).
+__device__ __noinline__ double dphi_row(const DphiRow* __restrict__ rows, double v) {
+  const int hi = __double2hiint(v);
+  const unsigned k = (unsigned)((hi >> 16) - ((1023 + kDphiLo) << 4));
+  if (k >= (unsigned)kDphiRows) return dphi_outside(v);
+  const double y = v - __hiloint2double((hi & 0xffff0000) | 0x8000, 0);
+  const DphiRow& r = rows[k];
+  const float yf = (float)y;
+  const float ph = fmaf(fmaf(fmaf(r.f[3], yf, r.f[2]), yf, r.f[1]), yf, r.f[0]);
+  double p = fma((double)ph, y, r.c[4]);
+  p = fma(p, y, r.c[3]);
+  p = fma(p, y, r.c[2]);
+  p = fma(p, y, r.c[1]);
+  return fma(p, y, r.c[0]);
 }
 
 constexpr int kMaxJobs = 160;
@@ -160,6 +237,7 @@ __global__ void __launch_bounds__(kTileI* kTileJ)
   __shared__ double s_tpl[kMaxLayers], s_amp[kMaxLayers], s_w[kMaxLayers];
   __shared__ double s_sm[kMaxLayers], s_sn[kMaxLayers];
   __shared__ int s_job;
+  chain_wait();
 
   if (threadIdx.x == 0 && threadIdx.y == 0) {
     int k = 0;
@@ -221,40 +299,41 @@ __global__ void __launch_bounds__(kTileI* kTileJ)
     const double du = __ldg(ul + pi) - __ldg(ul + pj);
     const double dv = __ldg(vl + pi) - __ldg(vl + pj);
     const double s1 = sml * 0.5, s2 = snl * 0.5;
-    const double tpl = s_tpl[l];
+    const double t2 = s_tpl[l] * s_tpl[l] * (1.0 / kXlim2);
     const double w = s_w[l] * s_amp[l];
+    auto D = [&](double x, double y) { return dphi_row(g.dphi, t2 * (x * x + y * y)); };
     if (s1 == s2) {
       // Equal subaperture sizes: ac = 0, ad = 2 s; XY and YX share 4 points.
       const double ad = s1 + s2;
-      const double d0 = (mask & 9u) ? D(du, dv, tpl) : 0.0;
+      const double d0 = (mask & 9u) ? D(du, dv) : 0.0;
       if (mask & 1u) {
-        const double xx = -d0 + D(du + ad, dv, tpl) + D(du - ad, dv, tpl) - d0;
+        const double xx = -d0 + D(du + ad, dv) + D(du - ad, dv) - d0;
         cxx += xx * w;
       }
       if (mask & 8u) {
-        const double yy = -d0 + D(du, dv + ad, tpl) + D(du, dv - ad, tpl) - d0;
+        const double yy = -d0 + D(du, dv + ad) + D(du, dv - ad) - d0;
         cyy += yy * w;
       }
       if (mask & 6u) {
-        const double pp = D(du + s1, dv + s2, tpl), pm = D(du + s1, dv - s2, tpl);
-        const double mp = D(du - s1, dv + s2, tpl), mm = D(du - s1, dv - s2, tpl);
+        const double pp = D(du + s1, dv + s2), pm = D(du + s1, dv - s2);
+        const double mp = D(du - s1, dv + s2), mm = D(du - s1, dv - s2);
         cxy += (-pm + pp + mm - mp) * w;
         cyx += (-mp + pp + mm - pm) * w;
       }
     } else {
       const double ac = s1 - s2, ad = s1 + s2, bc = -ad, bd = -ac;
       if (mask & 1u)
-        cxx += (-D(du + ac, dv, tpl) + D(du + ad, dv, tpl) + D(du + bc, dv, tpl) -
-                D(du + bd, dv, tpl)) * w;
+        cxx += (-D(du + ac, dv) + D(du + ad, dv) + D(du + bc, dv) -
+                D(du + bd, dv)) * w;
       if (mask & 8u)
-        cyy += (-D(du, dv + ac, tpl) + D(du, dv + ad, tpl) + D(du, dv + bc, tpl) -
-                D(du, dv + bd, tpl)) * w;
+        cyy += (-D(du, dv + ac) + D(du, dv + ad) + D(du, dv + bc) -
+                D(du, dv + bd)) * w;
       if (mask & 2u)
-        cxy += (-D(du + s1, dv - s2, tpl) + D(du + s1, dv + s2, tpl) +
-                D(du - s1, dv - s2, tpl) - D(du - s1, dv + s2, tpl)) * w;
+        cxy += (-D(du + s1, dv - s2) + D(du + s1, dv + s2) +
+                D(du - s1, dv - s2) - D(du - s1, dv + s2)) * w;
       if (mask & 4u)
-        cyx += (-D(du - s2, dv + s1, tpl) + D(du + s2, dv + s1, tpl) +
-                D(du - s2, dv - s1, tpl) - D(du + s2, dv - s1, tpl)) * w;
+        cyx += (-D(du - s2, dv + s1) + D(du + s2, dv + s1) +
+                D(du - s2, dv - s1) - D(du + s2, dv - s1)) * w;
     }
   }
 
@@ -296,37 +375,37 @@ __global__ void __launch_bounds__(kTileI* kTileJ)
 // evaluate DPHI at (edge or centre of i) - (edge or centre of j): XX at
 // (x-edges, y-centres), YY at (x-centres, y-edges), XY at (x-edge of i minus
 // x-centre of j, y-centre of i minus y-edge of j), YX the reverse. A block
-// handles a 4x4-cell tile of WFS m against an 8x8-cell tile of WFS n: it
-// evaluates the 4 x 1,440 distinct points of a layer once into shared memory
-// and each of its 1,024 pairs gathers its 16 values, 5.6 evaluations per pair
-// instead of 16.
+// handles a 4x4-cell tile of WFS m against an 8x8-cell tile of WFS n: 4 x 1,440
+// distinct points for its 1,024 pairs, 5.6 evaluations per pair instead of 16.
 //
-// Each covariance's points form an outer sum s = a[r] + b[c] of two short
-// arrays of scaled squared 1-D separations (x part and y part), so a layer
-// first fills the 306 entries of those arrays and each point then costs one
-// addition before DPHI. Point tables are row-major [r][c]; the i-cell indices
-// (a = column, b = row of the i tile) enter rows and columns with strides that
-// map the 16 lanes of a half-warp (a, b in 0..3) onto 16 distinct banks, and
-// every stencil value of a pair sits at a compile-time offset from one of
-// three per-thread bases:
-//   XX [ix = 5 ej + ei][iy = 4 rj + ri]      stride 36, base A = (5c + a) 36 + 4e + b
-//   YY [iy = 5 fj + fi][ix = 4 cj + ci]      stride 36, base Y = (5e + b) 36 + 4c + a
-//   XY [ix = 5 cj + ei][iy = 4 fj + ri]      stride 36, base A
-//   YX [ix = 4 ej + ci][iy = 5 rj + fi]      stride 44, base X = (4c + a) 44 + 5e + b
-// (e* edge, c* centre index along x; f* edge, r* centre index along y; i
-// indices run over the 4x4 tile, j indices over the 8x8 tile.)
+// A warp takes one covariance. A lane holds the two indices that are centres fixed
+// (one of the i tile, one of the j tile) and walks the 9 x 5 edges of the other two,
+// forming the stencil from the last two edges in registers, where the 32
+// covariances of its (edge-walked) cells accumulate over the layers: no point
+// passes through shared memory. With cells i = (a, b) and j = (c, e), columns and
+// rows of the two tiles, and u the 5 i-edges, v the 9 j-edges:
+//   XX  lane (b, e)  x = (u edge of a) - (v edge of c),   y = centres b - e
+//   YY  lane (a, c)  y = (u edge of b) - (v edge of e),   x = centres a - c
+//   XY  lane (b, c)  x = (u edge of a) - centre c,        y = centre b - (v edge of e)
+//   YX  lane (a, e)  y = (u edge of b) - centre e,        x = centre a - (v edge of c)
+// so s = S(u, v) + const for XX and YY (S: 45 values a layer, shared by the lanes)
+// and s = U(u) + V(v) for XY and YX.
 constexpr int kEA = 4, kEB = 8;                              // cells per tile side
-constexpr int kEThreads = 256;
-constexpr int kEPairs = kEA * kEA * kEB * kEB / kEThreads;   // pairs per thread (4)
-constexpr int kEKind = (kEA + 1) * kEA * (kEB + 1) * kEB;    // points per covariance (1,440)
-constexpr int kEOffYY = 45 * 36, kEOffXY = kEOffYY + 45 * 36, kEOffYX = kEOffXY + 40 * 36;
-constexpr int kEPtsTotal = kEOffYX + 36 * 44;                // 6,264 doubles
-// scaled squared separations: row array then column array of each covariance
-constexpr int kESqXXr = 0, kESqXXc = 45, kESqYYr = 77, kESqYYc = 122, kESqXYr = 154,
-              kESqXYc = 194, kESqYXr = 230, kESqYXc = 266, kESqTotal = 306;
-constexpr size_t kESmem = (size_t)(kEPtsTotal + kESqTotal) * sizeof(double);
-static_assert(kEKind == 45 * 32 && kEKind == 40 * 36 && kEKind % 32 == 0,
-              "a covariance's points must fill whole warps");
+constexpr int kEWarps = 16;                                  // per CTA, one CTA per SM
+constexpr int kEU = kEA + 1, kEV = kEB + 1;                  // edges per tile side
+constexpr int kECoord = 2 * (kEU + kEV);                     // centres: xm ym xn yn
+constexpr int kEPairs = kEA * kEA * kEB * kEB;               // 1,024
+static_assert(kEA * kEB == 32 && kECoord <= 32, "a lane per pair of fixed indices and per centre");
+// Shared memory: the structure-function table, then per warp half of the staged
+// output, the layer's centres, S, and the valid indices of the two tiles' cells.
+constexpr int kEWarpDoubles = kEPairs / 2 + kECoord + kEU * kEV + (kEA * kEA + kEB * kEB) / 2 + 1;
+constexpr size_t kESmem = (size_t)kTabBytes + kEWarps * kEWarpDoubles * sizeof(double);
+static_assert(kESmem <= 232448, "shared memory per CTA");
+// XX and YY: the lanes' (i, j) fixed indices in order of j - i, so that the eight lanes
+// of a 16-byte shared load's phase hold close separations and read few table rows.
+__constant__ unsigned char c_edge_lane[32] = {
+    3, 2, 7, 1, 6, 11, 0, 5, 10, 15, 4, 9, 14, 19, 8, 13, 18, 23, 12, 17, 22, 27,
+    16, 21, 26, 31, 20, 25, 30, 24, 29, 28};  // i + 4 j
 
 struct EdgeJob {
   int m, n;        // row WFS, column WFS
@@ -351,64 +430,89 @@ __device__ __forceinline__ double grid_centre(const DevGeometry& g, int c, doubl
   return (x + pup) * rr + shift;
 }
 
-template <typename OutT>
-__global__ void __launch_bounds__(kEThreads, 3)
-    matcov_edge_kernel(const __grid_constant__ EdgeLaunch d, const DevGeometry g,
-                       OutT* __restrict__ out) {
-  extern __shared__ double esm[];
-  double* pts = esm;                 // XX | YY | XY | YX point tables of the current layer
-  double* sq = esm + kEPtsTotal;     // the 8 separation arrays
-  __shared__ int s_job;
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    int k = 0;
-    while (k + 1 < d.njobs && d.jobs[k + 1].tile_base <= (int)blockIdx.x) ++k;
-    s_job = k;
+// Accumulates the 8 x 4 covariances of a lane over one layer. S: kEV x kEU shared
+// values (UNIFORM), or u_sep[5] of the lane and its v coordinate against the edges
+// ve[v] (v_sep = t2 (vc - ve[v])^2).
+template <bool UNIFORM>
+__device__ __forceinline__ void edge_layer(const char* tab, const double* S, double c0,
+                                           const double (&u_sep)[kEU], double vc, const double* ve,
+                                           double t2, double w, double (&acc)[kEB][kEA]) {
+  double prev[kEU];
+#pragma unroll
+  for (int v = 0; v < kEV; ++v) {
+    double cur[kEU];
+    double b = c0;
+    if (!UNIFORM) {
+      const double d = vc - ve[v];
+      b = t2 * (d * d);
+    }
+#pragma unroll
+    for (int u = 0; u < kEU; ++u)
+      cur[u] = dphi_v(tab, UNIFORM ? S[v * kEU + u] + b : u_sep[u] + b);
+    // the reference's stencil (cov_XX/YY/XY/YX, matcov_kernels.cpp:147-193): right and
+    // top edges are index + 1, left and bottom edges index + 0
+    if (v > 0) {
+#pragma unroll
+      for (int u = 0; u < kEA; ++u)
+        acc[v - 1][u] = fma(((-cur[u + 1] + prev[u + 1]) + cur[u]) - prev[u], w, acc[v - 1][u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kEU; ++u) prev[u] = cur[u];
   }
-  __syncthreads();
-  const EdgeJob& jb = d.jobs[s_job];
-  const int t = blockIdx.x - jb.tile_base;
+}
+
+// Item v: tile pair v / 4 and covariance v % 4, by one warp; wsm is the warp's shared
+// memory.
+template <typename OutT>
+__device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry& g,
+                                          OutT* __restrict__ out, const char* tab, double* wsm,
+                                          int v_item) {
+  const int lane = threadIdx.x & 31, kind = v_item & 3, tile = v_item >> 2;
+  double* o = wsm;                       // [32 j cells][i cell]
+  double* co = o + kEPairs / 2;              // centres of the current layer
+  double* S = co + kECoord;
+  int* s_vi = reinterpret_cast<int*>(S + kEU * kEV + 1);
+  int* s_vj = s_vi + kEA * kEA;
+  int job = 0;
+  while (job + 1 < d.njobs && d.jobs[job + 1].tile_base <= tile) ++job;
+  const EdgeJob& jb = d.jobs[job];
+  const int t = tile - jb.tile_base;
   const int ta = t % g.ntiles_a, tb = t / g.ntiles_a;
   const int ci0 = g.tiles_a[2 * ta], ri0 = g.tiles_a[2 * ta + 1];
   const int cj0 = g.tiles_b[2 * tb], rj0 = g.tiles_b[2 * tb + 1];
   const int N = g.nssp_grid, m = jb.m, n = jb.n;
   const int Nm = g.Nsubap[m], Nn = g.Nsubap[n];
-
-  // this thread's pairs: i cell (a, b) = tid % 16 of the 4x4 tile, j cells
-  // (c, e + 2 q) of the 8x8 tile with c = tid / 16 % 8, e = tid / 128
-  const int a = tid % kEA, b = tid / kEA % kEA;
-  const int c = tid / (kEA * kEA) % kEB, e = tid / (kEA * kEA * kEB);
-  const int ci = ci0 + a, ri = ri0 + b;
-  const int vi = (ci < N && ri < N) ? g.cell_idx[ri * N + ci] : -1;
+  __syncwarp();
+  for (int q = lane; q < kEA * kEA + kEB * kEB; q += 32) {
+    const bool of_i = q < kEA * kEA;
+    const int k = of_i ? q : q - kEA * kEA, side = of_i ? kEA : kEB;
+    const int c = (of_i ? ci0 : cj0) + k % side, r = (of_i ? ri0 : rj0) + k / side;
+    s_vi[q] = (c < N && r < N) ? g.cell_idx[r * N + c] : -1;  // s_vj follows s_vi
+  }
+  __syncwarp();
+  // rows and columns of pair (i, j) in this covariance (slope bit 1: y of i, bit 0: of j)
+  const int slope = kind == 0 ? 0 : (kind == 1 ? 3 : kind - 1);  // XX YY XY YX
   const int r1 = d.r0 + d.nrows, c1 = d.c0 + d.ncols;
   const bool lower = (d.type == 1 || d.type == 5);
-  auto want = [&](int r, int cc) {
-    return r >= d.r0 && r < r1 && cc >= d.c0 && cc < c1 && (!lower || r >= cc);
+  const int rbase = jb.rb + (slope & 2 ? Nm : 0), cbase = jb.cb + (slope & 1 ? Nn : 0);
+  auto wanted = [&](int i, int j) {
+    if (s_vi[i] < 0 || s_vj[j] < 0) return false;
+    const int r = rbase + s_vi[i], c = cbase + s_vj[j];
+    return r >= d.r0 && r < r1 && c >= d.c0 && c < c1 && (!lower || r >= c);
   };
-  unsigned mask[kEPairs];
-  int vj[kEPairs];
   bool any = false;
-#pragma unroll
-  for (int q = 0; q < kEPairs; ++q) {
-    const int cj = cj0 + c, rj = rj0 + e + 2 * q;
-    vj[q] = (cj < N && rj < N) ? g.cell_idx[rj * N + cj] : -1;
-    mask[q] = 0;
-    if (vi >= 0 && vj[q] >= 0) {
-      const int rx = jb.rb + vi, ry = jb.rb + Nm + vi;
-      const int cx = jb.cb + vj[q], cy = jb.cb + Nn + vj[q];
-      mask[q] = (want(rx, cx) ? 1u : 0u) | (want(rx, cy) ? 2u : 0u) | (want(ry, cx) ? 4u : 0u) |
-                (want(ry, cy) ? 8u : 0u);
-    }
-    any |= mask[q] != 0;
-  }
-  if (!__syncthreads_or(any)) return;  // the whole block: nothing to write
-  const int bA = (5 * c + a) * 36 + 4 * e + b;
-  const int bY = kEOffYY + (5 * e + b) * 36 + 4 * c + a;
-  const int bX = kEOffYX + (4 * c + a) * 44 + 5 * e + b;
+  for (int q = lane; q < kEPairs; q += 32) any |= wanted(q & 15, q >> 4);
+  if (!__any_sync(0xffffffffu, any)) return;  // nothing of this covariance is written
 
-  double acc[kEPairs][4];
+  double acc[kEB][kEA];
 #pragma unroll
-  for (int q = 0; q < kEPairs; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.0;
+  for (int v = 0; v < kEB; ++v)
+#pragma unroll
+    for (int u = 0; u < kEA; ++u) acc[v][u] = 0.0;
+  // the lane's fixed i and j indices
+  const int fix = kind < 2 ? c_edge_lane[lane] : lane, fi = fix & 3, fj = fix >> 2;
+  // centres in co: xm [0, 5), ym [5, 10), xn [10, 19), yn [19, 28)
+  const double *xm = co, *ym = co + kEU, *xn = co + 2 * kEU, *yn = xn + kEV;
   const int nL = g.nLayer;
   const double sspm = g.diam / g.Nssp[m], sspn = g.diam / g.Nssp[n];
   const double kk = kLambda2 / (sspm * sspn);
@@ -417,99 +521,99 @@ __global__ void __launch_bounds__(kEThreads, 3)
     if (!(sml > 0 && snl > 0)) continue;
     const double h = g.layer[3 * nL + g.nW * nL + l];
     const double tpl = g.layer[l];
-    const double t2 = tpl * tpl;
+    const double t2 = tpl * tpl * (1.0 / kXlim2);
     const double w = 0.5 * kk * g.layer[2 * nL + l] * g.layer[nL + l];
-    // 1. separations: value = t2 ((C_m(o_m + u) - [edge] s_m/2) - (C_n(o_n + v) - [edge] s_n/2))^2
-    for (int k = tid; k < kESqTotal; k += kEThreads) {
-      int arr, u0;
-      if (k < kESqXXc) { arr = 0; u0 = kESqXXr; }
-      else if (k < kESqYYr) { arr = 1; u0 = kESqXXc; }
-      else if (k < kESqYYc) { arr = 2; u0 = kESqYYr; }
-      else if (k < kESqXYr) { arr = 3; u0 = kESqYYc; }
-      else if (k < kESqXYc) { arr = 4; u0 = kESqXYr; }
-      else if (k < kESqYXr) { arr = 5; u0 = kESqXYc; }
-      else if (k < kESqYXc) { arr = 6; u0 = kESqYXr; }
-      else { arr = 7; u0 = kESqYXc; }
-      // axis (x = 0), i edge, j edge of each array: XXr XXc YYr YYc XYr XYc YXr YXc
-      const bool yax = (0xA6u >> arr) & 1u;     // XXc, YYr, XYc, YXc
-      const bool iedge = (0x95u >> arr) & 1u;   // XXr, YYr, XYr, YXc
-      const bool jedge = (0x65u >> arr) & 1u;   // XXr, YYr, XYc, YXr
-      const int nu = iedge ? kEA + 1 : kEA;
-      const int idx = k - u0, u = idx % nu, v = idx / nu;
-      const double rm = 1. - h * g.gsAlt[m], rn = 1. - h * g.gsAlt[n];
-      const double xm = yax ? grid_centre(g, ri0 + u, g.YPup[m], rm, g.alphaY[m] * h)
-                            : grid_centre(g, ci0 + u, g.XPup[m], rm, g.alphaX[m] * h);
-      const double xn = yax ? grid_centre(g, rj0 + v, g.YPup[n], rn, g.alphaY[n] * h)
-                            : grid_centre(g, cj0 + v, g.XPup[n], rn, g.alphaX[n] * h);
-      const double dv = (iedge ? xm - sml * 0.5 : xm) - (jedge ? xn - snl * 0.5 : xn);
-      sq[k] = t2 * (dv * dv);
+    __syncwarp();
+    if (lane < kECoord) {
+      const bool of_m = lane < 2 * kEU;
+      const int k = of_m ? lane : lane - 2 * kEU, ne = of_m ? kEU : kEV;
+      const bool yax = k >= ne;
+      const int wf = of_m ? m : n;
+      const int c = (yax ? k - ne : k) + (of_m ? (yax ? ri0 : ci0) : (yax ? rj0 : cj0));
+      co[lane] = grid_centre(g, c, yax ? g.YPup[wf] : g.XPup[wf], 1. - h * g.gsAlt[wf],
+                             (yax ? g.alphaY[wf] : g.alphaX[wf]) * h);
     }
-    __syncthreads();
-    // 2. points: 4 x 1,440, two independent evaluations per iteration (twice the
-    // FP64 chains in flight) with the table indices stepped, not divided out
-    {
-      // XX and YY (45 x 32 each, row stride 36): column tid % 32, rows tid / 32 + 8 k
-      const int cc = tid & 31;
-      const double scx = sq[kESqXXc + cc], scy = sq[kESqYYc + cc];
-      for (int r = tid >> 5; r < 45; r += kEThreads / 32) {
-        const double vx = dphi_unit_s_inl(sq[kESqXXr + r] + scx);
-        const double vy = dphi_unit_s_inl(sq[kESqYYr + r] + scy);
-        pts[r * 36 + cc] = vx;
-        pts[kEOffYY + r * 36 + cc] = vy;
+    __syncwarp();
+    // edge k of a WFS's tile is half a projected subaperture below centre k
+    const double em = sml * 0.5, en = snl * 0.5;
+    double u_sep[kEU];
+    if (kind < 2) {
+      const double *am = kind == 0 ? xm : ym, *an = kind == 0 ? xn : yn;
+      const double *bm = kind == 0 ? ym : xm, *bn = kind == 0 ? yn : xn;
+      for (int q = lane; q < kEU * kEV; q += 32) {
+        const double dv = (am[q % kEU] - em) - (an[q / kEU] - en);
+        S[q] = t2 * (dv * dv);
       }
-      // XY (40 x 36, stride 36) and YX (36 x 40, stride 44) by flat index
-      for (int f = tid; f < kEKind; f += kEThreads) {
-        const int r1 = f / 36, c1 = f - 36 * r1;
-        const int r2 = f / 40, c2 = f - 40 * r2;
-        const double v1 = dphi_unit_s_inl(sq[kESqXYr + r1] + sq[kESqXYc + c1]);
-        const double v2 = dphi_unit_s_inl(sq[kESqYXr + r2] + sq[kESqYXc + c2]);
-        pts[kEOffXY + r1 * 36 + c1] = v1;
-        pts[kEOffYX + r2 * 44 + c2] = v2;
-      }
-    }
-    __syncthreads();
-    // 3. the reference's stencils (cov_XX/YY/XY/YX, matcov_kernels.cpp:147-193), in its
-    // order: right/top edges are index + 1, left/bottom edges index + 0
+      const double dc = bm[fi] - bn[fj];
+      __syncwarp();
+      edge_layer<true>(tab, S, t2 * (dc * dc), u_sep, 0.0, nullptr, t2, w, acc);
+    } else {
+      const double *am = kind == 2 ? xm : ym, *an = kind == 2 ? xn : yn;  // u edges - centre
+      const double *bm = kind == 2 ? ym : xm, *bn = kind == 2 ? yn : xn;  // centre - v edges
 #pragma unroll
-    for (int q = 0; q < kEPairs; ++q) {
-      if (!mask[q]) continue;
-      const double* XX = pts + bA + 8 * q;             // XX(a + di, c + dj) at 36 di + 180 dj
-      const double* XY = pts + kEOffXY + bA + 8 * q;   // XY(a + di, e + dj) at 36 di + 4 dj
-      const double* YX = pts + bX + 10 * q;            // YX(b + di, c + dj) at di + 176 dj
-      const double* YY = pts + bY + 360 * q;           // YY(b + di, e + dj) at 36 di + 180 dj
-      if (mask[q] & 1u) acc[q][0] += (-XX[216] + XX[36] + XX[180] - XX[0]) * w;
-      if (mask[q] & 2u) acc[q][1] += (-XY[40] + XY[36] + XY[4] - XY[0]) * w;
-      if (mask[q] & 4u) acc[q][2] += (-YX[177] + YX[1] + YX[176] - YX[0]) * w;
-      if (mask[q] & 8u) acc[q][3] += (-YY[216] + YY[36] + YY[180] - YY[0]) * w;
+      for (int u = 0; u < kEU; ++u) {
+        const double dv = (am[u] - em) - an[fj];
+        u_sep[u] = t2 * (dv * dv);
+      }
+      edge_layer<false>(tab, nullptr, 0.0, u_sep, bm[fi] + en, bn, t2, w, acc);
     }
-    __syncthreads();
   }
+  // through shared memory in two halves (v < 4, v >= 4), so that neighbouring lanes
+  // store neighbouring rows
   const long long ld = d.ld;
+  const bool fixed_j = kind == 0 || kind == 3;  // j = 8 fj + v, else 8 v + fj
 #pragma unroll
-  for (int q = 0; q < kEPairs; ++q) {
-    if (!mask[q]) continue;
-    const int rx = jb.rb + vi, ry = jb.rb + Nm + vi;
-    const int cx = jb.cb + vj[q], cy = jb.cb + Nn + vj[q];
-    auto store = [&](int r, int cc, double val) {
-      out[(size_t)(cc - d.c0) * ld + (r - d.r0)] = (OutT)val;
-      if (d.type == 5 && r != cc) out[(size_t)(r - d.c0) * ld + (cc - d.r0)] = (OutT)val;
-    };
-    if (mask[q] & 1u) store(rx, cx, acc[q][0]);
-    if (mask[q] & 2u) store(rx, cy, acc[q][1]);
-    if (mask[q] & 4u) store(ry, cx, acc[q][2]);
-    if (mask[q] & 8u) store(ry, cy, acc[q][3]);
+  for (int half = 0; half < 2; ++half) {
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < kEB / 2; ++v)
+#pragma unroll
+      for (int u = 0; u < kEA; ++u) {
+        const int i = (kind == 0 || kind == 2) ? fi * kEA + u : u * kEA + fi;  // b * 4 + a
+        const int j = fixed_j ? fj * 4 + v : v * kEB + fj;
+        o[j * kEA * kEA + i] = acc[half * 4 + v][u];
+      }
+    __syncwarp();
+    for (int q = lane; q < kEPairs / 2; q += 32) {
+      const int i = q & 15, jj = q >> 4;
+      const int j = fixed_j ? (jj >> 2) * kEB + half * 4 + (jj & 3) : half * 32 + jj;  // e * 8 + c
+      if (!wanted(i, j)) continue;
+      const int r = rbase + s_vi[i], c = cbase + s_vj[j];
+      out[(size_t)(c - d.c0) * ld + (r - d.r0)] = (OutT)o[q];
+      if (d.type == 5 && r != c) out[(size_t)(r - d.c0) * ld + (c - d.r0)] = (OutT)o[q];
+    }
   }
+}
+
+// Persistent: one CTA per SM holds the table in shared memory; item v of the launch
+// goes to warp v / gridDim.x of CTA v % gridDim.x, so that a short launch spreads
+// over the SMs.
+template <typename OutT>
+__global__ void __launch_bounds__(kEWarps * 32, 1)
+    matcov_edge_kernel(const __grid_constant__ EdgeLaunch d, const DevGeometry g,
+                       OutT* __restrict__ out) {
+  extern __shared__ __align__(16) char esm[];
+  dphi_fill<kEWarps * 32>(esm, g.dphi);  // written once, long before: no need to wait for it
+  chain_wait();
+  __syncthreads();
+  const int warp = threadIdx.x >> 5;
+  double* wsm = reinterpret_cast<double*>(esm + kTabBytes) + warp * kEWarpDoubles;
+  for (int v = blockIdx.x + warp * gridDim.x; v < 4 * d.total_tiles; v += kEWarps * gridDim.x)
+    edge_item<OutT>(d, g, out, esm, wsm, v);
 }
 
 // Ctt (type 4): truth-sensor auto-covariance from the unprojected positions,
 // compute_element_ts_tile (common/kernels/matcov_kernels.cpp:423-483). The
 // reference indexes the truth sensor at Nsubap_ts * (nW - 1), which assumes
-// every WFS has the same number of valid subapertures; kept as is.
+// every WFS has the same number of valid subapertures; kept as is. Where they are on
+// the common grid, the pair's offset table holds every value (toeplitz_table_kernel):
+// 13.4 -> 0.1 ms for nmeasts 5,824.
 template <typename OutT>
 __global__ void __launch_bounds__(kTileI* kTileJ)
     matcov_ts_kernel(const DevGeometry g, int r0, int c0, int nrows, int ncols,
                      long long ld, OutT* __restrict__ out) {
   __shared__ double s_tpl[kMaxLayers], s_w[kMaxLayers];
+  chain_wait();
   const int nL = g.nLayer;
   const int ts = g.nW - 1;
   const int Nt = g.Nsubap[ts];
@@ -529,19 +633,32 @@ __global__ void __launch_bounds__(kTileI* kTileJ)
   const unsigned mask = (want(i, j) ? 1u : 0u) | (want(i, Nt + j) ? 2u : 0u) |
                         (want(Nt + i, j) ? 4u : 0u) | (want(Nt + i, Nt + j) ? 8u : 0u);
   if (!mask) return;
+  const int tab = g.ttab ? g.tpair[ts][ts] : -1;
+  double cxx = 0, cxy = 0, cyx = 0, cyy = 0;
+  if (tab >= 0) {
+    const int N = g.nssp_grid, W = 2 * N - 1;
+    const int2 a = reinterpret_cast<const int2*>(g.grid_cr)[i];
+    const int2 b = reinterpret_cast<const int2*>(g.grid_cr)[j];
+    const long off = ((long)tab * W * W + (long)(a.y - b.y + N - 1) * W + (a.x - b.x + N - 1)) * 4;
+    const double4 t4 = *reinterpret_cast<const double4*>(g.ttab + off);
+    cxx = t4.x;
+    cxy = t4.y;
+    cyx = t4.z;
+    cyy = t4.w;
+  }
   const int base = Nt * (g.nW - 1);
   const double du = g.X[base + i] - g.X[base + j];
   const double dv = g.Y[base + i] - g.Y[base + j];
   const double s = ssp * 0.5, ad = 2.0 * s;
-  double cxx = 0, cxy = 0, cyx = 0, cyy = 0;
-  for (int l = 0; l < nL; ++l) {
-    const double tpl = s_tpl[l], w = s_w[l];
-    const double d0 = (mask & 9u) ? D(du, dv, tpl) : 0.0;
-    if (mask & 1u) cxx += (-d0 + D(du + ad, dv, tpl) + D(du - ad, dv, tpl) - d0) * w;
-    if (mask & 8u) cyy += (-d0 + D(du, dv + ad, tpl) + D(du, dv - ad, tpl) - d0) * w;
+  for (int l = 0; l < nL && tab < 0; ++l) {
+    const double t2 = s_tpl[l] * s_tpl[l] * (1.0 / kXlim2), w = s_w[l];
+    auto D = [&](double x, double y) { return dphi_row(g.dphi, t2 * (x * x + y * y)); };
+    const double d0 = (mask & 9u) ? D(du, dv) : 0.0;
+    if (mask & 1u) cxx += (-d0 + D(du + ad, dv) + D(du - ad, dv) - d0) * w;
+    if (mask & 8u) cyy += (-d0 + D(du, dv + ad) + D(du, dv - ad) - d0) * w;
     if (mask & 6u) {
-      const double pp = D(du + s, dv + s, tpl), pm = D(du + s, dv - s, tpl);
-      const double mp = D(du - s, dv + s, tpl), mm = D(du - s, dv - s, tpl);
+      const double pp = D(du + s, dv + s), pm = D(du + s, dv - s);
+      const double mp = D(du - s, dv + s), mm = D(du - s, dv - s);
       cxy += (-pm + pp + mm - mp) * w;
       cyx += (-mp + pp + mm - pm) * w;
     }
@@ -580,23 +697,26 @@ __global__ void toeplitz_table_kernel(const DevGeometry g, const int2* __restric
     const double dx = dc * g.pitch, dy = dr * g.pitch;
     const double sspm = g.diam / g.Nssp[m], sspn = g.diam / g.Nssp[n];
     const double kk = kLambda2 / (sspm * sspn);
-    const double bx = g.G[m] * (dx * g.cth[m] - dy * g.sth[m]);
-    const double by = g.G[m] * (dx * g.sth[m] + dy * g.cth[m]);
+    const bool ctt = m == n && m == g.nW - 1;  // unprojected positions and sizes
+    const double bx = ctt ? dx : g.G[m] * (dx * g.cth[m] - dy * g.sth[m]);
+    const double by = ctt ? dy : g.G[m] * (dx * g.sth[m] + dy * g.cth[m]);
     double cxx = 0, cxy = 0, cyx = 0, cyy = 0;
     for (int l = 0; l < nL; ++l) {
-      const double sml = g.layer[3 * nL + m * nL + l];
+      const double sml = ctt ? sspm : g.layer[3 * nL + m * nL + l];
       if (!(sml > 0)) continue;
-      const double h = g.layer[3 * nL + g.nW * nL + l];
+      const double h = ctt ? 0.0 : g.layer[3 * nL + g.nW * nL + l];
       const double rr = 1. - h * g.gsAlt[m];
       const double du = (bx + (g.XPup[m] - g.XPup[n])) * rr + (g.alphaX[m] - g.alphaX[n]) * h;
       const double dv = (by + (g.YPup[m] - g.YPup[n])) * rr + (g.alphaY[m] - g.alphaY[n]) * h;
-      const double s = sml * 0.5, ad = s + s, tpl = g.layer[l];
+      const double s = sml * 0.5, ad = s + s;
+      const double t2 = g.layer[l] * g.layer[l] * (1.0 / kXlim2);
+      auto D = [&](double x, double y) { return dphi_row(g.dphi, t2 * (x * x + y * y)); };
       const double w = 0.5 * kk * g.layer[2 * nL + l] * g.layer[nL + l];
-      const double d0 = D(du, dv, tpl);
-      cxx += (-d0 + D(du + ad, dv, tpl) + D(du - ad, dv, tpl) - d0) * w;
-      cyy += (-d0 + D(du, dv + ad, tpl) + D(du, dv - ad, tpl) - d0) * w;
-      const double pp = D(du + s, dv + s, tpl), pm = D(du + s, dv - s, tpl);
-      const double mp = D(du - s, dv + s, tpl), mm = D(du - s, dv - s, tpl);
+      const double d0 = D(du, dv);
+      cxx += (-d0 + D(du + ad, dv) + D(du - ad, dv) - d0) * w;
+      cyy += (-d0 + D(du, dv + ad) + D(du, dv - ad) - d0) * w;
+      const double pp = D(du + s, dv + s), pm = D(du + s, dv - s);
+      const double mp = D(du - s, dv + s), mm = D(du - s, dv - s);
       cxy += (-pm + pp + mm - mp) * w;
       cyx += (-mp + pp + mm - pm) * w;
     }
@@ -623,7 +743,7 @@ void subap_range(int base, int N, int w0, int w1, int* lo, int* hi) {
 template <typename OutT>
 moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, int xoffset,
                         int yoffset, int lda, int type_mat, cudaStream_t s,
-                        long long* launches) {
+                        long long* launches, bool chained) {
   if (nrows < 0 || ncols < 0 || xoffset < 0 || yoffset < 0)
     return set_error(MOAO_ERR_BAD_ARG, "matcov: negative size or offset");
   if (nrows == 0 || ncols == 0) return MOAO_OK;
@@ -643,10 +763,9 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
     if ((long)Nt * g.nW > g.Nx)  // the reference's uniform-Nsubap indexing would overrun X, Y
       return set_error(MOAO_ERR_UNSUPPORTED, "matcov: Ctt needs equal subaperture counts per WFS");
     dim3 grid((Nt + kTileI - 1) / kTileI, (Nt + kTileJ - 1) / kTileJ);
-    matcov_ts_kernel<OutT><<<grid, dim3(kTileI, kTileJ), 0, s>>>(g, xoffset, yoffset, nrows,
-                                                                 ncols, lda, data);
+    MOAO_CUDA_TRY(launch_chained(chained, matcov_ts_kernel<OutT>, grid, dim3(kTileI, kTileJ), 0, s, g,
+                                 xoffset, yoffset, nrows, ncols, (long long)lda, data));
     if (launches) ++*launches;
-    MOAO_CUDA_TRY(cudaGetLastError());
     return MOAO_OK;
   }
   if (type_mat != 1 && type_mat != 2 && type_mat != 3 && type_mat != 5)
@@ -713,9 +832,10 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
     if (tiles == 0) continue;
     static std::atomic<unsigned long long> configured{0};
     MOAO_CUDA_TRY(set_smem_limit(matcov_edge_kernel<OutT>, (int)kESmem, configured));
-    matcov_edge_kernel<OutT><<<tiles, kEThreads, kESmem, s>>>(d, g, data);
+    const int ctas = std::min(148, 4 * tiles);
+    MOAO_CUDA_TRY(launch_chained(chained, matcov_edge_kernel<OutT>, dim3((unsigned)ctas),
+                                 dim3(kEWarps * 32), kESmem, s, d, g, data));
     if (launches) ++*launches;
-    MOAO_CUDA_TRY(cudaGetLastError());
   }
   // Launch in chunks of kMaxJobs jobs.
   for (size_t base = 0; base < jobs.size(); base += kMaxJobs) {
@@ -731,9 +851,9 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
     }
     d.total_tiles = tiles;
     if (tiles == 0) continue;
-    matcov_block_kernel<OutT><<<tiles, dim3(kTileI, kTileJ), 0, s>>>(d, g, data);
+    MOAO_CUDA_TRY(launch_chained(chained, matcov_block_kernel<OutT>, dim3((unsigned)tiles),
+                                 dim3(kTileI, kTileJ), 0, s, d, g, data));
     if (launches) ++*launches;
-    MOAO_CUDA_TRY(cudaGetLastError());
   }
   return MOAO_OK;
 }
@@ -751,11 +871,74 @@ void table_pairs(const DevGeometry& g, int2* pairs, int* npairs) {
   for (int m = 0; m < g.nW; ++m)
     for (int n = 0; n < g.nW; ++n) {
       const bool needed = (m < ts && n < ts && m >= n) || (m == ts && n < ts) || (n == ts && m < ts);
-      if (needed && same(m, n)) pairs[(*npairs)++] = make_int2(m, n);
+      // Ctt by the truth sensor with itself, where every WFS is on the common grid (its
+      // positions are then the grid's)
+      bool ctt = m == ts && n == ts;
+      for (int q = 0; q < g.nW && ctt; ++q)
+        ctt = g.Nsubap[q] == g.Nsubap[0] && g.Nssp[q] == g.nssp_grid;
+      if ((needed && same(m, n)) || ctt) pairs[(*npairs)++] = make_int2(m, n);
     }
 }
 
 }  // namespace
+
+const DphiRow* dphi_table() {
+  static const std::vector<DphiRow> table = [] {
+    // the coefficients of c_Ga and c_Gma
+    static const double Ga[11] = {0, 12.067619015983075, 5.17183672113560444, 0.795667187867016068,
+                                  0.0628158306210802181, 0.00301515986981185091,
+                                  9.72632216068338833e-05, 2.25320204494595251e-06,
+                                  3.93000356676612095e-08, 5.34694362825451923e-10,
+                                  5.83302941264329804e-12};
+    static const double Gma[11] = {-3.74878707653729304, -2.04479295083852408,
+                                   -0.360845814853857083, -0.0313778969438136685,
+                                   -0.001622994669507603, -5.56455315259749673e-05,
+                                   -1.35720808599938951e-06, -2.47515152461894642e-08,
+                                   -3.50257291219662472e-10, -3.95770950530691961e-12,
+                                   -3.65327031259100284e-14};
+    auto f = [](long double v, bool asym) {
+      const long double x = std::sqrt(v) * (long double)kXlim;
+      if (asym) {
+        const long double xi = 1.0L / x;
+        return (long double)kK2 - (long double)kK3 * std::exp(-x) * std::cbrt(x) *
+                                      (1.0L + xi * (kA1 + xi * (kA2 + xi * (long double)kA3)));
+      }
+      const long double c = std::cbrt(x), z = 0.25L * x * x;
+      long double pg = Gma[10], pa = Ga[10];
+      for (int n = 9; n >= 0; --n) pg = pg * z + Gma[n];
+      for (int n = 9; n >= 1; --n) pa = pa * z + Ga[n];
+      return -0.5L * (x * c * c * pg + z * pa);
+    };
+    constexpr int D = 8;  // degree
+    std::vector<DphiRow> t(kDphiRows);
+    for (int k = 0; k < kDphiRows; ++k) {
+      const int e = kDphiLo + k / kDphiSub;
+      const long double w = std::ldexp(1.0L, e) / kDphiSub;  // interval width
+      const long double mid = std::ldexp(1.0L, e) + w * (k % kDphiSub) + w / 2;
+      // Newton's divided differences at Chebyshev nodes in tau = (v - mid) / (w / 2),
+      // expanded to powers of tau
+      long double node[D + 1], d[D + 1], mono[D + 1] = {}, basis[D + 2] = {1.0L};
+      for (int i = 0; i <= D; ++i) {
+        node[i] = std::cos(3.141592653589793238462643L * (2 * i + 1) / (2 * (D + 1)));
+        d[i] = f(mid + node[i] * w / 2, e >= 0);
+      }
+      for (int o = 1; o <= D; ++o)
+        for (int i = D; i >= o; --i) d[i] = (d[i] - d[i - 1]) / (node[i] - node[i - o]);
+      for (int o = 0; o <= D; ++o) {
+        for (int i = 0; i <= o; ++i) mono[i] += d[o] * basis[i];
+        for (int i = o + 1; i >= 1; --i) basis[i] = basis[i - 1] - node[o] * basis[i];
+        basis[0] *= -node[o];
+      }
+      long double scale = 1.0L;
+      for (int i = 0; i <= D; ++i, scale *= 2.0L / w) {
+        if (i < 5) t[k].c[i] = (double)(mono[i] * scale);
+        else t[k].f[i - 5] = (float)(mono[i] * scale);
+      }
+    }
+    return t;
+  }();
+  return table.data();
+}
 
 long toeplitz_table_doubles(const DevGeometry& g, int* npairs) {
   int2 pairs[kMaxWfs * kMaxWfs];
@@ -789,16 +972,16 @@ moao_status build_toeplitz_tables(DevGeometry& g, cudaStream_t s, long long* lau
 
 moao_status launch_matcov(const DevGeometry& g, double* data, int nrows, int ncols,
                           int xoffset, int yoffset, int lda, int type_mat, cudaStream_t s,
-                          long long* launches) {
+                          long long* launches, bool chained) {
   return launch_impl<double>(g, data, nrows, ncols, xoffset, yoffset, lda, type_mat, s,
-                             launches);
+                             launches, chained);
 }
 
 moao_status launch_matcov_f32(const DevGeometry& g, float* data, int nrows, int ncols,
                               int xoffset, int yoffset, int lda, int type_mat, cudaStream_t s,
                               long long* launches) {
   return launch_impl<float>(g, data, nrows, ncols, xoffset, yoffset, lda, type_mat, s,
-                            launches);
+                            launches, false);
 }
 
 }  // namespace moao

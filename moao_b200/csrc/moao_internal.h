@@ -69,6 +69,8 @@ struct DevGeometry {
   // [3nL, 3nL + nW*nL) sspSizeL, then h [nL]
   double* layer = nullptr;
 
+  const struct DphiRow* dphi = nullptr;  // structure-function table (dphi_table)
+
   // Projection of each WFS onto a layer at altitude h (projectedSubap):
   //   u = (G (X cos - Y sin) + XPup) (1 - h gsAlt) + alphaX h
   //   v = (G (X sin + Y cos) + YPup) (1 - h gsAlt) + alphaY h
@@ -93,6 +95,18 @@ struct DevGeometry {
   int ntiles_a = 0, ntiles_b = 0;
 };
 
+// Piecewise polynomials of the structure function f(x) in v = x^2 / Xlim^2 (matcov.cu):
+// the host table (kDphiRows rows, computed once per process), which the caller keeps
+// in device memory.
+constexpr int kDphiLo = -12, kDphiHi = 6;  // 2^kDphiLo <= v < 2^kDphiHi
+constexpr int kDphiSub = 16;               // intervals per octave
+constexpr int kDphiRows = (kDphiHi - kDphiLo) * kDphiSub;
+struct alignas(8) DphiRow {
+  double c[5];  // of 1, y, .. y^4
+  float f[4];   // of y^5 .. y^8
+};
+const DphiRow* dphi_table();
+
 // Builds the offset tables of g's equal-projection WFS pairs into g.ttab (device
 // memory provided by the caller, toeplitz_table_doubles(g) doubles).
 long toeplitz_table_doubles(const DevGeometry& g, int* npairs);
@@ -102,9 +116,10 @@ moao_status build_toeplitz_tables(DevGeometry& g, cudaStream_t s, long long* lau
 // 5 Cmm full symmetric. The tile covers rows [xoffset, xoffset+nrows) and
 // columns [yoffset, yoffset+ncols) of the global matrix; data points at the
 // tile's first element.
+// chained: the launches may start beside their predecessors (chain.cuh).
 moao_status launch_matcov(const DevGeometry& g, double* data, int nrows, int ncols,
                           int xoffset, int yoffset, int lda, int type_mat,
-                          cudaStream_t s, long long* launches);
+                          cudaStream_t s, long long* launches, bool chained = false);
 // FP32 output variant (mixed path); same geometry, FP64 evaluation.
 moao_status launch_matcov_f32(const DevGeometry& g, float* data, int nrows, int ncols,
                               int xoffset, int yoffset, int lda, int type_mat,

@@ -69,7 +69,7 @@ struct moao_ctx {
   moao::DevBuf cx_qc, cx_ec;
   // FP64 products by residues (crt_f64.cu): operands' residues and row maxima,
   // the product's residues, the guard flags
-  moao::DevBuf cf_a, cf_b, cf_ma, cf_mb, cf_k, cf_z, cf_flag;
+  moao::DevBuf cf_a, cf_b, cf_c, cf_ma, cf_mb, cf_mc, cf_k, cf_z, cf_flag;
   bool chained = true;  // chained launches of the small FP64 kernels (off under stream capture)
   bool crt_f64 = true;  // off where nothing may be allocated (stream capture, no-alloc calls)
   long mx_factored_n = -1;  // size of the factorisation held in mx_* (reuse across targets)
@@ -144,7 +144,7 @@ struct moao_ctx {
     return {&ws_w,  &ws_dinv, &ws_info, &ws_tmp, &ws_host_t, &ws_corner, &mx_a32, &mx_lr,  &mx_lc,    &mx_t32,
             &mx_w1, &mx_w2,   &mx_x,    &mx_r64, &mx_e64, &mx_qa,  &mx_qb,    &mx_ea,
             &mx_fb, &mx_colmax, &mx_norm, &mx_rid, &mx_y, &mx_y2, &mx_zu, &mx_sinv, &mx_exps,
-            &mx_dsl, &cx_qc, &cx_ec, &cf_a, &cf_b, &cf_ma, &cf_mb, &cf_k, &cf_z, &cf_flag};
+            &mx_dsl, &cx_qc, &cx_ec, &cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z, &cf_flag};
   }
   // Device bytes held by the workspaces and the geometry caches.
   size_t bytes_held() {

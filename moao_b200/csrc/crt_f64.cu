@@ -18,7 +18,7 @@
 // rounded additions per element on the FP64 tensor cores.
 //
 // Measured (B200, against the FP64 tensor cores at 28-31 TF/s): the FP64
-// reconstructor at nmeas 29,120 563 -> 238 ms (lookahead included), its Cee/Cvv chain
+// reconstructor at nmeas 29,120 563 -> 201 ms (lookahead and groups included), its Cee/Cvv chain
 // 253 -> 84 ms; the int8 products alone run at 1.7 Pop/s over K = 1,024 and 2.1 over
 // K = 29,120. Error against an FP64 library's result 1.5e-11 -> 1.3e-11 and 1.1e-11 ->
 // 4.4e-12.
@@ -45,6 +45,8 @@ constexpr int kMaxBits = 57;
 // tiles) was slower at every size: the products lose what the overlap gains.
 constexpr long kPartTiles = 4096;
 constexpr long kMaxChunks = 4096;
+// cf_flag: the operands' guard, one word per part of a product, the group operand's guard
+constexpr long kGroupFlag = 1 + kMaxChunks, kFlags = kGroupFlag + 1;
 constexpr size_t kOperandBytes = (size_t)6 << 30;  // residues of one operand held at once
 
 // Bits of the scaled operands: |sum of K products| <= K 2^(2 bits) < M / 2.
@@ -333,6 +335,15 @@ size_t crt64_bytes(long n, long m, long nb, long nact) {
   product(rest, nb, nb, false, 1);
   product(m, nb, nb, false, 1);
   product(m, rest, nb, false, 1);
+  size_t qc = 0;
+  if (crt64_pays(&c, rest - nb, rest - nb, nb, true)) {
+    qc = (size_t)round128(kFactorGroup * nb) * kNM * rest + sizeof(int) * (size_t)rest;
+    z = std::max(z, z_bytes(tc_tile_count(rest, rest, true)));
+  }
+  if (crt64_pays(&c, m, nb, nb, false)) {
+    product(m, kSolveGroup * nb, nb, false, 1);
+    product(m, std::max(0L, n - kSolveGroup * nb), kSolveGroup * nb, false, 1);
+  }
   if (nact > 0) {
     product(m, m, n, true, 1);
     product(m, m, n, false, 1);
@@ -340,11 +351,11 @@ size_t crt64_bytes(long n, long m, long nb, long nact) {
     product(nact, m, m, false, 8);
     product(nact, nact, m, false, 1);
   }
-  return qa + qb + z + small;
+  return qa + qb + qc + z + small;
 }
 
 moao_status crt64_begin(moao_ctx* ctx) {
-  MOAO_TRY(ctx->cf_flag.ensure(sizeof(int) * (1 + kMaxChunks)));
+  MOAO_TRY(ctx->cf_flag.ensure(sizeof(int) * kFlags));
   MOAO_CUDA_TRY(cudaMemsetAsync(ctx->cf_flag.p, 0, sizeof(int), ctx->stream));
   return MOAO_OK;
 }
@@ -358,13 +369,13 @@ static moao_status make_operand(moao_ctx* ctx, int slot, CrtForm form, const dou
   o.rows = rows;
   o.K = K;
   o.ldq = round128(K);
-  DevBuf& qb = slot ? ctx->cf_b : ctx->cf_a;
-  DevBuf& mb = slot ? ctx->cf_mb : ctx->cf_ma;
+  DevBuf& qb = slot == 2 ? ctx->cf_c : slot ? ctx->cf_b : ctx->cf_a;
+  DevBuf& mb = slot == 2 ? ctx->cf_mc : slot ? ctx->cf_mb : ctx->cf_ma;
   MOAO_TRY(qb.ensure((size_t)kNM * rows * o.ldq));
   MOAO_TRY(mb.ensure(sizeof(int) * (size_t)rows));
   o.q = qb.as<int8_t>();
   o.erow = mb.as<int>();
-  int* flag = ctx->cf_flag.as<int>();
+  int* flag = o.flag = ctx->cf_flag.as<int>() + (slot == 2 ? kGroupFlag : 0);
   KernelTimer kt(ctx, "crt_operand", (double)rows * K);
   MOAO_CUDA_TRY(cudaMemsetAsync(o.erow, 0x80, sizeof(int) * (size_t)rows, s));
   const dim3 blk(32, 8);
@@ -416,8 +427,18 @@ static moao_status make_balance(moao_ctx* ctx, const CrtBalance* bal, long K, co
   return MOAO_OK;
 }
 
-moao_status crt64_reserve(moao_ctx* ctx, long M, long N, bool lower) {
-  return ctx->cf_z.ensure(z_bytes(tc_tile_count(M, N, lower)));
+moao_status crt64_reserve_group(moao_ctx* ctx, long n, long K) {
+  MOAO_TRY(ctx->cf_flag.ensure(sizeof(int) * kFlags));
+  const size_t rows = (size_t)std::max(1L, n);
+  MOAO_TRY(ctx->cf_c.ensure(kNM * rows * round128(K)));
+  MOAO_TRY(ctx->cf_mc.ensure(sizeof(int) * rows));
+  return ctx->cf_z.ensure(z_bytes(tc_tile_count(n, n, true)));
+}
+
+moao_status crt64_group_operand(moao_ctx* ctx, const double* A, long lda, long rows, long K,
+                                CrtOperand* out) {
+  MOAO_CUDA_TRY(cudaMemsetAsync(ctx->cf_flag.as<int>() + kGroupFlag, 0, sizeof(int), ctx->stream));
+  return make_operand(ctx, 2, CRT_ROWS, A, lda, rows, K, 0, nullptr, 0, out);
 }
 
 moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const CrtOperand& B, long b0,
@@ -467,7 +488,7 @@ moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const Crt
   z.beta = f.beta;
   z.C = f.C;
   z.ldc = f.ldc;
-  z.skip_a = flag;
+  z.skip_a = A.flag;
   for (long c = 0; c < parts; ++c) {
     g.tile0 = z.tile0 = c * part;
     g.tiles = z.tiles = std::min(part, total - c * part);

@@ -15,6 +15,7 @@ struct CrtOperand {
   long rows = 0, K = 0, ldq = 0;  // ldq: K rounded up to 128
   int8_t* q = nullptr;            // kCrt64Moduli planes of rows x ldq
   int* erow = nullptr;            // per row: largest biased exponent
+  int* flag = nullptr;            // its guard
 };
 
 // Whether C (M x N) over K is faster as residue products than on the FP64
@@ -34,6 +35,12 @@ moao_status crt64_begin(moao_ctx* ctx);
 moao_status crt64_operand(moao_ctx* ctx, const double* A, long lda, long rows, long K,
                           CrtOperand* out);
 
+// The same operand for a group of panels, in buffers and under a guard of its own: it
+// outlives the operands of other products. Reserve: for up to n rows, K columns.
+moao_status crt64_reserve_group(moao_ctx* ctx, long n, long K);
+moao_status crt64_group_operand(moao_ctx* ctx, const double* A, long lda, long rows, long K,
+                                CrtOperand* out);
+
 // fp64[0] from the operands' rows [a0, a0 + M) and [b0, b0 + N). Where the guard
 // is raised (a non-finite value or an exponent out of range in an operand, or a
 // tensor-core wait that ran out) the FP64 tensor cores compute fp64[0..n - 1] in
@@ -50,14 +57,15 @@ struct CrtBalance {
   int half, sign;
 };
 
-// Sizes the product's residue buffer for M x N (crt64_product does so itself).
-moao_status crt64_reserve(moao_ctx* ctx, long M, long N, bool lower);
-
 // g (triB: full) by residue products, operands included.
 moao_status crt64_gemm(moao_ctx* ctx, const GemmArgs& g, const CrtBalance* bal);
 // C (M x n) = A (M x n) S, S the symmetric n x n matrix in the lower triangle of B.
 moao_status crt64_symm(moao_ctx* ctx, long M, long n, const double* A, long lda, const double* B,
                        long ldb, double* C, long ldc);
+
+// Blocks whose update of what lies beyond them is taken together: in the factorisation,
+// where longer groups leave less to run beside the diagonal blocks, and in the solves.
+constexpr long kFactorGroup = 2, kSolveGroup = 4;
 
 // Device bytes the residue products of an FP64 reconstructor (nmeas n, nmeasts m,
 // panel nb) and, with nact > 0, of the Cee/Cvv chain hold on a context.

@@ -9,6 +9,7 @@
 //                    products with the stored inverse diagonal blocks.
 //   moao_cee_cvv     lapack/compute/cee_cvv.cpp:50-125 step for step.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "context.h"
@@ -104,76 +105,137 @@ moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long 
   return MOAO_OK;
 }
 
-// A22 (rest x rest, lower) -= P P^T by residue products with one panel of lookahead:
-// the update reaches the next panel's columns first, whose diagonal block
-// (next_block, on the side stream) is then factored beside the rest of the update,
-// which leaves it the context's lookahead SMs (nmeas 29,120: 270 -> 252 ms; not beside
+// The trailing updates of the factorisation by residue products. The blocks of a group
+// update only each other's columns; the columns beyond get the whole group's update at
+// once, over its K: the combine step and the products' epilogues are then fewer (nmeas
+// 29,120, groups of 1, 2 and 4: factorisation 131, 113 and 114 ms, solves 100, 85 and
+// 79 ms). The next diagonal block is always factored on the side stream, beside products
+// that leave it the context's lookahead SMs: its own columns are updated first, those it
+// does not need beside it. So the group's update beyond the next group runs in shares,
+// one beside each of that group's blocks. (270 -> 252 ms with groups of one; not beside
 // the FP64 tensor cores' update, whose CTAs hold their SMs for up to 70 us while the
-// block's ~90 launches wait for one). MOAO_ERR_OOM: nothing was done.
-template <class F>
-moao_status trailing_ahead(moao_ctx* ctx, const double* P, long lda, long rest, long kb, long kb1,
-                           double* A22, F next_block) {
-  MOAO_TRY(ensure_lookahead(ctx));
-  CrtOperand op;
-  MOAO_TRY(crt64_begin(ctx));
-  MOAO_TRY(crt64_operand(ctx, P, lda, rest, kb, &op));
-  MOAO_TRY(crt64_reserve(ctx, rest, rest, true));
-  cudaStream_t s = ctx->stream;
-  GemmArgs g;
-  g.M = rest; g.N = kb1; g.K = kb; g.alpha = -1.0; g.beta = 1.0;
-  g.A = P; g.lda = lda;
-  g.B = P; g.ldb = lda; g.transB = true;
-  g.C = A22; g.ldc = lda; g.lowerC = true;
-  MOAO_TRY(crt64_product(ctx, op, 0, op, 0, &g, 1));
-  MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[0], s));
-  MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->la_ev[0], 0));
-  MOAO_TRY(next_block(ctx->aux));
-  MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[1], ctx->aux));
-  g.M = g.N = rest - kb1;
-  g.A = g.B = P + kb1;
-  g.C = A22 + kb1 + kb1 * lda;
-  int nsm = 148;
-  MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-  MOAO_TRY(crt64_product(ctx, op, kb1, op, kb1, &g, 1, std::max(1, nsm - ctx->lookahead_sms)));
-  MOAO_CUDA_TRY(cudaStreamWaitEvent(s, ctx->la_ev[1], 0));
-  return MOAO_OK;
+// block's ~90 launches wait for one.)
+struct Trailing {
+  moao_ctx* ctx;
+  double* A;
+  long lda, n;
+  int max_ctas;
+  CrtOperand op;     // rows r0.. of columns [p0, r0): the last whole group
+  long p0 = 0, r0 = 0, done = 0;  // its update has reached columns [r0, done)
+
+  // A(c0.., c0..c1) -= its part of the product over o's columns [p, p + K), o's rows from q0 on
+  moao_status part(const CrtOperand& o, long q0, long p, long c0, long c1, int ctas) {
+    if (c1 <= c0) return MOAO_OK;
+    GemmArgs g;
+    g.M = n - c0; g.N = c1 - c0; g.K = o.K; g.alpha = -1.0; g.beta = 1.0;
+    g.A = g.B = A + c0 + p * lda;
+    g.lda = g.ldb = lda;
+    g.transB = true;
+    g.C = A + c0 + c0 * lda; g.ldc = lda; g.lowerC = true;
+    return crt64_product(ctx, o, c0 - q0, o, c0 - q0, &g, 1, ctas);
+  }
+  // columns up to c of what is due from the last group
+  moao_status advance(long c, int ctas) {
+    const long c0 = done;
+    done = std::max(done, std::min(c, n));
+    return part(op, r0, p0, c0, done, ctas);
+  }
+};
+
+// Columns up to which the first b of q shares of columns [c0, n) reach, equal areas of
+// the lower triangle each.
+long share(long c0, long n, long b, long q) {
+  return b >= q ? n : n - (long)((double)(n - c0) * std::sqrt(1.0 - (double)b / q));
 }
 
 moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, int* d_info) {
   const long nb = ctx->nb;
   MOAO_TRY(ctx->ws_w.ensure(sizeof(double) * (size_t)std::max(n, 1L) * nb));
   double* W = ctx->ws_w.as<double>();
-  MOAO_TRY(potrf_inv_block(ctx, A, lda, dinv, n, std::min(nb, n), 0, d_info, W));
-  for (long k0 = 0; k0 < n; k0 += nb) {
-    const long kb = std::min(nb, n - k0);
-    double* Dk = dinv + k0;  // rows k0.., ld n
-    const long rest = n - k0 - kb;
-    if (rest <= 0) break;
-    double* P = A + (k0 + kb) + k0 * lda;
-    // panel: P <- P L_kk^-T
-    // (column k of P goes with the variable whose pivot is 1 / Dk(k, k))
-    const CrtBalance piv{Dk, n + 1, 0, 1};
-    MOAO_TRY(gemm_long(ctx, rest, kb, kb, 1.0, P, lda, Dk, n, true, 0.0, W, rest, false, &piv));
-    MOAO_TRY(copy_matrix(W, rest, P, lda, rest, kb, ctx->stream));
-    // trailing: A22 -= P P^T on the lower tiles, then the next diagonal block
-    const long k1 = k0 + kb, kb1 = std::min(nb, rest), r2 = rest - kb1;
-    double* A22 = A + k1 + k1 * lda;
-    bool done = false;
-    if (ctx->lookahead_sms > 0 && r2 > 0 && crt64_pays(ctx, r2, r2, kb, true)) {
-      const moao_status st = trailing_ahead(ctx, P, lda, rest, kb, kb1, A22, [&](cudaStream_t s) {
-        cudaStream_t keep = ctx->stream;
-        ctx->stream = s;
-        const moao_status r = potrf_inv_block(ctx, A22, lda, dinv + k1, n, kb1, k1, d_info, W);
-        ctx->stream = keep;
-        return r;
-      });
-      if (st != MOAO_OK && st != MOAO_ERR_OOM) return st;
-      done = st == MOAO_OK;
+  auto diag_block = [&](long k0, cudaStream_t st) -> moao_status {
+    cudaStream_t keep = ctx->stream;
+    ctx->stream = st;  // potrf_inv_block launches on the context's stream
+    const moao_status r = potrf_inv_block(ctx, A + k0 + k0 * lda, lda, dinv + k0, n,
+                                          std::min(nb, n - k0), k0, d_info, W);
+    ctx->stream = keep;
+    return r;
+  };
+  // the next diagonal block beside what is launched until join()
+  auto fork = [&](long k0) -> moao_status {
+    MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[0], ctx->stream));
+    MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->la_ev[0], 0));
+    MOAO_TRY(diag_block(k0, ctx->aux));
+    MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[1], ctx->aux));
+    return MOAO_OK;
+  };
+  auto join = [&]() -> moao_status {
+    MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->la_ev[1], 0));
+    return MOAO_OK;
+  };
+  auto ahead_pays = [&](long k1) {  // the update from column k1 on, K = nb
+    return ctx->lookahead_sms > 0 && k1 + nb < n && crt64_pays(ctx, n - k1 - nb, n - k1 - nb, nb, true);
+  };
+  Trailing t{ctx, A, lda, n, 0};
+  t.done = n;  // nothing is due
+  bool ahead = ahead_pays(nb);
+  if (ahead) {
+    MOAO_TRY(ensure_lookahead(ctx));
+    int nsm = 148;
+    MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    t.max_ctas = std::max(1, nsm - ctx->lookahead_sms);
+    const moao_status st = crt64_reserve_group(ctx, n - nb, kFactorGroup * nb);
+    if (st != MOAO_OK && st != MOAO_ERR_OOM) return st;
+    ahead = st == MOAO_OK;
+  }
+  MOAO_TRY(diag_block(0, ctx->stream));
+  for (long s0 = 0; s0 < n;) {
+    const bool grouped = ahead && ahead_pays(s0 + nb);
+    const long s1 = std::min(n, s0 + (grouped ? kFactorGroup : 1) * nb);
+    const long nblk = (s1 - s0 + nb - 1) / nb;
+    // shares of the last group's update beyond this group, beside this group's blocks;
+    // the first was taken with this group's columns
+    const long due0 = t.done;
+    for (long k0 = s0, b = 0; k0 < s1; k0 += nb, ++b) {
+      const long kb = std::min(nb, n - k0), k1 = k0 + kb, rest = n - k1;
+      if (rest <= 0) break;
+      double* P = A + k1 + k0 * lda;
+      // panel: P <- P L_kk^-T
+      // (column k of P goes with the variable whose pivot is 1 / Dk(k, k))
+      const CrtBalance piv{dinv + k0, n + 1, 0, 1};
+      MOAO_TRY(gemm_long(ctx, rest, kb, kb, 1.0, P, lda, dinv + k0, n, true, 0.0, W, rest, false, &piv));
+      MOAO_TRY(copy_matrix(W, rest, P, lda, rest, kb, ctx->stream));
+      if (!grouped) {
+        MOAO_TRY(t.advance(n, 0));
+        MOAO_TRY(gemm_long(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A + k1 + k1 * lda, lda, true));
+        MOAO_TRY(diag_block(k1, ctx->stream));
+        continue;
+      }
+      if (k1 < s1) {
+        CrtOperand o;
+        MOAO_TRY(crt64_begin(ctx));
+        MOAO_TRY(crt64_operand(ctx, P, lda, rest, kb, &o));
+        const long c1 = std::min(s1, k1 + nb);
+        MOAO_TRY(t.part(o, k1, k0, k1, c1, 0));
+        MOAO_TRY(fork(k1));
+        MOAO_TRY(t.part(o, k1, k0, c1, s1, t.max_ctas));
+        MOAO_TRY(t.advance(share(due0, n, b + 1, nblk - 1), t.max_ctas));
+        MOAO_TRY(join());
+      } else {
+        MOAO_TRY(t.advance(n, 0));
+        t.p0 = s0;
+        t.r0 = t.done = s1;
+        MOAO_TRY(crt64_group_operand(ctx, A + s1 + s0 * lda, lda, n - s1, s1 - s0, &t.op));
+        const long c1 = std::min(n, s1 + nb);
+        MOAO_TRY(t.advance(c1, 0));
+        MOAO_TRY(fork(s1));
+        // the next group's other columns, and the first share of what is beyond
+        const long g = ahead_pays(s1 + nb) ? kFactorGroup : 1;
+        const long s2 = std::min(n, s1 + g * nb);
+        MOAO_TRY(t.advance(g > 1 ? share(s2, n, 1, g) : n, t.max_ctas));
+        MOAO_TRY(join());
+      }
     }
-    if (!done) {
-      MOAO_TRY(gemm_long(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A22, lda, true));
-      MOAO_TRY(potrf_inv_block(ctx, A22, lda, dinv + k1, n, kb1, k1, d_info, W));
-    }
+    s0 = s1;
   }
   return MOAO_OK;
 }
@@ -181,6 +243,8 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
 moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, const double* dinv,
                             double* B, long ldb, long m) {
   const long nb = ctx->nb;
+  // groups of blocks, as in the factorisation
+  const long group = (crt64_pays(ctx, m, nb, nb, false) ? kSolveGroup : 1) * nb;
   MOAO_TRY(ctx->ws_w.ensure(sizeof(double) * (size_t)std::max(m, 1L) * nb));
   double* W = ctx->ws_w.as<double>();
   // Forward: X L^T = B.
@@ -190,10 +254,14 @@ moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, co
     const CrtBalance piv{dinv + k0, n + 1, 0, 1};
     MOAO_TRY(gemm_long(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, true, 0.0, W, m, false, &piv));
     MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream));
-    const long rest = n - k0 - kb;
-    if (rest > 0)
-      MOAO_TRY(gemm_long(ctx, m, rest, kb, -1.0, Bk, ldb, L + (k0 + kb) + k0 * ldl, ldl, true, 1.0,
-                    B + (k0 + kb) * ldb, ldb));
+    // the group's own columns, and at its end the ones beyond with the group's K
+    const long k1 = k0 + kb, s0 = k0 / group * group, s1 = std::min(n, s0 + group);
+    if (k1 < s1)
+      MOAO_TRY(gemm_long(ctx, m, s1 - k1, kb, -1.0, Bk, ldb, L + k1 + k0 * ldl, ldl, true, 1.0,
+                         B + k1 * ldb, ldb));
+    else if (k1 < n)
+      MOAO_TRY(gemm_long(ctx, m, n - k1, k1 - s0, -1.0, B + s0 * ldb, ldb, L + k1 + s0 * ldl, ldl, true,
+                         1.0, B + k1 * ldb, ldb));
   }
   // Backward: R L = X.
   const long nblk = (n + nb - 1) / nb;
@@ -202,9 +270,15 @@ moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, co
     double* Bk = B + k0 * ldb;
     MOAO_TRY(gemm_long(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, false, 0.0, W, m));
     MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream));
-    if (k0 > 0) {
+    const long s0 = k0 / group * group, s1 = std::min(n, s0 + group);
+    if (k0 > s0) {
       const CrtBalance piv{L + k0 + k0 * ldl, ldl + 1, 0, 1};  // R(:, k) goes with L(k, :)
-      MOAO_TRY(gemm_long(ctx, m, k0, kb, -1.0, Bk, ldb, L + k0, ldl, false, 1.0, B, ldb, false, &piv));
+      MOAO_TRY(gemm_long(ctx, m, k0 - s0, kb, -1.0, Bk, ldb, L + k0 + s0 * ldl, ldl, false, 1.0,
+                         B + s0 * ldb, ldb, false, &piv));
+    } else if (s0 > 0) {
+      const CrtBalance piv{L + s0 + s0 * ldl, ldl + 1, 0, 1};
+      MOAO_TRY(gemm_long(ctx, m, s0, s1 - s0, -1.0, B + s0 * ldb, ldb, L + s0, ldl, false, 1.0, B, ldb,
+                         false, &piv));
     }
   }
   return MOAO_OK;

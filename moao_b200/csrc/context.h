@@ -70,6 +70,9 @@ struct moao_ctx {
   // FP64 products by residues (crt_f64.cu): operands' residues and row maxima,
   // the product's residues, the guard flags
   moao::DevBuf cf_a, cf_b, cf_c, cf_ma, cf_mb, cf_mc, cf_k, cf_z, cf_flag;
+  moao::DevBuf ws_sync;  // barrier word of the diagonal blocks (diag_block)
+  int diag_ctas = 96;    // its CTAs: the lookahead's SMs beside other work, not all SMs ever
+                         // (a collective's kernels may hold some)
   bool chained = true;  // chained launches of the small FP64 kernels (off under stream capture)
   bool crt_f64 = true;  // off where nothing may be allocated (stream capture, no-alloc calls)
   long mx_factored_n = -1;  // size of the factorisation held in mx_* (reuse across targets)
@@ -144,7 +147,7 @@ struct moao_ctx {
     return {&ws_w,  &ws_dinv, &ws_info, &ws_tmp, &ws_host_t, &ws_corner, &mx_a32, &mx_lr,  &mx_lc,    &mx_t32,
             &mx_w1, &mx_w2,   &mx_x,    &mx_r64, &mx_e64, &mx_qa,  &mx_qb,    &mx_ea,
             &mx_fb, &mx_colmax, &mx_norm, &mx_rid, &mx_y, &mx_y2, &mx_zu, &mx_sinv, &mx_exps,
-            &mx_dsl, &cx_qc, &cx_ec, &cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z, &cf_flag};
+            &mx_dsl, &cx_qc, &cx_ec, &ws_sync, &cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z, &cf_flag};
   }
   // Device bytes held by the workspaces and the geometry caches.
   size_t bytes_held() {
@@ -188,6 +191,11 @@ moao_status gemm(moao_ctx* ctx, long M, long N, long K, double alpha, const doub
                  bool lowerC = false, TriMode tri = TRI_FULL);
 // Creates the context's side stream and lookahead events on first use.
 moao_status ensure_lookahead(moao_ctx* ctx);
+// SMs to leave to a 1,024-wide diagonal block beside an update that takes `seconds` on
+// the whole chip: at least the context's lookahead SMs.
+int diag_sms(const moao_ctx* ctx, double seconds);
+// The diagonal blocks' barrier word, where they may take one launch (not under capture).
+moao_status ensure_diag_sync(moao_ctx* ctx);
 // Factor the nb x nb diagonal block A in place (FP64) and write its inverse into D.
 moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long ldd, long nb,
                             long col0, int* d_info, double* W);

@@ -107,6 +107,7 @@ struct KParams {
   long ldc;
   int triB;
   long tri_off;
+  int triA = 0;  // A lower triangular (zeros stored above): k <= row only
   // tile order (set by the launcher): bands of group_m row tiles; inside a band
   // the column tiles in turn, the band's row tiles fastest
   int tiles_m, tiles_n, group_m;
@@ -187,6 +188,7 @@ __device__ __forceinline__ void gemm_tile(const KParams& p, double* smem, const 
     if (!TRANSB) kb = n0 + p.tri_off;          // B(k, n) with k >= n
     else ke = min(p.K, n0 + p.tri_off + BN);   // B(n, k) with n >= k
   }
+  if (p.triA) ke = min(ke, m0 + BM);
   kb = (kb / BK) * BK;
   const int ntiles = (ke > kb) ? (int)((ke - kb + BK - 1) / BK) : 0;
 
@@ -453,6 +455,148 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1)
   leaf_factor_inverse(A, lda, Linv, ldi, n, col0, info, leaf_smem);
 }
 
+// A whole diagonal block in one launch: the recursion of potrf_inv_block as a list of
+// phases, a barrier over the (cooperative) grid between them. Its bound is the chain of
+// phases: 16 leaves of 11 us for 1,024 columns and, per node of the recursion, three
+// products of 1 to 9 us. As ~90 launches, chained, each phase cost 4 to 6 us more than its
+// work; a barrier costs about 1.5. Products that no later leaf waits for (W2, the
+// factor's block into place) run beside a leaf, and products with a triangle skip its
+// zeros. A block of 1,024: 1.24 ms -> 0.56 on 64 CTAs, 0.87 on 16, 1.28 on 8, where
+// the FP64 units bound it (64 x 64 tiles once every CTA has one; 32 x 32 throughout: 1.85).
+// nmeas 640 reconstructor 504 -> 421 us, the factorisation at nmeas 6,656 6.5 -> 6.1 ms, at
+// 18,688 37.2 -> 35.3 ms, mixed 23.5 -> 21.9 ms.
+// The operations on each element and their order are those of the launches.
+enum DiagType { DIAG_LEAF = 0, DIAG_PANEL = 1, DIAG_TRAIL = 2, DIAG_JOIN = 3 };
+struct DiagOp {
+  int type, o, n1, n2;  // node: columns o.., n1 | n2; leaf: n1 columns
+  unsigned w2;          // the node's W2 in the workspace
+};
+constexpr int kDiagOps = 128, kDiagMax = 2048;
+struct DiagPlan {
+  int n = 0;
+  unsigned w1 = 0;  // doubles of the workspace for W1, the W2 of nodes above each other behind it
+  DiagOp op[kDiagOps];
+  void add(int type, int o, int n1, int n2, unsigned w2) { op[n++] = DiagOp{type, o, n1, n2, w2}; }
+  void build(int o, int nb, unsigned w2) {
+    if (nb <= LEAF) return add(DIAG_LEAF, o, nb, 0, 0);
+    const int n1 = LEAF * ((nb + 2 * LEAF - 1) / (2 * LEAF)), n2 = nb - n1;
+    w1 = std::max(w1, n1 * even(n2));
+    build(o, n1, w2);
+    add(DIAG_PANEL, o, n1, n2, w2);
+    add(DIAG_TRAIL, o, n1, n2, w2);  // a leaf follows, with this node's products beside it
+    build(o + n1, n2, w2 + (unsigned)n1 * even(n2));
+    add(DIAG_JOIN, o, n1, n2, w2);
+  }
+  static unsigned even(int x) { return (unsigned)(x + 1) & ~1u; }
+};
+// 32 x 32 tiles by 8 warps of 16 x 8 (the leaf's 256 threads)
+using TileD = Tile<32, 32, 16, 32, 4, 8>;
+using TileD64 = Tile<64, 64, 32, 32, 4, 16>;
+static_assert(TileD::NTHREADS == LEAF_THREADS && TileD64::NTHREADS == LEAF_THREADS, "one CTA shape for products and leaves");
+constexpr size_t kDiagSmem =
+    TileD64::SMEM_BYTES > LEAF_SMEM_BYTES ? TileD64::SMEM_BYTES : LEAF_SMEM_BYTES;
+static_assert(TileD::SMEM_BYTES <= kDiagSmem, "one size for all");
+constexpr unsigned kDiagPolls = 1u << 22;  // some seconds
+
+// All CTAs of the grid have arrived, count of them since the launch; false when the
+// wait ran out (then *err is raised and the kernel leaves).
+__device__ __forceinline__ bool diag_barrier(unsigned* arrived, unsigned count, int* err) {
+  __syncthreads();
+  int ok = 1;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    atomicAdd(arrived, 1u);
+    unsigned v, polls = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(arrived) : "memory");
+    } while (v < count && ++polls < kDiagPolls);
+    ok = v >= count;
+    if (!ok) atomicExch(err, 1);
+    __threadfence();
+  }
+  return __syncthreads_and(ok || threadIdx.x != 0);
+}
+
+template <class TL, bool TRANSB, bool LOWERC, int VEC>
+__device__ __forceinline__ void diag_tiles(const KParams& p, double* smem, int cta, int ctas) {
+  const int tm = (int)((p.M + TL::BM - 1) / TL::BM), tiles = tm * (int)((p.N + TL::BN - 1) / TL::BN);
+  if (LOWERC) {  // a square C: tiles m >= n only, by columns
+    int n = 0, first = 0;  // column n starts at the first-th tile
+    for (int v = cta; v < tm * (tm + 1) / 2; v += ctas) {
+      while (v >= first + tm - n) first += tm - n++;
+      const int m = n + v - first;
+      gemm_tile<TL, TRANSB, LOWERC, VEC, true>(p, smem, (long)m * TL::BM, (long)n * TL::BN);
+      __syncthreads();
+    }
+    return;
+  }
+  // a CTA's tiles spread over the rows: K grows along them with a triangular A
+  for (int v = cta; v < tiles; v += ctas) {
+    const int n = v / tm, m = (v + n) % tm;
+    gemm_tile<TL, TRANSB, LOWERC, VEC, true>(p, smem, (long)m * TL::BM, (long)n * TL::BN);
+    __syncthreads();
+  }
+}
+
+template <bool TRANSB, bool LOWERC, int VEC>
+__device__ __forceinline__ void diag_product(const KParams& p, double* smem, int cta, int ctas) {
+  const long t64 = ((p.M + 63) / 64) * ((p.N + 63) / 64);
+  if ((LOWERC ? (t64 + 1) / 2 : t64) >= ctas) diag_tiles<TileD64, TRANSB, LOWERC, VEC>(p, smem, cta, ctas);
+  else diag_tiles<TileD, TRANSB, LOWERC, VEC>(p, smem, cta, ctas);
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(LEAF_THREADS, 1)
+    diag_block_kernel(const __grid_constant__ DiagPlan plan, double* A, long lda, double* D, long ldd,
+                      double* W, long col0, int* info, unsigned* arrived) {
+  extern __shared__ __align__(16) double diag_smem[];
+  double* sm = diag_smem;
+  const int ctas = gridDim.x;
+  for (int k = 0; k < plan.n; ++k) {
+    const DiagOp op = plan.op[k];
+    if (op.type == DIAG_LEAF) {
+      if (blockIdx.x == 0)
+        leaf_factor_inverse(A + op.o * (lda + 1), lda, D + op.o * (ldd + 1), ldd, op.n1, col0 + op.o, info,
+                            sm);
+      __syncthreads();
+      const int workers = ctas > 1 ? ctas - 1 : 1, me = ctas > 1 ? (int)blockIdx.x - 1 : 0;
+      if (k > 0 && plan.op[k - 1].type == DIAG_TRAIL && me >= 0) {
+        const DiagOp q = plan.op[k - 1];
+        const long n1 = q.n1, n2 = q.n2, ldw = (n2 + 1) & ~1L;
+        double* D11 = D + q.o * (ldd + 1);
+        // W2 = L21 D11
+        const KParams p{n2, n1, n1, 1.0, 0.0, W, ldw, D11, ldd, W + plan.w1 + q.w2, ldw, TRI_LOWER, 0};
+        diag_product<false, false, VEC>(p, sm, me, workers);
+        // L21 into place, zeros above the inverse's diagonal
+        double *A21 = A + q.o * (lda + 1) + n1, *D12 = D11 + n1 * ldd;
+        const int lane = threadIdx.x & 31, warps = workers * (LEAF_THREADS / 32);
+        const int w0 = me * (LEAF_THREADS / 32) + (threadIdx.x >> 5);
+        for (long c = w0; c < n1; c += warps)
+#pragma unroll 4
+          for (long r = lane; r < n2; r += 32) A21[c * lda + r] = W[c * ldw + r];
+        for (long c = w0; c < n2; c += warps)
+          for (long r = lane; r < n1; r += 32) D12[c * ldd + r] = 0.0;
+      }
+    } else {
+      const long n1 = op.n1, n2 = op.n2, ldw = (n2 + 1) & ~1L;
+      double *A11 = A + op.o * (lda + 1), *D11 = D + op.o * (ldd + 1);
+      if (op.type == DIAG_PANEL) {  // W = L21 = A21 L11^-T
+        const KParams p{n2, n1, n1, 1.0, 0.0, A11 + n1, lda, D11, ldd, W, ldw, TRI_LOWER, 0};
+        diag_product<true, false, VEC>(p, sm, blockIdx.x, ctas);
+      } else if (op.type == DIAG_TRAIL) {  // A22 -= L21 L21^T
+        const KParams p{n2, n2, n1, -1.0, 1.0, W, ldw, W, ldw, A11 + n1 * (lda + 1), lda, 0, 0};
+        diag_product<true, true, VEC>(p, sm, blockIdx.x, ctas);
+      } else {  // D21 = -D22 W2
+        KParams p{n2, n1, n2, -1.0, 0.0, D11 + n1 * (ldd + 1), ldd, W + plan.w1 + op.w2, ldw, D11 + n1, ldd,
+                  0, 0};
+        p.triA = 1;
+        diag_product<false, false, VEC>(p, sm, blockIdx.x, ctas);
+      }
+    }
+    if (k + 1 < plan.n && !diag_barrier(arrived, (unsigned)ctas * (k + 1), info + 1)) return;
+  }
+}
+
 // dst (m x n) = src, and the zn x zm block at z (null: none) = 0: the factor's block
 // into place and the zeros above the diagonal of its inverse.
 __global__ void copy_zero_kernel(const double* __restrict__ src, long lds, double* __restrict__ dst,
@@ -542,6 +686,34 @@ moao_status potrf_inv_leaf(double* A, long lda, double* Linv, long ldi, int n, l
   MOAO_CUDA_TRY(set_smem_limit(potrf_inv_leaf_kernel, smem, configured));
   MOAO_CUDA_TRY(launch_chained(chained, potrf_inv_leaf_kernel, dim3(1), dim3(LEAF_THREADS), (size_t)smem,
                                s, A, lda, Linv, ldi, n, col0, d_info));
+  if (launches) ++*launches;
+  return MOAO_OK;
+}
+
+bool diag_block_fits(long nb) { return nb > LEAF && nb <= kDiagMax; }
+
+moao_status diag_block(double* A, long lda, double* D, long ldd, long nb, long col0, int* d_info,
+                       double* W, unsigned* d_sync, int ctas, cudaStream_t s, long long* launches) {
+  if (!diag_block_fits(nb)) return set_error(MOAO_ERR_BAD_ARG, "diag_block: size");
+  DiagPlan plan;
+  plan.build(0, (int)nb, 0);
+  MOAO_CUDA_TRY(cudaMemsetAsync(d_sync, 0, sizeof(unsigned), s));
+  const bool v2 = aligned16(A) && aligned16(D) && aligned16(W) && lda % 2 == 0 && ldd % 2 == 0;
+  auto kern = v2 ? diag_block_kernel<2> : diag_block_kernel<1>;
+  static std::atomic<unsigned long long> configured[2];
+  MOAO_CUDA_TRY(set_smem_limit(kern, (int)kDiagSmem, configured[v2]));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(LEAF_THREADS);
+  cfg.dynamicSmemBytes = kDiagSmem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MOAO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const DiagPlan&)plan, A, lda, D, ldd, W, col0, d_info,
+                                   d_sync));
   if (launches) ++*launches;
   return MOAO_OK;
 }

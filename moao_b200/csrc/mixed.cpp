@@ -538,10 +538,13 @@ moao_status reconstructor_mixed(moao_ctx* ctx, long n, long m, double* Cmm, long
     MOAO_TRY(cvt_lower_minus_offsets(Cmm, ldCmm, A32, n, n, rid, off, s));
     // the ragged last diagonal block leaves K columns of its copies unused: zeros
     if (f16) MOAO_CUDA_TRY(cudaMemsetAsync(dr, 0, z.dsl, s));
+    MOAO_TRY(ensure_diag_sync(ctx));
     // Diagonal block at k0: FP64 factor and inverse (dinv), FP32 factor back into
     // A32, fp16 copies of the inverse. Runs on stream st.
-    auto diag_block = [&](long k0, long kb, cudaStream_t st) -> moao_status {
+    auto diag_block = [&](long k0, long kb, cudaStream_t st, int sms = 0) -> moao_status {
       cudaStream_t keep = ctx->stream;
+      const int ctas = ctx->diag_ctas;
+      if (sms > 0) ctx->diag_ctas = sms;
       ctx->stream = st;  // potrf_inv_block launches on the context's stream
       float* Akk = A32 + k0 + k0 * n;
       moao_status r = cvt_f32_to_f64(Akk, n, W1, kb, kb, kb, true, st);
@@ -561,6 +564,7 @@ moao_status reconstructor_mixed(moao_ctx* ctx, long n, long m, double* Cmm, long
           r = split_f16(dinv + k0, n, kb, kb, nsl, br, nb, sc.edr + k0, bc, nb, sc.edc + k0, st);
       }
       ctx->stream = keep;
+      ctx->diag_ctas = ctas;
       return r;
     };
     // Lookahead (not under capture): once the trailing update has reached the next
@@ -608,13 +612,16 @@ moao_status reconstructor_mixed(moao_ctx* ctx, long n, long m, double* Cmm, long
                            (double)(2 * rest - kb1) * kb1 * kb, er, er));
         MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[0], s));
         MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->la_ev[0], 0));
-        MOAO_TRY(diag_block(k1, kb1, ctx->aux));
-        MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[1], ctx->aux));
         const long r2 = rest - kb1;
+        // the slice products run at 0.96 PFLOP/s
+        const int sms = std::max(lookahead_for(ctx, rest),
+                                 diag_sms(ctx, (double)r2 * r2 * kb * full.n / 0.96e15));
+        MOAO_TRY(diag_block(k1, kb1, ctx->aux, sms));
+        MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[1], ctx->aux));
         MOAO_TRY(tc_update(ctx, mp.lrA, (int)(k1 + kb1), (int)k0, mp.lrB, (int)(k1 + kb1), (int)k0,
                            nk, full, r2, r2, A32 + (k1 + kb1) + (k1 + kb1) * n, n, true, err,
                            (double)r2 * r2 * kb, er ? er + kb1 : nullptr, er ? er + kb1 : nullptr,
-                           std::max(1, nsm - lookahead_for(ctx, rest))));
+                           std::max(1, nsm - sms)));
         MOAO_CUDA_TRY(cudaStreamWaitEvent(s, ctx->la_ev[1], 0));
       } else {
         MOAO_TRY(tc_update(ctx, mp.lrA, (int)k1, (int)k0, mp.lrB, (int)k1, (int)k0, nk, full, rest,

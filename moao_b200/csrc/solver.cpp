@@ -74,10 +74,36 @@ moao_status ensure_lookahead(moao_ctx* ctx) {
   return MOAO_OK;
 }
 
+int diag_sms(const moao_ctx* ctx, double seconds) {
+  // A block of 1,024 takes 0.45 ms (its chain) + 6.6 ms over the SMs, one CTA on each. As
+  // many as let it end with the update, 64 at most (0.56 ms).
+  // The block's CTAs must not outnumber the SMs left: each would take one of the update's,
+  // whose persistent CTA would then start when the block ends (2.2 -> 3.2 ms).
+  int sms = ctx->lookahead_sms;
+  while (sms < 64 && 0.45e-3 + 6.6e-3 / sms > seconds * 148.0 / (148 - sms))
+    sms = std::min(64, sms + std::max(1, sms / 2));
+  return sms;
+}
+
+moao_status ensure_diag_sync(moao_ctx* ctx) {
+  return ctx->chained && !ctx->graph_mode ? ctx->ws_sync.ensure(sizeof(unsigned)) : MOAO_OK;
+}
+
 // Factor the nb x nb diagonal block A (lda) and write its inverse into D (ldd).
-// W is scratch of at least nb*nb/4 doubles... (nb/2 x nb/2 + margin).
+// W is scratch of nb x nb doubles. One launch (diag_block) on contexts that own the word
+// its barrier counts in; launch by launch where there is none (the call without
+// allocations, whose scratch is fixed), and under capture, where graphs of several
+// instances run side by side and should not wait for SMs to be free all at once.
 moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long ldd, long nb,
                             long col0, int* d_info, double* W) {
+  if (ctx->ws_sync.p && !ctx->graph_mode && diag_block_fits(nb)) {
+    int nsm = 148;
+    MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
+    const int ctas = std::min(nsm, std::max(1, ctx->diag_ctas));
+    KernelTimer kt(ctx, "diag_block", (double)nb * nb * nb * (2.0 / 3));
+    return diag_block(A, lda, D, ldd, nb, col0, d_info, W, ctx->ws_sync.as<unsigned>(), ctas, ctx->stream,
+                      &ctx->launches);
+  }
   if (nb <= kLeaf) {
     KernelTimer kt(ctx, "potrf_leaf", (double)nb * nb * nb * (1.0 / 3 + 1.0 / 3));
     return potrf_inv_leaf(A, lda, D, ldd, (int)nb, col0, d_info, ctx->chained, ctx->stream,
@@ -113,8 +139,7 @@ moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long 
 // that leave it the context's lookahead SMs: its own columns are updated first, those it
 // does not need beside it. So the group's update beyond the next group runs in shares,
 // one beside each of that group's blocks. (270 -> 252 ms with groups of one; not beside
-// the FP64 tensor cores' update, whose CTAs hold their SMs for up to 70 us while the
-// block's ~90 launches wait for one.)
+// the FP64 tensor cores' update, whose CTAs leave no SM free.)
 struct Trailing {
   moao_ctx* ctx;
   double* A;
@@ -152,19 +177,30 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
   const long nb = ctx->nb;
   MOAO_TRY(ctx->ws_w.ensure(sizeof(double) * (size_t)std::max(n, 1L) * nb));
   double* W = ctx->ws_w.as<double>();
-  auto diag_block = [&](long k0, cudaStream_t st) -> moao_status {
+  MOAO_TRY(ensure_diag_sync(ctx));
+  int nsm = 148;
+  Trailing t{ctx, A, lda, n, 0};
+  t.done = n;  // nothing is due
+  auto diag_block = [&](long k0, cudaStream_t st, int sms = 0) -> moao_status {
     cudaStream_t keep = ctx->stream;
+    const int ctas = ctx->diag_ctas;
+    if (sms > 0) ctx->diag_ctas = sms;
     ctx->stream = st;  // potrf_inv_block launches on the context's stream
     const moao_status r = potrf_inv_block(ctx, A + k0 + k0 * lda, lda, dinv + k0, n,
                                           std::min(nb, n - k0), k0, d_info, W);
     ctx->stream = keep;
+    ctx->diag_ctas = ctas;
     return r;
   };
-  // the next diagonal block beside what is launched until join()
-  auto fork = [&](long k0) -> moao_status {
+  // the next diagonal block beside what is launched until join(): updates of columns
+  // [c0, c1) over K from the first group and [d0, d1) over L from the last
+  auto fork = [&](long k0, long c0, long c1, long K, long d0, long d1, long L) -> moao_status {
+    auto area = [&](long x, long y) { return 0.5 * ((double)(n - x) * (n - x) - (double)(n - y) * (n - y)); };
+    const int sms = diag_sms(ctx, 2.0 * 16 / 1.9e15 * (area(c0, c1) * K + area(d0, d1) * L));
+    t.max_ctas = std::max(1, nsm - sms);
     MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[0], ctx->stream));
     MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->aux, ctx->la_ev[0], 0));
-    MOAO_TRY(diag_block(k0, ctx->aux));
+    MOAO_TRY(diag_block(k0, ctx->aux, sms));
     MOAO_CUDA_TRY(cudaEventRecord(ctx->la_ev[1], ctx->aux));
     return MOAO_OK;
   };
@@ -175,14 +211,10 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
   auto ahead_pays = [&](long k1) {  // the update from column k1 on, K = nb
     return ctx->lookahead_sms > 0 && k1 + nb < n && crt64_pays(ctx, n - k1 - nb, n - k1 - nb, nb, true);
   };
-  Trailing t{ctx, A, lda, n, 0};
-  t.done = n;  // nothing is due
   bool ahead = ahead_pays(nb);
   if (ahead) {
     MOAO_TRY(ensure_lookahead(ctx));
-    int nsm = 148;
     MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-    t.max_ctas = std::max(1, nsm - ctx->lookahead_sms);
     const moao_status st = crt64_reserve_group(ctx, n - nb, kFactorGroup * nb);
     if (st != MOAO_OK && st != MOAO_ERR_OOM) return st;
     ahead = st == MOAO_OK;
@@ -216,9 +248,10 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
         MOAO_TRY(crt64_operand(ctx, P, lda, rest, kb, &o));
         const long c1 = std::min(s1, k1 + nb);
         MOAO_TRY(t.part(o, k1, k0, k1, c1, 0));
-        MOAO_TRY(fork(k1));
+        const long d1 = share(due0, n, b + 1, nblk - 1);
+        MOAO_TRY(fork(k1, c1, s1, kb, t.done, d1, t.op.K));
         MOAO_TRY(t.part(o, k1, k0, c1, s1, t.max_ctas));
-        MOAO_TRY(t.advance(share(due0, n, b + 1, nblk - 1), t.max_ctas));
+        MOAO_TRY(t.advance(d1, t.max_ctas));
         MOAO_TRY(join());
       } else {
         MOAO_TRY(t.advance(n, 0));
@@ -227,11 +260,11 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
         MOAO_TRY(crt64_group_operand(ctx, A + s1 + s0 * lda, lda, n - s1, s1 - s0, &t.op));
         const long c1 = std::min(n, s1 + nb);
         MOAO_TRY(t.advance(c1, 0));
-        MOAO_TRY(fork(s1));
         // the next group's other columns, and the first share of what is beyond
         const long g = ahead_pays(s1 + nb) ? kFactorGroup : 1;
-        const long s2 = std::min(n, s1 + g * nb);
-        MOAO_TRY(t.advance(g > 1 ? share(s2, n, 1, g) : n, t.max_ctas));
+        const long d1 = g > 1 ? share(std::min(n, s1 + g * nb), n, 1, g) : n;
+        MOAO_TRY(fork(s1, n, n, 0, c1, d1, s1 - s0));
+        MOAO_TRY(t.advance(d1, t.max_ctas));
         MOAO_TRY(join());
       }
     }
@@ -319,16 +352,17 @@ moao_status reconstructor_fp64(moao_ctx* ctx, long nmeas, long nmeasts, double* 
                                double* d_Ctm, long ldCtm, long g0, long ngal,
                                moao_solve_report* r) {
   MOAO_TRY(ctx->ws_dinv.ensure(sizeof(double) * (size_t)nmeas * ctx->nb));
-  MOAO_TRY(ctx->ws_info.ensure(sizeof(int)));
+  MOAO_TRY(ctx->ws_info.ensure(3 * sizeof(int)));
   int* d_info = ctx->ws_info.as<int>();
-  MOAO_CUDA_TRY(cudaMemsetAsync(d_info, 0, sizeof(int), ctx->stream));
+  MOAO_CUDA_TRY(cudaMemsetAsync(d_info, 0, 3 * sizeof(int), ctx->stream));
   cudaEventRecord(ctx->ev[0], ctx->stream);
   MOAO_TRY(potrf_f64(ctx, d_Cmm, ldCmm, nmeas, ctx->ws_dinv.as<double>(), d_info));
   cudaEventRecord(ctx->ev[1], ctx->stream);
-  int info = 0;
-  MOAO_CUDA_TRY(cudaMemcpyAsync(&info, d_info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  int infos[2] = {0, 0};
+  MOAO_CUDA_TRY(cudaMemcpyAsync(infos, d_info, sizeof(infos), cudaMemcpyDeviceToHost, ctx->stream));
   MOAO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  r->info = info;
+  if (infos[1]) return set_error(MOAO_ERR_TIMEOUT, "dpotrf: bounded wait expired");
+  const int info = r->info = infos[0];
   if (info != 0) {
     // The reference prints and returns without solving (reconstructor.cpp:34-38).
     return set_error(MOAO_ERR_NOT_SPD, "dpotrf: non-positive pivot at column " +
@@ -464,11 +498,14 @@ moao_status moao_dense_potrf_inv(moao_ctx* ctx, long n, double* A, long lda, dou
   MOAO_TRY(ctx->ws_w.ensure(sizeof(double) * (size_t)n * n));
   MOAO_TRY(ctx->ws_info.ensure(3 * sizeof(int)));
   int* d_info = ctx->ws_info.as<int>();
-  MOAO_CUDA_TRY(cudaMemsetAsync(d_info, 0, sizeof(int), ctx->stream));
+  MOAO_CUDA_TRY(cudaMemsetAsync(d_info, 0, 3 * sizeof(int), ctx->stream));
+  MOAO_TRY(ensure_diag_sync(ctx));
   MOAO_TRY(potrf_inv_block(ctx, A, lda, Ainv, ldi, n, 0, d_info, ctx->ws_w.as<double>()));
-  int h = 0;
-  MOAO_CUDA_TRY(cudaMemcpyAsync(&h, d_info, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  int hi[2] = {0, 0};
+  MOAO_CUDA_TRY(cudaMemcpyAsync(hi, d_info, sizeof(hi), cudaMemcpyDeviceToHost, ctx->stream));
   MOAO_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+  if (hi[1]) return set_error(MOAO_ERR_TIMEOUT, "dense_potrf_inv: bounded wait expired");
+  const int h = hi[0];
   if (info) *info = h;
   if (h) return set_error(MOAO_ERR_NOT_SPD, "dense_potrf_inv: non-positive pivot at column " +
                                                 std::to_string(h));

@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1)
 // products of 1 to 9 us. As ~90 launches, chained, each phase cost 4 to 6 us more than its
 // work; a barrier costs about 1.5. Products that no later leaf waits for (W2, the
 // factor's block into place) run beside a leaf, and products with a triangle skip its
-// zeros. A block of 1,024: 1.24 ms -> 0.56 on 64 CTAs, 0.87 on 16, 1.28 on 8, where
+// zeros. A block of 1,024: 0.67 ms -> 0.52 on 96 CTAs, 0.56 on 64, 0.87 on 16, 1.28 on 8, where
 // the FP64 units bound it (64 x 64 tiles once every CTA has one; 32 x 32 throughout: 1.85).
 // nmeas 640 reconstructor 504 -> 421 us, the factorisation at nmeas 6,656 6.5 -> 6.1 ms, at
 // 18,688 37.2 -> 35.3 ms, mixed 23.5 -> 21.9 ms.

@@ -56,7 +56,7 @@ moao_status diag_block(double* A, long lda, double* D, long ldd, long nb, long c
 
 // Elementwise helpers (column-major).
 moao_status copy_matrix(const double* src, long lds, double* dst, long ldd, long m, long n,
-                        cudaStream_t s);
+                        cudaStream_t s, long long* launches = nullptr);
 // dst (m x n) = src and the zm x zn block at z = 0, in one launch.
 moao_status copy_zero(const double* src, long lds, double* dst, long ldd, long m, long n, double* z,
                       long ldz, long zm, long zn, bool chained, cudaStream_t s,

@@ -235,7 +235,7 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
       // (column k of P goes with the variable whose pivot is 1 / Dk(k, k))
       const CrtBalance piv{dinv + k0, n + 1, 0, 1};
       MOAO_TRY(gemm_long(ctx, rest, kb, kb, 1.0, P, lda, dinv + k0, n, true, 0.0, W, rest, false, &piv));
-      MOAO_TRY(copy_matrix(W, rest, P, lda, rest, kb, ctx->stream));
+      MOAO_TRY(copy_matrix(W, rest, P, lda, rest, kb, ctx->stream, &ctx->launches));
       if (!grouped) {
         MOAO_TRY(t.advance(n, 0));
         MOAO_TRY(gemm_long(ctx, rest, rest, kb, -1.0, P, lda, P, lda, true, 1.0, A + k1 + k1 * lda, lda, true));
@@ -286,7 +286,7 @@ moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, co
     double* Bk = B + k0 * ldb;
     const CrtBalance piv{dinv + k0, n + 1, 0, 1};
     MOAO_TRY(gemm_long(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, true, 0.0, W, m, false, &piv));
-    MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream));
+    MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream, &ctx->launches));
     // the group's own columns, and at its end the ones beyond with the group's K
     const long k1 = k0 + kb, s0 = k0 / group * group, s1 = std::min(n, s0 + group);
     if (k1 < s1)
@@ -302,7 +302,7 @@ moao_status solve_right_f64(moao_ctx* ctx, const double* L, long ldl, long n, co
     const long k0 = b * nb, kb = std::min(nb, n - k0);
     double* Bk = B + k0 * ldb;
     MOAO_TRY(gemm_long(ctx, m, kb, kb, 1.0, Bk, ldb, dinv + k0, n, false, 0.0, W, m));
-    MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream));
+    MOAO_TRY(copy_matrix(W, m, Bk, ldb, m, kb, ctx->stream, &ctx->launches));
     const long s0 = k0 / group * group, s1 = std::min(n, s0 + group);
     if (k0 > s0) {
       const CrtBalance piv{L + k0 + k0 * ldl, ldl + 1, 0, 1};  // R(:, k) goes with L(k, :)

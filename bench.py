@@ -798,7 +798,7 @@ def probe_main(args):
         res = []
         for cfg in range(4):
             ctx.set_gemm_tile(cfg)
-            rates, builds, leaf_us = [], [], []
+            rates, builds, diag_us = [], [], []
             for rep in range(4):
                 M.matcov_tile(Cmm, nm, nm, 0, 0, nm, t, 1, ctx=ctx)
                 M.matcov_tile(Ctm, nts, nm, 0, 0, nts, t, 3, ctx=ctx)
@@ -811,16 +811,16 @@ def probe_main(args):
                 e1.record()
                 torch.cuda.synchronize()
                 st = ctx.kernel_stats("gemm_f64")
-                lf = ctx.kernel_stats("potrf_leaf")
+                lf = ctx.kernel_stats("diag_block")
                 ctx.set_kernel_timing(False)
                 if rep:
                     rates.append(st["work"] / st["ms"] / 1e9)
                     builds.append(e0.elapsed_time(e1))
-                    leaf_us.append(1000.0 * lf["ms"] / max(lf["launches"], 1))
+                    diag_us.append(1000.0 * lf["ms"] / max(lf["launches"], 1))
             res.append({"cfg": cfg, "gemm_tflops": float(np.median(rates)),
                         "of_cublas": float(np.median(rates)) / peak,
                         "build_ms": float(np.median(builds)),
-                        "leaf_us_per_launch": float(np.median(leaf_us))})
+                        "diag_us_per_block": float(np.median(diag_us))})
         ctx.set_gemm_tile(1)
         print(json.dumps({"probe": "gemm_tiles", "nssp": args.nssp, "nmeas": nm,
                           "cublas_dgemm_tflops": peak, "configs": res}), flush=True)
@@ -998,6 +998,7 @@ def main():
                                          main_run["launches"], main_run["clocks"])
     value = world * args.steps / (total_ms / 1000.0)
     stats = {f: ctx.kernel_stats(f) for f in ("gemm_f64", "matcov", "matcov_table", "potrf_leaf",
+                                              "diag_block", "crt_int8", "crt_operand", "crt_combine",
                                               "tc_split", "tc_int8")}
 
     # The mixed path is reported beside the FP64 path of the same build: its
@@ -1097,14 +1098,16 @@ def main():
                     "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (no FP64 figure in MEASURED_PEAKS.json)",
                     "traffic": (ratio * s["work"] / s["launches"]) if ratio else None,
                     "launches": s["launches"], "share": share}
-        if fam in ("tc_split", "tc_int8"):
+        if fam in ("tc_split", "tc_int8", "crt_int8"):
             # timed inside a seconds-long build: the sustained (power-capped) peak
             bf16 = float(peaks.get("bf16_tflops_sustained", 1400.0))
-            peak = bf16 * (2.0 if fam == "tc_int8" else 1.0)
+            peak = bf16 * (1.0 if fam == "tc_split" else 2.0)
             achieved = s["work"] / (s["ms"] / 1000.0) / 1e12
-            what = "int8" if fam == "tc_int8" else "fp16/bf16 split"
-            ratio = read_traffic_ratio("tc_gemm_int8_crt_nmeas15936.txt" if fam == "tc_int8"
-                                       else "tc_gemm_f16_trailing_nmeas15936.txt")
+            what = {"tc_int8": "int8", "crt_int8": "int8 residue products of the FP64 path"}.get(
+                fam, "fp16/bf16 split")
+            ratio = None if fam == "crt_int8" else read_traffic_ratio(
+                "tc_gemm_int8_crt_nmeas15936.txt" if fam == "tc_int8"
+                else "tc_gemm_f16_trailing_nmeas15936.txt")
             return {"kernel": f"tc_gemm_kernel ({what} tcgen05, TMA, TMEM)", "bound": "tensor",
                     "achieved": round(achieved, 3), "peak": round(peak, 3),
                     "unit": "TFLOP/s" if fam == "tc_split" else "TOP/s",
@@ -1129,7 +1132,8 @@ def main():
                     "traffic_note": ("bytes stored per launch; at ELT size Cmm (18 GB) exceeds L2 so "
                                      "DRAM writes equal them (ncu on a small case: "
                                      f"{ratio} B per element, the rest still in L2)"),
-                    "real_bound": "FP64 pipe", "fp64_pipe_active": pipe,
+                    "real_bound": "shared-memory reads of the structure-function table",
+                    "fp64_pipe_active": pipe,
                     "launches": s["launches"], "share": share}
         return {"kernel": fam, "ms": s["ms"], "share": share}
 

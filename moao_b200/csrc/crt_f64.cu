@@ -7,9 +7,10 @@
 //             two taken from the system's own diagonal (A's column k times 2^s, B's
 //             times 2^-s), so that a diagonal scaling of the system, whose effect on
 //             the two cancels in FP64, costs no bits here either; then every row of
-//             A and of B is scaled by a power of two and rounded to integers of `bits` bits (X, |X| <= 2^bits, bits as large as the
-//             moduli allow for this K: 57 for K <= 1,024, 53 for K near 2^17), and
-//             stored as centred residues modulo 16 pairwise coprime m_i <= 256;
+//             A and of B is scaled by a power of two and rounded to integers X of
+//             `bits` bits (|X| <= 2^bits, bits as large as the moduli allow for this K:
+//             57 for K <= 1,024, 53 for K near 2^17), and stored as centred residues
+//             modulo 16 pairwise coprime m_i <= 256;
 //   product   one int8 GEMM per modulus with exact int32 sums, reduced modulo m_i
 //             in its epilogue (tc_gemm, all moduli in one launch);
 //   combine   X Y^T from its residues, scaled back and added to C (tc_modz_combine).
@@ -18,10 +19,10 @@
 // rounded additions per element on the FP64 tensor cores.
 //
 // Measured (B200, against the FP64 tensor cores at 28-31 TF/s): the FP64
-// reconstructor at nmeas 29,120 563 -> 201 ms (lookahead and groups included), its Cee/Cvv chain
-// 253 -> 84 ms; the int8 products alone run at 1.7 Pop/s over K = 1,024 and 2.1 over
-// K = 29,120. Error against an FP64 library's result 1.5e-11 -> 1.3e-11 and 1.1e-11 ->
-// 4.4e-12.
+// reconstructor at nmeas 29,120 563 -> 190 ms (lookahead and groups included), its Cee/Cvv chain
+// 253 -> 81 ms; the int8 products alone run at 1.7 Pop/s over K = 1,024 and 2.2 over
+// K = 29,120. Error against an FP64 library's result 1.5e-11 -> 1.3e-11 and 9.9e-12 ->
+// 3.9e-12.
 //
 // Guard: a NaN, an infinity or a magnitude outside 2^-900 .. 2^900 in an operand
 // (found with the row exponents) or a tensor-core wait that ran out raises a flag on
@@ -446,9 +447,11 @@ static moao_status make_balance(moao_ctx* ctx, const CrtBalance* bal, long K, co
   return MOAO_OK;
 }
 
-moao_status crt64_reserve_group(moao_ctx* ctx, long n, long K) {
+moao_status crt64_reserve_group(moao_ctx* ctx, long n, long nb, long K) {
   MOAO_TRY(ctx->cf_flag.ensure(sizeof(int) * kFlags));
   const size_t rows = (size_t)std::max(1L, n);
+  MOAO_TRY(ctx->cf_a.ensure(kNM * rows * round128(nb)));
+  MOAO_TRY(ctx->cf_ma.ensure(sizeof(int) * rows));
   MOAO_TRY(ctx->cf_c.ensure(kNM * rows * round128(K)));
   MOAO_TRY(ctx->cf_mc.ensure(sizeof(int) * rows));
   return ctx->cf_z.ensure(z_bytes(tc_tile_count(n, n, true)));

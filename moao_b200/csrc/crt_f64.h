@@ -36,8 +36,9 @@ moao_status crt64_operand(moao_ctx* ctx, const double* A, long lda, long rows, l
                           CrtOperand* out);
 
 // The same operand for a group of panels, in buffers and under a guard of its own: it
-// outlives the operands of other products. Reserve: for up to n rows, K columns.
-moao_status crt64_reserve_group(moao_ctx* ctx, long n, long K);
+// outlives the operands of other products. Reserve: its buffers for up to n rows and K
+// columns, and those of its panels of nb, so that nothing is allocated in between.
+moao_status crt64_reserve_group(moao_ctx* ctx, long n, long nb, long K);
 moao_status crt64_group_operand(moao_ctx* ctx, const double* A, long lda, long rows, long K,
                                 CrtOperand* out);
 

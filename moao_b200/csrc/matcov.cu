@@ -607,7 +607,7 @@ __global__ void __launch_bounds__(kEWarps * 32, 1)
 // reference indexes the truth sensor at Nsubap_ts * (nW - 1), which assumes
 // every WFS has the same number of valid subapertures; kept as is. Where they are on
 // the common grid, the pair's offset table holds every value (toeplitz_table_kernel):
-// 13.4 -> 0.1 ms for nmeasts 5,824.
+// 13.4 -> 0.1 ms for nmeasts 5,944.
 template <typename OutT>
 __global__ void __launch_bounds__(kTileI* kTileJ)
     matcov_ts_kernel(const DevGeometry g, int r0, int c0, int nrows, int ncols,

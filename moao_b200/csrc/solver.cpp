@@ -215,7 +215,7 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
   if (ahead) {
     MOAO_TRY(ensure_lookahead(ctx));
     MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
-    const moao_status st = crt64_reserve_group(ctx, n - nb, kFactorGroup * nb);
+    const moao_status st = crt64_reserve_group(ctx, n - nb, nb, kFactorGroup * nb);
     if (st != MOAO_OK && st != MOAO_ERR_OOM) return st;
     ahead = st == MOAO_OK;
   }

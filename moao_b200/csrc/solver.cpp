@@ -195,6 +195,7 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
   // the next diagonal block beside what is launched until join(): updates of columns
   // [c0, c1) over K from the first group and [d0, d1) over L from the last
   auto fork = [&](long k0, long c0, long c1, long K, long d0, long d1, long L) -> moao_status {
+    if (ctx->lookahead_sms == 0) return diag_block(k0, ctx->stream);  // the same steps in order
     auto area = [&](long x, long y) { return 0.5 * ((double)(n - x) * (n - x) - (double)(n - y) * (n - y)); };
     const int sms = diag_sms(ctx, 2.0 * 16 / 1.9e15 * (area(c0, c1) * K + area(d0, d1) * L));
     t.max_ctas = std::max(1, nsm - sms);
@@ -205,15 +206,16 @@ moao_status potrf_f64(moao_ctx* ctx, double* A, long lda, long n, double* dinv, 
     return MOAO_OK;
   };
   auto join = [&]() -> moao_status {
+    if (ctx->lookahead_sms == 0) return MOAO_OK;
     MOAO_CUDA_TRY(cudaStreamWaitEvent(ctx->stream, ctx->la_ev[1], 0));
     return MOAO_OK;
   };
   auto ahead_pays = [&](long k1) {  // the update from column k1 on, K = nb
-    return ctx->lookahead_sms > 0 && k1 + nb < n && crt64_pays(ctx, n - k1 - nb, n - k1 - nb, nb, true);
+    return k1 + nb < n && crt64_pays(ctx, n - k1 - nb, n - k1 - nb, nb, true);
   };
   bool ahead = ahead_pays(nb);
   if (ahead) {
-    MOAO_TRY(ensure_lookahead(ctx));
+    if (ctx->lookahead_sms > 0) MOAO_TRY(ensure_lookahead(ctx));
     MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     const moao_status st = crt64_reserve_group(ctx, n - nb, nb, kFactorGroup * nb);
     if (st != MOAO_OK && st != MOAO_ERR_OOM) return st;

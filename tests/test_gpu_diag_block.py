@@ -79,7 +79,4 @@ def test_number_of_ctas_does_not_change_R(prec, built, cuda):
         M.reconstructor(n, m, Cmm, n, Ctm, m, 1, prec=prec, ctx=ctx)
         out.append(Ctm)
         ctx.close()
-    if prec == "mixed":
-        assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
-    else:  # without lookahead the panels are not grouped
-        assert torch.equal(out[0], out[1])
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])

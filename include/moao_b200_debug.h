@@ -50,6 +50,16 @@ moao_status moao_debug_crt64(moao_ctx* ctx, int form, int lower, long M, long N,
                              double alpha, const double* A, long lda, const double* B, long ldb,
                              double beta, double* C, long ldc);
 
+/* Limits for tests of the paths taken where memory is short or a product is large
+ * (0: none, or the default): device bytes the context may hold in workspaces and
+ * geometry, beyond which an allocation fails as on a full device; of the FP64
+ * residue products, the bytes of one operand's residues held at once (at least 256
+ * rows are) and the 128 x 256 tiles of a product per launch. */
+moao_status moao_debug_limits(moao_ctx* ctx, long long workspace_bytes, long long operand_bytes,
+                              long long part_tiles);
+/* Device bytes the context holds in workspaces and geometry (-1: null). */
+long long moao_debug_bytes_held(moao_ctx* ctx);
+
 #ifdef __cplusplus
 }
 #endif

@@ -24,6 +24,8 @@ moao_status set_error(moao_status s, const std::string& msg) {
 moao_status DevBuf::ensure(size_t n) {
   if (n <= bytes) return MOAO_OK;
   release();
+  if (owner && owner->workspace_limit && owner->bytes_held() + n > owner->workspace_limit)
+    return set_error(MOAO_ERR_OOM, std::to_string(n) + " bytes exceed the workspace limit");
   cudaError_t e = cudaMalloc(&p, n);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -602,6 +604,23 @@ moao_status moao_debug_residual(moao_ctx* c, int scheme, long m, long n, const d
   std::lock_guard<std::mutex> lk(c->mu);
   MOAO_CUDA_TRY(cudaSetDevice(c->device));
   return debug_residual(c, scheme, m, n, R, ldR, Cmm, ldCmm, Ctm, ldCtm, E, ldE);
+}
+
+moao_status moao_debug_limits(moao_ctx* c, long long workspace_bytes, long long operand_bytes,
+                              long long part_tiles) {
+  if (!c || workspace_bytes < 0 || operand_bytes < 0 || part_tiles < 0)
+    return set_error(MOAO_ERR_BAD_ARG, "debug_limits: limits >= 0");
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->workspace_limit = (size_t)workspace_bytes;
+  c->cf_operand_bytes = (size_t)operand_bytes;
+  c->cf_part_tiles = (long)part_tiles;
+  return MOAO_OK;
+}
+
+long long moao_debug_bytes_held(moao_ctx* c) {
+  if (!c) return -1;
+  std::lock_guard<std::mutex> lk(c->mu);
+  return (long long)c->bytes_held();
 }
 
 int moao_debug_crt_moduli(int ns, long K) { return crt_moduli_for(ns, K); }

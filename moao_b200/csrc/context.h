@@ -24,7 +24,9 @@ namespace moao {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  moao_ctx* owner = nullptr;  // a context's workspace: counts against its limit
   unsigned long long generation = 0;  // bumped by every (re)allocation and release
+  // At least n bytes, contents undefined after growth; MOAO_ERR_OOM leaves it empty.
   moao_status ensure(size_t n);
   void release();
   template <typename T>
@@ -75,6 +77,11 @@ struct moao_ctx {
                          // (a collective's kernels may hold some)
   bool chained = true;  // chained launches of the small FP64 kernels (off under stream capture)
   bool crt_f64 = true;  // off where nothing may be allocated (stream capture, no-alloc calls)
+  // Limits of the residue products that tests lower (0: the defaults in crt_f64.cu):
+  // bytes of one operand's residues held at once, tiles of a product per launch.
+  size_t cf_operand_bytes = 0;
+  long cf_part_tiles = 0;
+  size_t workspace_limit = 0;  // bytes_held above which an allocation fails (0: none; tests)
   long mx_factored_n = -1;  // size of the factorisation held in mx_* (reuse across targets)
   // Block-constant offsets of Cmm known to the caller (moao_ctx_set_offsets):
   // the mixed path factors Cmm minus them and adds them back exactly.
@@ -142,6 +149,9 @@ struct moao_ctx {
   std::vector<Pending> pending;
   std::vector<cudaEvent_t> event_pool;
 
+  moao_ctx() {
+    for (moao::DevBuf* b : workspaces()) b->owner = this;
+  }
   // Every workspace buffer of the context (not the geometry caches).
   std::vector<moao::DevBuf*> workspaces() {
     return {&ws_w,  &ws_dinv, &ws_info, &ws_tmp, &ws_host_t, &ws_corner, &mx_a32, &mx_lr,  &mx_lc,    &mx_t32,

@@ -320,8 +320,16 @@ long round128(long x) { return (x + 127) / 128 * 128; }
 
 }  // namespace
 
-static size_t z_bytes(long tiles) {
-  return (size_t)std::min(tiles, kPartTiles) * kNM * kTcZTile;
+static long part_tiles(const moao_ctx* ctx) {
+  return ctx->cf_part_tiles > 0 ? ctx->cf_part_tiles : kPartTiles;
+}
+static size_t z_bytes(const moao_ctx* ctx, long tiles) {
+  return (size_t)std::min(tiles, part_tiles(ctx)) * kNM * kTcZTile;
+}
+// Rows of an operand over K whose residues are held at once.
+static long part_rows(const moao_ctx* ctx, long K) {
+  const size_t bytes = ctx->cf_operand_bytes ? ctx->cf_operand_bytes : kOperandBytes;
+  return std::max(256L, (long)(bytes / ((size_t)kNM * round128(K))) / 256 * 256);
 }
 
 bool crt64_pays(const moao_ctx* ctx, long M, long N, long K, bool lower) {
@@ -347,7 +355,7 @@ size_t crt64_bytes(long n, long m, long nb, long nact) {
     const size_t row = (size_t)round128(K) * kNM;
     qa = std::max(qa, std::min(kOperandBytes, row * (size_t)M));
     qb = std::max(qb, std::min(kOperandBytes / share, row * (size_t)N));
-    z = std::max(z, z_bytes(tc_tile_count(M, N, lower)));
+    z = std::max(z, z_bytes(&c, tc_tile_count(M, N, lower)));
     small = std::max(small, sizeof(int) * (size_t)(M + N + K + kMaxChunks + 1));
   };
   const long rest = n - nb;
@@ -358,7 +366,7 @@ size_t crt64_bytes(long n, long m, long nb, long nact) {
   size_t qc = 0;
   if (crt64_pays(&c, rest - nb, rest - nb, nb, true)) {
     qc = (size_t)round128(kFactorGroup * nb) * kNM * rest + sizeof(int) * (size_t)rest;
-    z = std::max(z, z_bytes(tc_tile_count(rest, rest, true)));
+    z = std::max(z, z_bytes(&c, tc_tile_count(rest, rest, true)));
   }
   if (crt64_pays(&c, m, nb, nb, false)) {
     product(m, kSolveGroup * nb, nb, false, 1);
@@ -447,14 +455,27 @@ static moao_status make_balance(moao_ctx* ctx, const CrtBalance* bal, long K, co
   return MOAO_OK;
 }
 
-moao_status crt64_reserve_group(moao_ctx* ctx, long n, long nb, long K) {
+// Buffers of products of up to rows_a x rows_b over K and `tiles` tiles. A product that
+// adds to C takes all it needs here before it writes: MOAO_ERR_OOM then means that C is
+// as given, and the caller may compute it another way. rows_b 0: one operand; bal: with
+// a balance along K.
+static moao_status reserve(moao_ctx* ctx, long rows_a, long rows_b, long K, bool bal, long tiles) {
   MOAO_TRY(ctx->cf_flag.ensure(sizeof(int) * kFlags));
-  const size_t rows = (size_t)std::max(1L, n);
-  MOAO_TRY(ctx->cf_a.ensure(kNM * rows * round128(nb)));
-  MOAO_TRY(ctx->cf_ma.ensure(sizeof(int) * rows));
-  MOAO_TRY(ctx->cf_c.ensure(kNM * rows * round128(K)));
-  MOAO_TRY(ctx->cf_mc.ensure(sizeof(int) * rows));
-  return ctx->cf_z.ensure(z_bytes(tc_tile_count(n, n, true)));
+  MOAO_TRY(ctx->cf_a.ensure((size_t)kNM * rows_a * round128(K)));
+  MOAO_TRY(ctx->cf_ma.ensure(sizeof(int) * (size_t)rows_a));
+  if (rows_b > 0) {
+    MOAO_TRY(ctx->cf_b.ensure((size_t)kNM * rows_b * round128(K)));
+    MOAO_TRY(ctx->cf_mb.ensure(sizeof(int) * (size_t)rows_b));
+  }
+  if (bal) MOAO_TRY(ctx->cf_k.ensure(sizeof(int) * (size_t)K));
+  return ctx->cf_z.ensure(z_bytes(ctx, tiles));
+}
+
+moao_status crt64_reserve_group(moao_ctx* ctx, long n, long nb, long K) {
+  const long rows = std::max(1L, n);
+  MOAO_TRY(reserve(ctx, rows, 0, nb, false, tc_tile_count(n, n, true)));
+  MOAO_TRY(ctx->cf_c.ensure((size_t)kNM * rows * round128(K)));
+  return ctx->cf_mc.ensure(sizeof(int) * (size_t)rows);
 }
 
 moao_status crt64_group_operand(moao_ctx* ctx, const double* A, long lda, long rows, long K,
@@ -493,9 +514,9 @@ moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const Crt
   g.lower = f.lowerC ? 1 : 0;
   g.max_ctas = max_ctas;
   const long total = tc_tile_count(M, N, f.lowerC);
-  const long part = kPartTiles, parts = (total + part - 1) / part;
+  const long part = part_tiles(ctx), parts = (total + part - 1) / part;
   if (parts > kMaxChunks) return set_error(MOAO_ERR_UNSUPPORTED, "crt64: product too large");
-  MOAO_TRY(ctx->cf_z.ensure(z_bytes(total)));
+  MOAO_TRY(ctx->cf_z.ensure(z_bytes(ctx, total)));
   MOAO_CUDA_TRY(cudaMemsetAsync(flag + 1, 0, sizeof(int) * (size_t)parts, s));
   g.C = ctx->cf_z.p;
   TcModz z;
@@ -532,9 +553,13 @@ moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const Crt
 
 moao_status crt64_gemm(moao_ctx* ctx, const GemmArgs& g, const CrtBalance* bal) {
   // the operands' rows in parts that fit the residue buffers
-  const size_t per_row = (size_t)kNM * round128(g.K);
-  const long part = std::max(256L, (long)(kOperandBytes / per_row) / 256 * 256);
+  const long part = part_rows(ctx, g.K);
   const bool same = g.transB && g.A == g.B && g.lda == g.ldb && g.M == g.N && g.M <= part;
+  // the first part is the largest, but of a lower C it is a triangle, and a part below
+  // it may hold more tiles
+  long tiles = tc_tile_count(std::min(part, g.M), std::min(part, g.N), g.lowerC);
+  if (g.lowerC && g.M > part) tiles = std::max(tiles, tc_tile_count(std::min(part, g.M - part), part, false));
+  MOAO_TRY(reserve(ctx, std::min(part, g.M), same ? 0 : std::min(part, g.N), g.K, bal && !same, tiles));
   for (long n0 = 0; n0 < g.N; n0 += part) {
     const long nn = std::min(part, g.N - n0);
     for (long m0 = g.lowerC ? n0 : 0; m0 < g.M; m0 += part) {
@@ -566,8 +591,11 @@ moao_status crt64_gemm(moao_ctx* ctx, const GemmArgs& g, const CrtBalance* bal) 
 
 moao_status crt64_symm(moao_ctx* ctx, long M, long n, const double* A, long lda, const double* B,
                        long ldb, double* C, long ldc) {
-  const size_t per_row = (size_t)kNM * round128(n);
-  const long part = std::max(256L, (long)(kOperandBytes / per_row) / 256 * 256);
+  // columns of S in parts of an eighth of the buffer: their residues are written
+  // and read once each
+  const long part = part_rows(ctx, n), cpart = std::max(256L, part / 8 / 256 * 256);
+  MOAO_TRY(reserve(ctx, std::min(part, M), std::min(cpart, n), n, true,
+                   tc_tile_count(std::min(part, M), std::min(cpart, n), false)));
   for (long m0 = 0; m0 < M; m0 += part) {
     const long mm = std::min(part, M - m0);
     MOAO_TRY(crt64_begin(ctx));
@@ -576,9 +604,6 @@ moao_status crt64_symm(moao_ctx* ctx, long M, long n, const double* A, long lda,
     const CrtBalance bal{B, ldb + 1, 1, 1};  // S's own diagonal: A(:, k) goes with S(k, :)
     MOAO_TRY(make_balance(ctx, &bal, n, &off));
     MOAO_TRY(make_operand(ctx, 0, CRT_ROWS, A + m0, lda, mm, n, 0, off, 1, &a));
-    // columns of S in parts of an eighth of the buffer: their residues are written
-    // and read once each
-    const long cpart = std::max(256L, part / 8 / 256 * 256);
     for (long c0 = 0; c0 < n; c0 += cpart) {
       const long cc = std::min(cpart, n - c0);
       MOAO_TRY(make_operand(ctx, 1, CRT_SYM, B, ldb, cc, n, c0, off, -1, &b));

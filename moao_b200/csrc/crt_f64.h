@@ -58,7 +58,7 @@ struct CrtBalance {
   int half, sign;
 };
 
-// g (triB: full) by residue products, operands included.
+// g (triB: full) by residue products, operands included. MOAO_ERR_OOM: C is as given.
 moao_status crt64_gemm(moao_ctx* ctx, const GemmArgs& g, const CrtBalance* bal);
 // C (M x n) = A (M x n) S, S the symmetric n x n matrix in the lower triangle of B.
 moao_status crt64_symm(moao_ctx* ctx, long M, long n, const double* A, long lda, const double* B,

@@ -37,12 +37,24 @@ moao_status gemm(moao_ctx* ctx, long M, long N, long K, double alpha, const doub
   return gemm_f64(g, ctx->stream, &ctx->launches);
 }
 
+// Whether a product goes by residues. Under stream capture it does not: their buffers
+// cannot be allocated there, and a graph would keep addresses that a later call moves.
+static bool by_residues(const moao_ctx* ctx, long M, long N, long K, bool lower) {
+  if (!crt64_pays(ctx, M, N, K, lower)) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &cap) != cudaSuccess) {
+    cudaGetLastError();  // the legacy stream while another one captures
+    return false;
+  }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
 // The same product by int8 residue products where those are faster (crt_f64.cu);
 // the FP64 tensor cores where not, or where their buffers do not fit.
 moao_status gemm_long(moao_ctx* ctx, long M, long N, long K, double alpha, const double* A,
                       long lda, const double* B, long ldb, bool transB, double beta, double* C,
                       long ldc, bool lowerC = false, const CrtBalance* bal = nullptr) {
-  if (crt64_pays(ctx, M, N, K, lowerC)) {
+  if (by_residues(ctx, M, N, K, lowerC)) {
     GemmArgs g;
     g.M = M; g.N = N; g.K = K; g.alpha = alpha; g.beta = beta;
     g.A = A; g.lda = lda; g.B = B; g.ldb = ldb; g.transB = transB;
@@ -56,7 +68,7 @@ moao_status gemm_long(moao_ctx* ctx, long M, long N, long K, double alpha, const
 // C (M x n) = A (M x n) S, S the symmetric n x n matrix in the lower triangle of B.
 moao_status symm_right(moao_ctx* ctx, long M, long n, const double* A, long lda, const double* B,
                        long ldb, double* C, long ldc) {
-  if (crt64_pays(ctx, M, n, n, false)) {
+  if (by_residues(ctx, M, n, n, false)) {
     const moao_status st = crt64_symm(ctx, M, n, A, lda, B, ldb, C, ldc);
     if (st != MOAO_ERR_OOM) return st;
   }

@@ -241,12 +241,14 @@ moao_status run_batch(moao_ctx* ctx, int count, moao_batch_item* items, moao_bat
     }
     return b;
   };
-  // Budget: what is free plus what the sub-contexts already hold (reused).
+  // Budget: what is free plus what the sub-contexts already hold (reused) and what the
+  // context would give back (its residue buffers).
   size_t fr = 0, tot = 0, held = 0;
   MOAO_CUDA_TRY(cudaMemGetInfo(&fr, &tot));
   for (moao_ctx* c : sub_contexts(ctx)) held += c->bytes_held();
-  const size_t budget_all = o->hbm_budget_gb > 0 ? (size_t)(o->hbm_budget_gb * 1e9)
-                                                 : (size_t)(0.85 * (double)(fr + held));
+  const size_t budget_all = o->hbm_budget_gb > 0
+                                ? (size_t)(o->hbm_budget_gb * 1e9)
+                                : (size_t)(0.85 * (double)(fr + held + ctx->residue_bytes()));
   if (pk_bytes > budget_all)
     return set_error(MOAO_ERR_OOM, "batch: the packed instances exceed the device budget");
   const size_t budget = budget_all - pk_bytes;
@@ -298,6 +300,7 @@ moao_status run_batch(moao_ctx* ctx, int count, moao_batch_item* items, moao_bat
     per[k].push_back(i);
   }
   S = (int)per.size();
+  if ((double)(planned + pk_bytes) > 0.85 * (double)(fr + held)) ctx->release_residues();
   // Workspaces kept from earlier batches: drop those much larger than this
   // plan needs and those of streams this batch does not use.
   {

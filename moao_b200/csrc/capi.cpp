@@ -24,19 +24,29 @@ moao_status set_error(moao_status s, const std::string& msg) {
 moao_status DevBuf::ensure(size_t n) {
   if (n <= bytes) return MOAO_OK;
   release();
-  if (owner && owner->workspace_limit && owner->bytes_held() + n > owner->workspace_limit)
-    return set_error(MOAO_ERR_OOM, std::to_string(n) + " bytes exceed the workspace limit");
-  cudaError_t e = cudaMalloc(&p, n);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    p = nullptr;
-    bytes = 0;
-    return set_error(MOAO_ERR_OOM, "cudaMalloc of " + std::to_string(n) + " bytes failed: " +
-                                       cudaGetErrorString(e));
-  }
+  if (allocate(n)) return MOAO_OK;
+  if (owner && !optional && owner->release_residues() > 0 && allocate(n)) return MOAO_OK;
+  return set_error(MOAO_ERR_OOM, "no device memory for " + std::to_string(n) + " bytes");
+}
+
+static bool try_malloc(moao_ctx* owner, void** p, size_t n) {
+  if (owner && owner->workspace_limit && owner->bytes_held() + n > owner->workspace_limit) return false;
+  if (cudaMalloc(p, n) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
+bool DevBuf::allocate(size_t n) {
+  if (!try_malloc(owner, &p, n)) return false;
   bytes = n;
   ++generation;
-  return MOAO_OK;
+  return true;
+}
+
+bool device_alloc(moao_ctx* ctx, void** p, size_t bytes) {
+  std::lock_guard<std::mutex> lk(ctx->mu);
+  return try_malloc(ctx, p, bytes) || (ctx->release_residues() > 0 && try_malloc(ctx, p, bytes));
 }
 
 void DevBuf::release() {
@@ -158,6 +168,7 @@ moao_status device_geometry(moao_ctx* ctx, const moao_tomo* tp, const DevGeometr
   }
   for (int k = 0; k < nW * nL; ++k) h[olay + 3 * nL + k] = t.sspSizeL[k];
   for (int l = 0; l < nL; ++l) h[olay + 3 * nL + nW * nL + l] = t.atm.h[l];
+  e.buf.owner = ctx;
   MOAO_TRY(e.buf.ensure(total_all * sizeof(double)));
   double* d = e.buf.as<double>();
   MOAO_CUDA_TRY(cudaMemcpyAsync(d, h.data(), total * sizeof(double), cudaMemcpyHostToDevice,
@@ -911,7 +922,7 @@ moao_status moao_cee_cvv_host(moao_ctx* ctx, long nmeas, long nmeasts, long nact
   cudaStream_t s = ctx->stream;
   moao_status st = MOAO_OK;
   for (auto& m : mats) {
-    if (cudaMalloc(&m.d, sizeof(double) * std::max(1L, m.m * m.n)) != cudaSuccess) {
+    if (!device_alloc(ctx, (void**)&m.d, sizeof(double) * std::max(1L, m.m * m.n))) {
       st = set_error(MOAO_ERR_OOM, "Cee_Cvv_host: device allocation");
       break;
     }

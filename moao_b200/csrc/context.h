@@ -24,11 +24,15 @@ namespace moao {
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
-  moao_ctx* owner = nullptr;  // a context's workspace: counts against its limit
+  moao_ctx* owner = nullptr;  // a context's buffer: counts against its limit
+  bool optional = false;      // the owner's calls run without it: gives way to the others
   unsigned long long generation = 0;  // bumped by every (re)allocation and release
   // At least n bytes, contents undefined after growth; MOAO_ERR_OOM leaves it empty.
   moao_status ensure(size_t n);
   void release();
+ private:
+  bool allocate(size_t n);
+ public:
   template <typename T>
   T* as() const { return static_cast<T*>(p); }
 };
@@ -151,6 +155,7 @@ struct moao_ctx {
 
   moao_ctx() {
     for (moao::DevBuf* b : workspaces()) b->owner = this;
+    for (moao::DevBuf* b : residue_buffers()) b->optional = true;
   }
   // Every workspace buffer of the context (not the geometry caches).
   std::vector<moao::DevBuf*> workspaces() {
@@ -158,6 +163,22 @@ struct moao_ctx {
             &mx_w1, &mx_w2,   &mx_x,    &mx_r64, &mx_e64, &mx_qa,  &mx_qb,    &mx_ea,
             &mx_fb, &mx_colmax, &mx_norm, &mx_rid, &mx_y, &mx_y2, &mx_zu, &mx_sinv, &mx_exps,
             &mx_dsl, &cx_qc, &cx_ec, &ws_sync, &cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z, &cf_flag};
+  }
+  // The FP64 residue products' buffers: kept from call to call, but an allocation that
+  // would fail beside them takes their room (FP64 calls run without them).
+  std::vector<moao::DevBuf*> residue_buffers() {
+    return {&cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z};
+  }
+  size_t residue_bytes() {
+    size_t b = 0;
+    for (moao::DevBuf* d : residue_buffers()) b += d->bytes;
+    return b;
+  }
+  // Gives them back (cudaFree waits for the device); the bytes.
+  size_t release_residues() {
+    const size_t b = residue_bytes();
+    for (moao::DevBuf* d : residue_buffers()) d->release();
+    return b;
   }
   // Device bytes held by the workspaces and the geometry caches.
   size_t bytes_held() {
@@ -186,6 +207,10 @@ class KernelTimer {
 };
 // Folds completed event pairs into the per-family totals (synchronises).
 moao_status collect_kernel_stats(moao_ctx* ctx);
+
+// cudaMalloc for a call's own buffers (not under ctx->mu): with the room of the context's
+// residue buffers where there is none beside them. false: no memory.
+bool device_alloc(moao_ctx* ctx, void** p, size_t bytes);
 
 // Uploads (or reuses) the device copy of a tomo's geometry tables.
 moao_status device_geometry(moao_ctx* ctx, const moao_tomo* t, const DevGeometry** out);

@@ -335,7 +335,7 @@ moao_status moao_intersample_create(moao_ctx* ctx, long nidx, long np, double Dt
   const size_t NN = (size_t)N * N;
   moao_status st = MOAO_OK;
   auto alloc = [&](void** p, size_t bytes) {
-    if (st == MOAO_OK && cudaMalloc(p, bytes) != cudaSuccess)
+    if (st == MOAO_OK && !device_alloc(ctx, p, bytes))
       st = set_error(MOAO_ERR_OOM, "intersample_create: device allocation");
   };
   alloc((void**)&is->abs2fi, NN * 8);
@@ -430,9 +430,9 @@ moao_status moao_intersample_process_host(moao_isample* is, const double* Cvv, d
   MOAO_CUDA_TRY(cudaSetDevice(ctx->device));
   const long N = is->info.N;
   double *dc = nullptr, *dp = nullptr;
-  if (cudaMalloc(&dc, is->info.nidx * 8) != cudaSuccess)
+  if (!device_alloc(ctx, (void**)&dc, is->info.nidx * 8))
     return set_error(MOAO_ERR_OOM, "intersample_process_host: Cvv");
-  if (cudaMalloc(&dp, N * N * 8) != cudaSuccess) {
+  if (!device_alloc(ctx, (void**)&dp, N * N * 8)) {
     cudaFree(dc);
     return set_error(MOAO_ERR_OOM, "intersample_process_host: psf");
   }

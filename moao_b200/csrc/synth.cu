@@ -148,9 +148,9 @@ extern "C" moao_status moao_intersample_inputs(moao_ctx* ctx, long nssp, double 
   const double scale = ud / (Dtel / 2.0);
   Cplx* z = nullptr;
   double* d = nullptr;
-  if (cudaMalloc(&z, sizeof(Cplx) * NN) != cudaSuccess)
+  if (!device_alloc(ctx, (void**)&z, sizeof(Cplx) * NN))
     return set_error(MOAO_ERR_OOM, "intersample_inputs: device buffer");
-  if (cudaMalloc(&d, sizeof(double) * NN) != cudaSuccess) {
+  if (!device_alloc(ctx, (void**)&d, sizeof(double) * NN)) {
     cudaFree(z);
     return set_error(MOAO_ERR_OOM, "intersample_inputs: device buffer");
   }

@@ -414,7 +414,7 @@ typedef struct {
   double refine_resid;
   double queue_ms, run_ms, latency_ms;  /* submit->start, start->done, submit->done */
   double start_ms, end_ms;              /* start and end, ms since server creation */
-  double footprint_gb;   /* device bytes admitted for it */
+  double footprint_gb;   /* device bytes it was admitted with (optional buffers aside) */
   char message[256];     /* error text when status is an error */
 } moao_request_result;
 typedef struct {

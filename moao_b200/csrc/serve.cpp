@@ -11,6 +11,11 @@
 // starts as soon as a slot and memory free up, not when the batch drains).
 // The head of the queue is never bypassed, so a large request cannot starve.
 //
+// An FP64 request runs faster with the residue products' buffers (crt_f64.cu) but does
+// not need them: they are no part of what it is admitted with. It gets them where they
+// fit the budget and take no other request's place; else it runs on the FP64 tensor
+// cores. What an idle slot keeps of them goes before a request has to wait for memory.
+//
 // Per request on its slot: set the profile and target; matcov Cmm (type 1)
 // and Ctm (type 3); reconstructor (FP64 or mixed with the model's LGS
 // offsets declared); if Cvv is wanted, Ctm and Ctt (type 4) again and Cee/Cvv
@@ -63,7 +68,10 @@ struct Request {
   long long id = 0;
   moao_request r{};
   std::vector<double> cn2, h, L0;
-  size_t footprint = 0;
+  size_t footprint = 0;  // device bytes it cannot do without
+  size_t residues = 0;   // of the residue products
+  size_t extra = 0;      // of them (or of its slot's kept ones), what it was admitted with
+  size_t charge() const { return footprint + extra; }
   Clock::time_point t_submit, t_start, t_done;
   moao_request_result res{};
   bool done = false, cancelled = false, running = false;
@@ -82,6 +90,7 @@ struct Slot {
   std::map<int, SlotSystem> systems;
   std::shared_ptr<Request> job;
   size_t held = 0;  // device bytes this slot holds (buffers, workspaces, geometry)
+  size_t residues = 0;  // of them, the residue products'
   std::thread thread;
 };
 
@@ -100,6 +109,7 @@ struct moao_server {
   long long next_id = 1;
   bool stopping = false;
   size_t in_flight_bytes = 0;
+  size_t smallest = 0, largest = 0;  // footprints submitted so far
   moao_server_stats stats{};
   std::thread scheduler;
   std::chrono::steady_clock::time_point t0 = std::chrono::steady_clock::now();
@@ -123,13 +133,19 @@ size_t footprint(const moao_server* s, const System& sys, const moao_request& r)
     f += 2 * bytes_of(n, nb);
   }
   const bool cvv = (r.Cvv || r.psf) && a > 0;
-  if (r.prec != MOAO_PREC_MIXED) f += crt64_bytes(n, m, nb, cvv ? a : 0);
   if (cvv) f += 2 * bytes_of(m, m) + bytes_of(a, a) + 3 * bytes_of(a, m) + bytes_of(m, n);
   if (r.psf && sys.has_psf)
     f += bytes_of(sys.psf_n, sys.psf_n) * 7 + sizeof(int) * 2 * (size_t)sys.idx.size();
   // geometry tables (u, v per layer, per-WFS tables)
   f += sizeof(double) * (size_t)sys.tomo.Nx * (2 * (size_t)r.nlayer + 8) + (1 << 20);
   return f;
+}
+
+// Device bytes of its residue products, which it can run without.
+size_t residues_of(const moao_server* s, const System& sys, const moao_request& r) {
+  if (r.prec == MOAO_PREC_MIXED) return 0;  // nor does a fallback to FP64 use them
+  const bool cvv = (r.Cvv || r.psf) && sys.nact > 0;
+  return crt64_bytes(sys.nmeas, sys.nmeasts, s->opt.nb > 0 ? s->opt.nb : 1024, cvv ? sys.nact : 0);
 }
 
 void finish(moao_server* s, Slot& slot, const std::shared_ptr<Request>& q, moao_status st,
@@ -149,7 +165,8 @@ void finish(moao_server* s, Slot& slot, const std::shared_ptr<Request>& q, moao_
   std::snprintf(q->res.message, sizeof(q->res.message), "%s", err.c_str());
   q->done = true;
   q->running = false;
-  s->in_flight_bytes -= q->footprint;
+  s->in_flight_bytes -= q->charge();
+  if (!s->opt.dry_run && slot.ctx) slot.residues = slot.ctx->residue_bytes();
   if (!s->opt.dry_run && slot.ctx) slot.held = slot.ctx->bytes_held() + slot.cmm.bytes +
                                                slot.ctm.bytes + slot.ctt.bytes + slot.cee.bytes +
                                                slot.cvv.bytes + slot.tmp.bytes + slot.dx.bytes +
@@ -182,6 +199,7 @@ moao_status run_request(moao_server* s, Slot& slot, Request& q, moao_solve_repor
   const bool mixed = q.r.prec == MOAO_PREC_MIXED;
   if (mixed) MOAO_TRY(moao_ctx_set_offsets_from_tomo(ctx, ss.tomo.get()));
   ctx->keep_cmm = mixed;
+  ctx->crt_f64 = q.residues > 0 && q.extra > 0;
   moao_status st = moao_reconstructor(ctx, n, m, Cmm, n, Ctm, m, 1, q.r.prec, rep);
   ctx->keep_cmm = false;
   if (st != MOAO_OK) return st;
@@ -258,6 +276,50 @@ void slot_main(moao_server* s, Slot* slot) {
   }
 }
 
+// Gives back what an idle slot keeps of the residue products' buffers.
+void drop_residues(moao_server* s, Slot& sl) {
+  if (sl.residues == 0) return;
+  if (!s->opt.dry_run) {
+    cudaSetDevice(s->opt.device);
+    sl.ctx->release_residues();
+  }
+  sl.held -= std::min(sl.held, sl.residues);
+  sl.residues = 0;
+}
+
+// Requests of `unit` bytes that the slots idle beside `mine` could take within the budget
+// if it were charged with `charge`.
+int fit_beside(const moao_server* s, const Slot& mine, size_t charge, size_t unit) {
+  size_t total = charge;
+  for (auto& sl : s->slots)
+    if (sl.get() != &mine) total += sl->job ? std::max(sl->held, sl->job->charge()) : sl->held;
+  int n = 0;
+  for (auto& sl : s->slots) {
+    if (sl.get() == &mine || sl->job) continue;
+    total += std::max(sl->held, unit) - sl->held;
+    if (total > s->budget) break;
+    ++n;
+  }
+  return n;
+}
+
+// Bytes of the residue products' buffers that q is admitted with on slot sl (its own, or
+// what the slot keeps of another request's): where they fit the budget and leave the
+// other idle slots room for as many requests as without them, of its own size and of
+// the smallest and largest seen; else 0.
+size_t residues_admitted(const moao_server* s, const Slot& sl, const Request& q) {
+  const size_t extra = std::max(q.residues, sl.residues);
+  const size_t without = std::max(sl.held - std::min(sl.held, sl.residues), q.footprint);
+  const size_t with = std::max(sl.held, q.footprint + extra);
+  size_t total = with;
+  for (auto& o : s->slots)
+    if (o.get() != &sl) total += o->job ? std::max(o->held, o->job->charge()) : o->held;
+  if (total > s->budget) return 0;
+  for (size_t unit : {q.footprint, s->smallest, s->largest})
+    if (fit_beside(s, sl, with, unit) < fit_beside(s, sl, without, unit)) return 0;
+  return extra;
+}
+
 // Admits queue heads while a slot is idle and the head fits. Called with mu held.
 void admit(moao_server* s) {
   while (!s->queue.empty()) {
@@ -271,7 +333,7 @@ void admit(moao_server* s) {
     Slot* best = nullptr;
     size_t best_need = 0;
     size_t total_held = 0;
-    for (auto& sl : s->slots) total_held += sl->job ? std::max(sl->held, sl->job->footprint) : sl->held;
+    for (auto& sl : s->slots) total_held += sl->job ? std::max(sl->held, sl->job->charge()) : sl->held;
     for (auto& sl : s->slots) {
       if (sl->job) continue;
       const size_t need = total_held - sl->held + std::max(sl->held, q->footprint);
@@ -281,6 +343,13 @@ void admit(moao_server* s) {
       }
     }
     if (!best) {
+      bool dropped = false;
+      for (auto& sl : s->slots)
+        if (!sl->job && sl->residues > 0) {
+          drop_residues(s, *sl);
+          dropped = true;
+        }
+      if (dropped) continue;
       // free an idle slot's resident buffers if that makes the head fit
       for (auto& sl : s->slots) {
         if (sl->job || sl->held == 0) continue;
@@ -293,7 +362,7 @@ void admit(moao_server* s) {
                               &sl->psf})
               b->release();
           }
-          sl->held = 0;
+          sl->held = sl->residues = 0;
           best = sl.get();
           best_need = total_held - 0 + q->footprint;
           break;
@@ -305,14 +374,19 @@ void admit(moao_server* s) {
     q->running = true;
     q->t_start = Clock::now();
     q->res.footprint_gb = q->footprint / 1e9;
-    s->in_flight_bytes += q->footprint;
+    q->extra = residues_admitted(s, *best, *q);
+    if (q->extra == 0) drop_residues(s, *best);
+    s->in_flight_bytes += q->charge();
     best->job = q;
-    if (s->opt.dry_run) best->held = std::max(best->held, q->footprint);
+    if (s->opt.dry_run) {
+      best->held = std::max(best->held, q->charge());
+      best->residues = q->extra;
+    }
     int busy = 0;
     for (auto& sl : s->slots) busy += sl->job ? 1 : 0;
     s->stats.max_in_flight = std::max(s->stats.max_in_flight, busy);
     size_t admitted = 0;
-    for (auto& sl : s->slots) admitted += sl->job ? std::max(sl->held, sl->job->footprint) : sl->held;
+    for (auto& sl : s->slots) admitted += sl->job ? std::max(sl->held, sl->job->charge()) : sl->held;
     s->stats.peak_admitted_gb = std::max(s->stats.peak_admitted_gb, admitted / 1e9);
     s->cv_slot.notify_all();
   }
@@ -475,6 +549,7 @@ moao_status moao_serve_submit(moao_server* s, const moao_request* r, long long* 
   if (r->psf && !sys.has_psf)
     return set_error(MOAO_ERR_BAD_ARG, "serve_submit: PSF needs a system registered with its tables");
   q->footprint = footprint(s, sys, *r);
+  q->residues = residues_of(s, sys, *r);
   if (q->footprint > s->budget) {
     ++s->stats.rejected;
     return set_error(MOAO_ERR_OOM, "serve_submit: request needs " + std::to_string(q->footprint) +
@@ -489,6 +564,8 @@ moao_status moao_serve_submit(moao_server* s, const moao_request* r, long long* 
   q->res.status = MOAO_ERR_BUSY;
   s->requests[q->id] = q;
   s->queue.push_back(q);
+  s->smallest = s->smallest ? std::min(s->smallest, q->footprint) : q->footprint;
+  s->largest = std::max(s->largest, q->footprint);
   ++s->stats.submitted;
   *id = q->id;
   s->cv_sched.notify_all();

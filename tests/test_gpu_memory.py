@@ -133,3 +133,38 @@ def test_batch_after_fp64(own, tmp_path):
     got = outs[1].clone()
     assert batch(1) == 0
     assert torch.equal(got, outs[1]) and bool(torch.isfinite(got).all())
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_server_stays_in_its_budget(built, cuda, tmp_path, prec):
+    """A budget without room for residue buffers: the request runs, its result is that of
+    a roomy server within the FP64 products' accuracy (kappa of these systems is below
+    1e6, so 1e-9 covers n eps kappa), and the slot's memory stays inside the budget."""
+    import torch
+    from moao_b200.serve import Server
+    s, a = P.config_scaled(24, 3)
+    P.write_system(str(tmp_path), s, a)
+    files = os.path.join(tmp_path, "sys-params.txt"), os.path.join(tmp_path, "prof-1-atmos-night0.txt")
+    prof = np.array(a.cn2), np.array(a.h), np.array(a.L0)
+    out, foot = [], None
+    for k in range(2):
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        free = torch.cuda.mem_get_info()[0]
+        budget = 60.0 if k == 0 else 1.001 * foot
+        with Server(slots=1, hbm_budget_gb=budget) as srv:
+            sid = srv.add_system(*files)
+            info = srv.system_info(sid)
+            R = np.zeros(info["nmeas"] * info["nmeasts"])
+            r = srv.wait(srv.submit(sid, *prof, prec=prec, R=R))
+            assert r["status"] == 0, r
+            foot = r["footprint_gb"]
+            used = (free - torch.cuda.mem_get_info()[0]) / 1e9
+            admitted = srv.stats()["peak_admitted_gb"]
+            # streams, modules and the structure-function table come on top
+            assert used <= admitted + 0.1, (used, admitted, foot)
+            assert admitted <= budget
+            if prec == "fp64":
+                assert (admitted > 1.2 * foot) == (k == 0)
+        out.append(R)
+    assert np.linalg.norm(out[0] - out[1]) <= 1e-9 * np.linalg.norm(out[1])

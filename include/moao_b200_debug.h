@@ -57,6 +57,11 @@ moao_status moao_debug_crt64(moao_ctx* ctx, int form, int lower, long M, long N,
  * rows are) and the 128 x 256 tiles of a product per launch. */
 moao_status moao_debug_limits(moao_ctx* ctx, long long workspace_bytes, long long operand_bytes,
                               long long part_tiles);
+/* Bounds of the FP64 path's device waits, in polls (0: the defaults): those of the
+ * residue products, where a wait that runs out makes the FP64 tensor cores compute the
+ * product instead, and of the diagonal blocks' grid barrier, where the call then returns
+ * MOAO_ERR_TIMEOUT. */
+moao_status moao_debug_fp64_waits(moao_ctx* ctx, long long product_polls, int barrier_polls);
 /* Device bytes the context holds in workspaces and geometry (-1: null). */
 long long moao_debug_bytes_held(moao_ctx* ctx);
 

@@ -166,6 +166,7 @@ SIGNATURES = {
     "moao_debug_residual": (i32, [vp, i32, i64, i64, dp, i64, dp, i64, dp, i64, dp, i64]),
     "moao_debug_crt_moduli": (i32, [i32, i64]),
     "moao_debug_limits": (i32, [vp, C.c_longlong, C.c_longlong, C.c_longlong]),
+    "moao_debug_fp64_waits": (i32, [vp, C.c_longlong, i32]),
     "moao_debug_bytes_held": (C.c_longlong, [vp]),
     "moao_debug_crt64": (i32, [vp, i32, i32, i64, i64, i64, C.c_double, dp, i64, dp, i64, C.c_double,
                                dp, i64]),

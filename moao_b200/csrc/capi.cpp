@@ -628,6 +628,15 @@ moao_status moao_debug_limits(moao_ctx* c, long long workspace_bytes, long long 
   return MOAO_OK;
 }
 
+moao_status moao_debug_fp64_waits(moao_ctx* c, long long product_polls, int barrier_polls) {
+  if (!c || product_polls < 0 || barrier_polls < 0)
+    return set_error(MOAO_ERR_BAD_ARG, "debug_fp64_waits: polls >= 0");
+  std::lock_guard<std::mutex> lk(c->mu);
+  c->cf_polls = (unsigned long long)product_polls;
+  c->diag_polls = (unsigned)barrier_polls;
+  return MOAO_OK;
+}
+
 long long moao_debug_bytes_held(moao_ctx* c) {
   if (!c) return -1;
   std::lock_guard<std::mutex> lk(c->mu);

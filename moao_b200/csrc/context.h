@@ -85,6 +85,11 @@ struct moao_ctx {
   // bytes of one operand's residues held at once, tiles of a product per launch.
   size_t cf_operand_bytes = 0;
   long cf_part_tiles = 0;
+  // polls of the residue products' waits and of the diagonal blocks' barrier (0: the
+  // defaults; lowered by tests, not by moao_ctx_set_wait_limit, so that the FP64 path
+  // runs under any limit of the mixed path's)
+  unsigned long long cf_polls = 0;
+  unsigned diag_polls = 0;
   size_t workspace_limit = 0;  // bytes_held above which an allocation fails (0: none; tests)
   long mx_factored_n = -1;  // size of the factorisation held in mx_* (reuse across targets)
   // Block-constant offsets of Cmm known to the caller (moao_ctx_set_offsets):

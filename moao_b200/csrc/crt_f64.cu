@@ -513,6 +513,7 @@ moao_status crt64_product(moao_ctx* ctx, const CrtOperand& A, long a0, const Crt
   g.nseg = 1;
   g.lower = f.lowerC ? 1 : 0;
   g.max_ctas = max_ctas;
+  g.spin_limit = ctx->cf_polls;
   const long total = tc_tile_count(M, N, f.lowerC);
   const long part = part_tiles(ctx), parts = (total + part - 1) / part;
   if (parts > kMaxChunks) return set_error(MOAO_ERR_UNSUPPORTED, "crt64: product too large");

@@ -49,10 +49,11 @@ moao_status potrf_inv_leaf(double* A, long lda, double* Linv, long ldi, int n, l
 
 // Factor and inverse of the nb x nb diagonal block A in one cooperative launch of `ctas`
 // CTAs (nb for which diag_block_fits). W: nb^2 doubles, d_sync: one word. A barrier whose
-// wait ran out raises d_info[1].
+// wait (of `polls` polls, 0: the default, some seconds) ran out raises d_info[1].
 bool diag_block_fits(long nb);
 moao_status diag_block(double* A, long lda, double* D, long ldd, long nb, long col0, int* d_info,
-                       double* W, unsigned* d_sync, int ctas, cudaStream_t s, long long* launches);
+                       double* W, unsigned* d_sync, int ctas, unsigned polls, cudaStream_t s,
+                       long long* launches);
 
 // Elementwise helpers (column-major).
 moao_status copy_matrix(const double* src, long lds, double* dst, long ldd, long m, long n,

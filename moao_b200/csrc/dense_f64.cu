@@ -496,11 +496,11 @@ static_assert(TileD::NTHREADS == LEAF_THREADS && TileD64::NTHREADS == LEAF_THREA
 constexpr size_t kDiagSmem =
     TileD64::SMEM_BYTES > LEAF_SMEM_BYTES ? TileD64::SMEM_BYTES : LEAF_SMEM_BYTES;
 static_assert(TileD::SMEM_BYTES <= kDiagSmem, "one size for all");
-constexpr unsigned kDiagPolls = 1u << 22;  // some seconds
+constexpr unsigned kDiagPolls = 1u << 22;  // default of the barrier's wait: some seconds
 
 // All CTAs of the grid have arrived, count of them since the launch; false when the
 // wait ran out (then *err is raised and the kernel leaves).
-__device__ __forceinline__ bool diag_barrier(unsigned* arrived, unsigned count, int* err) {
+__device__ __forceinline__ bool diag_barrier(unsigned* arrived, unsigned count, unsigned limit, int* err) {
   __syncthreads();
   int ok = 1;
   if (threadIdx.x == 0) {
@@ -509,7 +509,7 @@ __device__ __forceinline__ bool diag_barrier(unsigned* arrived, unsigned count, 
     unsigned v, polls = 0;
     do {
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(arrived) : "memory");
-    } while (v < count && ++polls < kDiagPolls);
+    } while (v < count && ++polls < limit);
     ok = v >= count;
     if (!ok) atomicExch(err, 1);
     __threadfence();
@@ -548,7 +548,7 @@ __device__ __forceinline__ void diag_product(const KParams& p, double* smem, int
 template <int VEC>
 __global__ void __launch_bounds__(LEAF_THREADS, 1)
     diag_block_kernel(const __grid_constant__ DiagPlan plan, double* A, long lda, double* D, long ldd,
-                      double* W, long col0, int* info, unsigned* arrived) {
+                      double* W, long col0, int* info, unsigned* arrived, unsigned limit) {
   extern __shared__ __align__(16) double diag_smem[];
   double* sm = diag_smem;
   const int ctas = gridDim.x;
@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(LEAF_THREADS, 1)
         diag_product<false, false, VEC>(p, sm, blockIdx.x, ctas);
       }
     }
-    if (k + 1 < plan.n && !diag_barrier(arrived, (unsigned)ctas * (k + 1), info + 1)) return;
+    if (k + 1 < plan.n && !diag_barrier(arrived, (unsigned)ctas * (k + 1), limit, info + 1)) return;
   }
 }
 
@@ -714,7 +714,8 @@ moao_status potrf_inv_leaf(double* A, long lda, double* Linv, long ldi, int n, l
 bool diag_block_fits(long nb) { return nb > LEAF && nb <= kDiagMax; }
 
 moao_status diag_block(double* A, long lda, double* D, long ldd, long nb, long col0, int* d_info,
-                       double* W, unsigned* d_sync, int ctas, cudaStream_t s, long long* launches) {
+                       double* W, unsigned* d_sync, int ctas, unsigned polls, cudaStream_t s,
+                       long long* launches) {
   if (!diag_block_fits(nb)) return set_error(MOAO_ERR_BAD_ARG, "diag_block: size");
   DiagPlan plan;
   plan.build(0, (int)nb, 0);
@@ -734,7 +735,7 @@ moao_status diag_block(double* A, long lda, double* D, long ldd, long nb, long c
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   MOAO_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, (const DiagPlan&)plan, A, lda, D, ldd, W, col0, d_info,
-                                   d_sync));
+                                   d_sync, polls ? polls : kDiagPolls));
   if (launches) ++*launches;
   return MOAO_OK;
 }

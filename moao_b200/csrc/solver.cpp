@@ -113,8 +113,8 @@ moao_status potrf_inv_block(moao_ctx* ctx, double* A, long lda, double* D, long 
     MOAO_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, ctx->device));
     const int ctas = std::min(nsm, std::max(1, ctx->diag_ctas));
     KernelTimer kt(ctx, "diag_block", (double)nb * nb * nb * (2.0 / 3));
-    return diag_block(A, lda, D, ldd, nb, col0, d_info, W, ctx->ws_sync.as<unsigned>(), ctas, ctx->stream,
-                      &ctx->launches);
+    return diag_block(A, lda, D, ldd, nb, col0, d_info, W, ctx->ws_sync.as<unsigned>(), ctas,
+                      ctx->diag_polls, ctx->stream, &ctx->launches);
   }
   if (nb <= kLeaf) {
     KernelTimer kt(ctx, "potrf_leaf", (double)nb * nb * nb * (1.0 / 3 + 1.0 / 3));

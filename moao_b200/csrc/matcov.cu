@@ -132,7 +132,7 @@ __device__ __forceinline__ double dphi_unit_s_inl(double s) {
 
 __device__ __noinline__ double dphi_unit_s(double s) { return dphi_unit_s_inl(s); }
 
-// The same function of v = s / Xlim^2 from the table: kDphiSub intervals per octave
+// The same function from the table, of v = s / Xlim^2: kDphiSub intervals per octave
 // from v's leading bits (the two forms of f meet at v = 1, an interval's edge), then
 // a polynomial of degree 8 in the distance y from the interval's middle, against ~40
 // FP64 operations of the series and ~55 of the asymptotic form with exp. The
@@ -148,6 +148,13 @@ __device__ __noinline__ double dphi_unit_s(double s) { return dphi_unit_s_inl(s)
 // of its own, so that lanes on different rows never conflict: 14 wavefronts a warp.
 // One copy (degree 5, 64 intervals per octave, 48 bytes a value) took 21 in conflicts
 // and 7.2 against 5.5 ms for the Ctm of nmeas 15,936; in L1 7.4 ms.
+//
+// The two forms differ by 5e-7 of f where they meet, at separations of 0.75 L0, which a
+// grid can hold exactly. So s is summed as for the direct form, and scaled by the neighbour of
+// 1 / Xlim^2 that puts s = Xlim^2 below 1 and the next double not.
+constexpr double kPerXlim2 = 0x1.70e6301e60654p-5;
+static_assert(kXlim2 * kPerXlim2 < 1.0 && kXlim2 * (1.0 + 0x1p-52) * kPerXlim2 >= 1.0,
+              "v >= 1 where s > Xlim^2");
 constexpr int kTab01 = 0, kTab23 = kTab01 + kDphiRows * 8 * 16, kTabF = kTab23 + kDphiRows * 8 * 16,
               kTab4 = kTabF + kDphiRows * 8 * 16, kTabBytes = kTab4 + kDphiRows * 16 * 8;
 
@@ -172,12 +179,13 @@ __device__ __forceinline__ void dphi_fill(char* tab, const DphiRow* __restrict__
   }
 }
 
-__device__ __noinline__ double dphi_outside(double v) { return dphi_unit_s_inl(v * kXlim2); }
+__device__ __noinline__ double dphi_outside(double s) { return dphi_unit_s_inl(s); }
 
-__device__ __forceinline__ double dphi_v(const char* tab, double v) {
+__device__ __forceinline__ double dphi_v(const char* tab, double s) {
+  const double v = s * kPerXlim2;
   const int hi = __double2hiint(v), lane = threadIdx.x & 31;
   const unsigned k = (unsigned)((hi >> 16) - ((1023 + kDphiLo) << 4));
-  if (k >= (unsigned)kDphiRows) return dphi_outside(v);
+  if (k >= (unsigned)kDphiRows) return dphi_outside(s);
   const double y = v - __hiloint2double((hi & 0xffff0000) | 0x8000, 0);
   const char* t = tab + (k * 8 + (lane & 7)) * 16;
   const float4 f = *reinterpret_cast<const float4*>(t + kTabF);
@@ -195,10 +203,11 @@ __device__ __forceinline__ double dphi_v(const char* tab, double v) {
 
 // The same from the rows in global memory (the per-pair and table kernels; not
 // inlined, so that their 9 or 16 points per layer share one body).
-__device__ __noinline__ double dphi_row(const DphiRow* __restrict__ rows, double v) {
+__device__ __noinline__ double dphi_row(const DphiRow* __restrict__ rows, double s) {
+  const double v = s * kPerXlim2;
   const int hi = __double2hiint(v);
   const unsigned k = (unsigned)((hi >> 16) - ((1023 + kDphiLo) << 4));
-  if (k >= (unsigned)kDphiRows) return dphi_outside(v);
+  if (k >= (unsigned)kDphiRows) return dphi_outside(s);
   const double y = v - __hiloint2double((hi & 0xffff0000) | 0x8000, 0);
   const DphiRow& r = rows[k];
   const float yf = (float)y;
@@ -299,7 +308,7 @@ __global__ void __launch_bounds__(kTileI* kTileJ)
     const double du = __ldg(ul + pi) - __ldg(ul + pj);
     const double dv = __ldg(vl + pi) - __ldg(vl + pj);
     const double s1 = sml * 0.5, s2 = snl * 0.5;
-    const double t2 = s_tpl[l] * s_tpl[l] * (1.0 / kXlim2);
+    const double t2 = s_tpl[l] * s_tpl[l];
     const double w = s_w[l] * s_amp[l];
     auto D = [&](double x, double y) { return dphi_row(g.dphi, t2 * (x * x + y * y)); };
     if (s1 == s2) {
@@ -432,10 +441,10 @@ __device__ __forceinline__ double grid_centre(const DevGeometry& g, int c, doubl
 
 // Accumulates the 8 x 4 covariances of a lane over one layer. S: kEV x kEU shared
 // values (UNIFORM), or u_sep[5] of the lane and its v coordinate against the edges
-// ve[v] (v_sep = t2 (vc - ve[v])^2).
+// ve[v] - en (v_sep = t2 (vc - (ve[v] - en))^2).
 template <bool UNIFORM>
 __device__ __forceinline__ void edge_layer(const char* tab, const double* S, double c0,
-                                           const double (&u_sep)[kEU], double vc, const double* ve,
+                                           const double (&u_sep)[kEU], double vc, const double* ve, double en,
                                            double t2, double w, double (&acc)[kEB][kEA]) {
   double prev[kEU];
 #pragma unroll
@@ -443,7 +452,7 @@ __device__ __forceinline__ void edge_layer(const char* tab, const double* S, dou
     double cur[kEU];
     double b = c0;
     if (!UNIFORM) {
-      const double d = vc - ve[v];
+      const double d = vc - (ve[v] - en);
       b = t2 * (d * d);
     }
 #pragma unroll
@@ -521,7 +530,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
     if (!(sml > 0 && snl > 0)) continue;
     const double h = g.layer[3 * nL + g.nW * nL + l];
     const double tpl = g.layer[l];
-    const double t2 = tpl * tpl * (1.0 / kXlim2);
+    const double t2 = tpl * tpl;
     const double w = 0.5 * kk * g.layer[2 * nL + l] * g.layer[nL + l];
     __syncwarp();
     if (lane < kECoord) {
@@ -546,7 +555,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
       }
       const double dc = bm[fi] - bn[fj];
       __syncwarp();
-      edge_layer<true>(tab, S, t2 * (dc * dc), u_sep, 0.0, nullptr, t2, w, acc);
+      edge_layer<true>(tab, S, t2 * (dc * dc), u_sep, 0.0, nullptr, 0.0, t2, w, acc);
     } else {
       const double *am = kind == 2 ? xm : ym, *an = kind == 2 ? xn : yn;  // u edges - centre
       const double *bm = kind == 2 ? ym : xm, *bn = kind == 2 ? yn : xn;  // centre - v edges
@@ -555,7 +564,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
         const double dv = (am[u] - em) - an[fj];
         u_sep[u] = t2 * (dv * dv);
       }
-      edge_layer<false>(tab, nullptr, 0.0, u_sep, bm[fi] + en, bn, t2, w, acc);
+      edge_layer<false>(tab, nullptr, 0.0, u_sep, bm[fi], bn, en, t2, w, acc);
     }
   }
   // through shared memory in two halves (v < 4, v >= 4), so that neighbouring lanes
@@ -651,7 +660,7 @@ __global__ void __launch_bounds__(kTileI* kTileJ)
   const double dv = g.Y[base + i] - g.Y[base + j];
   const double s = ssp * 0.5, ad = 2.0 * s;
   for (int l = 0; l < nL && tab < 0; ++l) {
-    const double t2 = s_tpl[l] * s_tpl[l] * (1.0 / kXlim2), w = s_w[l];
+    const double t2 = s_tpl[l] * s_tpl[l], w = s_w[l];
     auto D = [&](double x, double y) { return dphi_row(g.dphi, t2 * (x * x + y * y)); };
     const double d0 = (mask & 9u) ? D(du, dv) : 0.0;
     if (mask & 1u) cxx += (-d0 + D(du + ad, dv) + D(du - ad, dv) - d0) * w;
@@ -709,7 +718,7 @@ __global__ void toeplitz_table_kernel(const DevGeometry g, const int2* __restric
       const double du = (bx + (g.XPup[m] - g.XPup[n])) * rr + (g.alphaX[m] - g.alphaX[n]) * h;
       const double dv = (by + (g.YPup[m] - g.YPup[n])) * rr + (g.alphaY[m] - g.alphaY[n]) * h;
       const double s = sml * 0.5, ad = s + s;
-      const double t2 = g.layer[l] * g.layer[l] * (1.0 / kXlim2);
+      const double t2 = g.layer[l] * g.layer[l];
       auto D = [&](double x, double y) { return dphi_row(g.dphi, t2 * (x * x + y * y)); };
       const double w = 0.5 * kk * g.layer[2 * nL + l] * g.layer[nL + l];
       const double d0 = D(du, dv);

@@ -162,6 +162,7 @@ moao_status device_geometry(moao_ctx* ctx, const moao_tomo* tp, const DevGeometr
   const double k1 = 0.1716613621245709486;
   for (int l = 0; l < nL; ++l) {
     const double L0 = t.L0diff[l];
+    g.outer = std::max(g.outer, L0);
     h[olay + l] = 2 * pi / L0;                         // rodconan :107
     h[olay + nL + l] = k1 * std::pow(L0, 5. / 3.0);    // rodconan :114
     h[olay + 2 * nL + l] = t.atm.cn2[l];

@@ -33,23 +33,18 @@ namespace moao {
 namespace {
 
 // Constants of the reference model (common/moao_defs.h:15-38).
-__constant__ double c_Ga[11] = {0,
-                                12.067619015983075,
-                                5.17183672113560444,
-                                0.795667187867016068,
-                                0.0628158306210802181,
-                                0.00301515986981185091,
-                                9.72632216068338833e-05,
-                                2.25320204494595251e-06,
-                                3.93000356676612095e-08,
-                                5.34694362825451923e-10,
-                                5.83302941264329804e-12};
-__constant__ double c_Gma[11] = {-3.74878707653729304,   -2.04479295083852408,
-                                 -0.360845814853857083,  -0.0313778969438136685,
-                                 -0.001622994669507603,  -5.56455315259749673e-05,
-                                 -1.35720808599938951e-06, -2.47515152461894642e-08,
-                                 -3.50257291219662472e-10, -3.95770950530691961e-12,
-                                 -3.65327031259100284e-14};
+struct Series {
+  double c[11];
+};
+constexpr Series kGa = {{0, 12.067619015983075, 5.17183672113560444, 0.795667187867016068,
+                         0.0628158306210802181, 0.00301515986981185091, 9.72632216068338833e-05,
+                         2.25320204494595251e-06, 3.93000356676612095e-08, 5.34694362825451923e-10,
+                         5.83302941264329804e-12}};
+constexpr Series kGma = {{-3.74878707653729304, -2.04479295083852408, -0.360845814853857083,
+                          -0.0313778969438136685, -0.001622994669507603, -5.56455315259749673e-05,
+                          -1.35720808599938951e-06, -2.47515152461894642e-08, -3.50257291219662472e-10,
+                          -3.95770950530691961e-12, -3.65327031259100284e-14}};
+__constant__ Series c_Ga = kGa, c_Gma = kGma;
 constexpr double kPi = 3.1415926535897932384626433;
 constexpr double kK1 = 0.1716613621245709486;
 constexpr double kK2 = 1.00563491799858928388289314170833;
@@ -69,124 +64,144 @@ __device__ __forceinline__ double dphi_unit(double x) {
   const double c = cbrt(x);
   const double x2a = x * c * c;  // x^(5/3)
   const double z = 0.25 * x * x;  // (x/2)^2
-  double pg = c_Gma[10];
+  double pg = c_Gma.c[10];
 #pragma unroll
-  for (int n = 9; n >= 0; --n) pg = fma(pg, z, c_Gma[n]);
-  double pa = c_Ga[10];
+  for (int n = 9; n >= 0; --n) pg = fma(pg, z, c_Gma.c[n]);
+  double pa = c_Ga.c[10];
 #pragma unroll
-  for (int n = 9; n >= 1; --n) pa = fma(pa, z, c_Ga[n]);
+  for (int n = 9; n >= 1; --n) pa = fma(pa, z, c_Ga.c[n]);
   return -0.5 * (x2a * pg + z * pa);
 }
 
-// The same function of s = x^2, without the square root and cube root:
-// y = s^(-1/6) = x^(-1/3) by Newton's iteration for y^-6 = s,
-//   y <- y (7 - s y^6) / 6        (quadratic convergence, no division),
-// started from a single-precision seed 2^(-log2(s) / 6) (relative error
-// ~1e-6, so two steps reach double precision). Then x^(5/3) = s y, x = s y^3,
-// 1/x = y^3 and x^(1/3) = x y^2. Below s = 1e-30 (a float seed would lose
-// range) the direct form is used. The per-pair kernels call the non-inlined
-// copy below: their 9 or 16 stencil points per layer then share one body,
-// which keeps them inside the instruction cache (inlined, they stalled on
-// instruction fetch; ~8% slower). The shared-point kernel inlines it at its
-// four call sites (two evaluations per loop iteration, two loops).
-// The two uncommon branches are separate functions, so that the series path,
-// the one most points take, issues none of their instructions (inlined, the
-// compiler predicates them into every evaluation).
-__device__ __noinline__ double dphi_tiny_s(double s) { return s > 0 ? dphi_unit(sqrt(s)) : 0.0; }
-__device__ __noinline__ double dphi_asym_y(double s, double y) {
-  const double xi = y * y * y;  // 1/x
-  const double x = s * xi;
-  return kK2 - kK3 * exp(-x) * (x * y * y) * (1.0 + xi * (kA1 + xi * (kA2 + xi * kA3)));
+// From here on f is taken of v = x^2 / Xlim^2, without square roots and cube roots. The
+// two forms differ by 5e-7 of f where they meet, at separations of 0.75 L0, which a grid
+// can hold exactly. So s = x^2 is summed as for the direct form, and scaled by the
+// neighbour of 1 / Xlim^2 that puts s = Xlim^2 below 1 and the next double not.
+constexpr double kXlim2 = kXlim * kXlim, kPerXlim2 = 0x1.70e6301e60654p-5;
+static_assert(kXlim2 * kPerXlim2 < 1.0 && kXlim2 * (1.0 + 0x1p-52) * kPerXlim2 >= 1.0,
+              "v >= 1 where s > Xlim^2");
+
+// Values outside the other forms: 0, below kDphiTiny (whose float seeds would lose range),
+// not finite.
+__device__ __noinline__ double dphi_rare(double v) {
+  const double s = v * kXlim2;
+  return s > 0 ? dphi_unit(sqrt(s)) : 0.0;
 }
 
-// The branch is taken on s = x^2 against xlim^2, so the series path never forms
-// x (points within an ulp of the boundary may take either form, as they may in
-// the reference's own rounding of x).
-constexpr double kXlim2 = kXlim * kXlim;
-
-__device__ __forceinline__ double dphi_unit_s_inl(double s) {
-  if (!(s > 1e-30)) return dphi_tiny_s(s);
-  // seed 2^(-log2(s)/6) from the PTX approximations (flush-to-zero forms: s is
-  // a normal float here, and so is the seed), then y <- y (7/6 - (s/6) y^6)
-  float l2, y0;
-  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l2) : "f"((float)s));
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(l2 * (-1.0f / 6.0f)));
-  double y = (double)y0;
-  const double s6 = s * (1.0 / 6.0);
-#pragma unroll
-  for (int it = 0; it < 2; ++it) {
-    const double y2 = y * y;
-    y = y * fma(-s6, y2 * y2 * y2, 7.0 / 6.0);
+// The series of small x, with the constants of z = (x/2)^2 = Xlim^2 v / 4 and x^(5/3)
+// folded into the coefficients: f = v (y G(v) + A(v)), y = v^(-1/6), N terms of each. y
+// comes from a seed 2^(-log2(v)/6) by the PTX approximations (flush-to-zero forms: v is a
+// normal float here, and so is the seed; good to 2e-6) and one step of fourth order,
+// r = 1 - v y^6, (1 - r)^(-1/6) = 1 + r/6 + 7 r^2/72 + 91 r^3/1296 + O(r^4). 9 + 2 N
+// FP64 operations; within 3.7e-16 of f for v < 2^-12 with N = 5 and 6.4e-16 for v < 2^-6
+// with N = 9 (sampled against 50 digits; all 11 terms with Newton's iteration, which it
+// takes the place of, 6.7e-16 and 1.1e-15).
+constexpr double kDphiTiny = 1e-31;
+constexpr double kZ = 0.25 * kXlim2, kXlim53 = 13.245505975797633;  // kXlim^(5/3)
+constexpr int kSeriesTerms = 9;
+struct FoldedSeries {
+  double G[kSeriesTerms], A[kSeriesTerms];
+};
+constexpr FoldedSeries folded_series() {
+  FoldedSeries f{};
+  double z = 1.0;
+  for (int n = 0; n < kSeriesTerms; ++n, z *= kZ) {
+    f.G[n] = -0.5 * kXlim53 * z * kGma.c[n];
+    f.A[n] = -0.5 * z * kZ * kGa.c[n + 1];
   }
-  if (s > kXlim2) return dphi_asym_y(s, y);
-  const double x53 = s * y;        // x^(5/3)
-  const double z = 0.25 * s;       // (x/2)^2
-  double pg = c_Gma[10];
-#pragma unroll
-  for (int n = 9; n >= 0; --n) pg = fma(pg, z, c_Gma[n]);
-  double pa = c_Ga[10];
-#pragma unroll
-  for (int n = 9; n >= 1; --n) pa = fma(pa, z, c_Ga[n]);
-  return -0.5 * (x53 * pg + z * pa);
+  return f;
 }
+template <int N>
+__device__ __forceinline__ double dphi_series(double v) {
+  constexpr FoldedSeries f = folded_series();
+  float l2, seed;
+  asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l2) : "f"((float)v));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(seed) : "f"(l2 * (-1.0f / 6.0f)));
+  const double y0 = (double)seed, y2 = y0 * y0;
+  const double r = fma(-v, y2 * y2 * y2, 1.0);
+  const double p = y0 * (r * fma(fma(91.0 / 1296, r, 7.0 / 72), r, 1.0 / 6));  // y = y0 + p
+  double g = f.G[N - 1];
+#pragma unroll
+  for (int n = N - 2; n >= 0; --n) g = fma(g, v, f.G[n]);
+  double a = f.A[N - 1];
+#pragma unroll
+  for (int n = N - 2; n >= 0; --n) a = fma(a, v, f.A[n]);
+  return v * fma(y0, g, fma(p, g, a));
+}
+// Below the table, kDphiTiny < v < 2^kDphiLo.
+__device__ __forceinline__ double dphi_low(double v) { return dphi_series<5>(v); }
 
-__device__ __noinline__ double dphi_unit_s(double s) { return dphi_unit_s_inl(s); }
-
-// The same function from the table, of v = s / Xlim^2: kDphiSub intervals per octave
+// f from the table: kDphiSub intervals per octave
 // from v's leading bits (the two forms of f meet at v = 1, an interval's edge), then
 // a polynomial of degree 8 in the distance y from the interval's middle, against ~40
 // FP64 operations of the series and ~55 of the asymptotic form with exp. The
 // polynomials interpolate f, evaluated in 80-bit arithmetic, at Chebyshev nodes: an
 // interval's half width is at most v / 32 and f's nearest singularity is v = 0, so the
-// truncation is below 92^-9 of f. The terms y^5 and up are at most 3e-10 of f, so
-// their FP32 coefficients and evaluation are good to 2e-17 of it. Outside the table
-// (separations of a few centimetres, or where f is within 2e-16 of its limit) the
-// direct form.
+// truncation is at most 3.1e-18 of f. The terms y^5 and up are at most 1.7e-9 of f, so
+// their FP32 coefficients and evaluation cost at most 7.3e-17 of it; a whole
+// evaluation is within 2.1e-16 of f. Below the table (separations under 0.0117 L0) the
+// series; above it f is constant in 64 bits.
 //
 // What bounds it is shared-memory reads: 56 bytes a value. The table is held in
 // copies, one per lane of a load's phase (8 lanes of 16 bytes, 16 of 8), each in banks
 // of its own, so that lanes on different rows never conflict: 14 wavefronts a warp.
 // One copy (degree 5, 64 intervals per octave, 48 bytes a value) took 21 in conflicts
 // and 7.2 against 5.5 ms for the Ctm of nmeas 15,936; in L1 7.4 ms.
-//
-// The two forms differ by 5e-7 of f where they meet, at separations of 0.75 L0, which a
-// grid can hold exactly. So s is summed as for the direct form, and scaled by the neighbour of
-// 1 / Xlim^2 that puts s = Xlim^2 below 1 and the next double not.
-constexpr double kPerXlim2 = 0x1.70e6301e60654p-5;
-static_assert(kXlim2 * kPerXlim2 < 1.0 && kXlim2 * (1.0 + 0x1p-52) * kPerXlim2 >= 1.0,
-              "v >= 1 where s > Xlim^2");
 constexpr int kTab01 = 0, kTab23 = kTab01 + kDphiRows * 8 * 16, kTabF = kTab23 + kDphiRows * 8 * 16,
               kTab4 = kTabF + kDphiRows * 8 * 16, kTabBytes = kTab4 + kDphiRows * 16 * 8;
 
+__device__ __forceinline__ void dphi_put(char* tab, const DphiRow& r, int q) {  // copy q % 16 of row q / 16
+  const int k = q >> 4, p = q & 15;
+  reinterpret_cast<double*>(tab + kTab4)[q] = r.c[4];
+  if (p < 8) {
+    reinterpret_cast<double2*>(tab + kTab01)[k * 8 + p] = make_double2(r.c[0], r.c[1]);
+    reinterpret_cast<double2*>(tab + kTab23)[k * 8 + p] = make_double2(r.c[2], r.c[3]);
+  } else {
+    reinterpret_cast<float4*>(tab + kTabF)[k * 8 + p - 8] = make_float4(r.f[0], r.f[1], r.f[2], r.f[3]);
+  }
+}
+
 template <int THREADS>
 __device__ __forceinline__ void dphi_fill(char* tab, const DphiRow* __restrict__ rows) {
-  constexpr int PER = kDphiRows * 16 / THREADS;
-  static_assert(PER * THREADS == kDphiRows * 16, "copies per thread");
+  constexpr int PER = kDphiRows * 16 / THREADS, REST = kDphiRows * 16 % THREADS;
   DphiRow r[PER];  // every row's loads in flight together
 #pragma unroll
   for (int u = 0; u < PER; ++u) r[u] = rows[(threadIdx.x + u * THREADS) >> 4];
 #pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int q = threadIdx.x + u * THREADS, k = q >> 4, p = q & 15;
-    reinterpret_cast<double*>(tab + kTab4)[q] = r[u].c[4];
-    if (p < 8) {
-      reinterpret_cast<double2*>(tab + kTab01)[k * 8 + p] = make_double2(r[u].c[0], r[u].c[1]);
-      reinterpret_cast<double2*>(tab + kTab23)[k * 8 + p] = make_double2(r[u].c[2], r[u].c[3]);
-    } else {
-      reinterpret_cast<float4*>(tab + kTabF)[k * 8 + p - 8] =
-          make_float4(r[u].f[0], r[u].f[1], r[u].f[2], r[u].f[3]);
-    }
+  for (int u = 0; u < PER; ++u) dphi_put(tab, r[u], threadIdx.x + u * THREADS);
+  if (threadIdx.x < REST) {
+    const int q = threadIdx.x + PER * THREADS;
+    dphi_put(tab, rows[q >> 4], q);
   }
 }
 
-__device__ __noinline__ double dphi_outside(double s) { return dphi_unit_s_inl(s); }
+// Interval of v, counted from the table's first; intervals from the last row's on share
+// it. Outside (unsigned) [0, kDphiInf): below the table, not finite, or negative.
+constexpr int kDphiInf = 0x7ff0 - ((1023 + kDphiLo) << 4);
+__device__ __forceinline__ int dphi_interval(double v) {
+  return (__double2hiint(v) >> 16) - ((1023 + kDphiLo) << 4);
+}
+__device__ __forceinline__ double dphi_middle(double v) {
+  return __hiloint2double((__double2hiint(v) & 0xffff0000) | 0x8000, 0);
+}
 
-__device__ __forceinline__ double dphi_v(const char* tab, double s) {
-  const double v = s * kPerXlim2;
-  const int hi = __double2hiint(v), lane = threadIdx.x & 31;
-  const unsigned k = (unsigned)((hi >> 16) - ((1023 + kDphiLo) << 4));
-  if (k >= (unsigned)kDphiRows) return dphi_outside(s);
-  const double y = v - __hiloint2double((hi & 0xffff0000) | 0x8000, 0);
+// v in an interval from 0 on, from one copy of the rows.
+__device__ __forceinline__ double dphi_one(const DphiRow* rows, double v) {
+  const DphiRow& r = rows[min(dphi_interval(v), kDphiRows - 1)];
+  const double y = v - dphi_middle(v);
+  const float yf = (float)y;
+  const float ph = fmaf(fmaf(fmaf(r.f[3], yf, r.f[2]), yf, r.f[1]), yf, r.f[0]);
+  double p = fma((double)ph, y, r.c[4]);
+  p = fma(p, y, r.c[3]);
+  p = fma(p, y, r.c[2]);
+  p = fma(p, y, r.c[1]);
+  return fma(p, y, r.c[0]);
+}
+
+// The same from the copies.
+__device__ __forceinline__ double dphi_v(const char* tab, double v) {
+  const int lane = threadIdx.x & 31, k = min(dphi_interval(v), kDphiRows - 1);
+  const double y = v - dphi_middle(v);
   const char* t = tab + (k * 8 + (lane & 7)) * 16;
   const float4 f = *reinterpret_cast<const float4*>(t + kTabF);
   const double2 c0 = *reinterpret_cast<const double2*>(t + kTab01);
@@ -201,24 +216,29 @@ __device__ __forceinline__ double dphi_v(const char* tab, double s) {
   return fma(p, y, c0.x);
 }
 
+// A value outside the table, in interval k.
+__device__ __forceinline__ double dphi_outside(double v, int k) {
+  return k < 0 && v > kDphiTiny ? dphi_low(v) : dphi_rare(v);
+}
+__device__ __noinline__ double dphi_outside_call(double v) { return dphi_outside(v, dphi_interval(v)); }
+
+// Any v, with a branch for the lanes outside the table.
+__device__ __forceinline__ double dphi_any(const char* tab, double v) {
+  if ((unsigned)dphi_interval(v) >= (unsigned)kDphiInf) return dphi_outside_call(v);
+  return dphi_v(tab, v);
+}
+
 // The same from the rows in global memory (the per-pair and table kernels; not
 // inlined, so that their 9 or 16 points per layer share one body).
 __device__ __noinline__ double dphi_row(const DphiRow* __restrict__ rows, double s) {
   const double v = s * kPerXlim2;
-  const int hi = __double2hiint(v);
-  const unsigned k = (unsigned)((hi >> 16) - ((1023 + kDphiLo) << 4));
-  if (k >= (unsigned)kDphiRows) return dphi_outside(s);
-  const double y = v - __hiloint2double((hi & 0xffff0000) | 0x8000, 0);
-  const DphiRow& r = rows[k];
-  const float yf = (float)y;
-  const float ph = fmaf(fmaf(fmaf(r.f[3], yf, r.f[2]), yf, r.f[1]), yf, r.f[0]);
-  double p = fma((double)ph, y, r.c[4]);
-  p = fma(p, y, r.c[3]);
-  p = fma(p, y, r.c[2]);
-  p = fma(p, y, r.c[1]);
-  return fma(p, y, r.c[0]);
+  const int k = dphi_interval(v);
+  if ((unsigned)k >= (unsigned)kDphiInf) return dphi_outside(v, k);
+  return dphi_one(rows, v);
 }
 
+constexpr double kDphiReach = 0.75 / 64;  // separation at the table's lower end, in outer scales
+static_assert(kDphiLo == -12, "2^-6 of Xlim / 2 pi");
 constexpr int kMaxJobs = 160;
 constexpr int kTileI = 32;
 constexpr int kTileJ = 8;
@@ -439,25 +459,69 @@ __device__ __forceinline__ double grid_centre(const DevGeometry& g, int c, doubl
   return (x + pup) * rr + shift;
 }
 
+// The values of one step of the walk below in a system where many lie below the table:
+// all five in flight, by the form that covers every lane of the warp. Called by whole
+// warps. (One call a value by the lanes below the table took 1.46 times as long at
+// L0 = 10 km as at 25 m, 29 x 29; the direct form in FP64 that was there before the
+// table, 0.79 times.)
+struct EdgeRow {
+  double v[kEU];
+};
+__device__ __noinline__ EdgeRow edge_low(const char* tab, EdgeRow r) {
+  int least = dphi_interval(r.v[0]), most = least;
+#pragma unroll
+  for (int u = 1; u < kEU; ++u) {
+    least = min(least, dphi_interval(r.v[u]));
+    most = max(most, dphi_interval(r.v[u]));
+  }
+  EdgeRow o;
+  if (!__any_sync(0xffffffffu, least < 0 || most >= kDphiInf)) {
+#pragma unroll
+    for (int u = 0; u < kEU; ++u) o.v[u] = dphi_v(tab, r.v[u]);
+    return o;
+  }
+  if (!__any_sync(0xffffffffu, most >= 0)) {
+#pragma unroll
+    for (int u = 0; u < kEU; ++u) o.v[u] = dphi_low(r.v[u]);
+  } else if (!__any_sync(0xffffffffu, most >= (-6 - kDphiLo) * kDphiSub)) {  // v < 2^-6
+#pragma unroll
+    for (int u = 0; u < kEU; ++u) o.v[u] = dphi_series<9>(r.v[u]);
+  } else {
+#pragma unroll
+    for (int u = 0; u < kEU; ++u) {
+      const bool low = dphi_interval(r.v[u]) < 0;
+      const double p = dphi_low(r.v[u]), q = dphi_v(tab, low ? 1.0 : r.v[u]);
+      o.v[u] = low ? p : q;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < kEU; ++u)
+    if (!(r.v[u] > kDphiTiny) || dphi_interval(r.v[u]) >= kDphiInf) o.v[u] = dphi_rare(r.v[u]);
+  return o;
+}
+
 // Accumulates the 8 x 4 covariances of a lane over one layer. S: kEV x kEU shared
 // values (UNIFORM), or u_sep[5] of the lane and its v coordinate against the edges
-// ve[v] - en (v_sep = t2 (vc - (ve[v] - en))^2).
-template <bool UNIFORM>
+// ve[v] - en (v_sep = t2 (vc - (ve[v] - en))^2). LOW: many values lie below the table.
+template <bool UNIFORM, bool LOW, int NV>
 __device__ __forceinline__ void edge_layer(const char* tab, const double* S, double c0,
                                            const double (&u_sep)[kEU], double vc, const double* ve, double en,
-                                           double t2, double w, double (&acc)[kEB][kEA]) {
+                                           double t2, double w, double (&acc)[NV][kEA]) {
   double prev[kEU];
 #pragma unroll
-  for (int v = 0; v < kEV; ++v) {
+  for (int v = 0; v <= NV; ++v) {
     double cur[kEU];
     double b = c0;
     if (!UNIFORM) {
       const double d = vc - (ve[v] - en);
       b = t2 * (d * d);
     }
+    EdgeRow r;
 #pragma unroll
-    for (int u = 0; u < kEU; ++u)
-      cur[u] = dphi_v(tab, UNIFORM ? S[v * kEU + u] + b : u_sep[u] + b);
+    for (int u = 0; u < kEU; ++u) r.v[u] = (UNIFORM ? S[v * kEU + u] + b : u_sep[u] + b) * kPerXlim2;
+    if (LOW) r = edge_low(tab, r);
+#pragma unroll
+    for (int u = 0; u < kEU; ++u) cur[u] = LOW ? r.v[u] : dphi_any(tab, r.v[u]);
     // the reference's stencil (cov_XX/YY/XY/YX, matcov_kernels.cpp:147-193): right and
     // top edges are index + 1, left and bottom edges index + 0
     if (v > 0) {
@@ -472,11 +536,13 @@ __device__ __forceinline__ void edge_layer(const char* tab, const double* S, dou
 
 // Item v: tile pair v / 4 and covariance v % 4, by one warp; wsm is the warp's shared
 // memory.
-template <typename OutT>
+template <typename OutT, bool LOW, int PARTS>
 __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry& g,
                                           OutT* __restrict__ out, const char* tab, double* wsm,
                                           int v_item) {
-  const int lane = threadIdx.x & 31, kind = v_item & 3, tile = v_item >> 2;
+  constexpr int NV = kEB / PARTS;
+  const int lane = threadIdx.x & 31, kind = v_item & 3, tile = (v_item >> 2) / PARTS;
+  const int v0 = (v_item >> 2) % PARTS * NV;  // the edges v0 .. v0 + NV
   double* o = wsm;                       // [32 j cells][i cell]
   double* co = o + kEPairs / 2;              // centres of the current layer
   double* S = co + kECoord;
@@ -513,9 +579,9 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
   for (int q = lane; q < kEPairs; q += 32) any |= wanted(q & 15, q >> 4);
   if (!__any_sync(0xffffffffu, any)) return;  // nothing of this covariance is written
 
-  double acc[kEB][kEA];
+  double acc[NV][kEA];
 #pragma unroll
-  for (int v = 0; v < kEB; ++v)
+  for (int v = 0; v < NV; ++v)
 #pragma unroll
     for (int u = 0; u < kEA; ++u) acc[v][u] = 0.0;
   // the lane's fixed i and j indices
@@ -555,7 +621,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
       }
       const double dc = bm[fi] - bn[fj];
       __syncwarp();
-      edge_layer<true>(tab, S, t2 * (dc * dc), u_sep, 0.0, nullptr, 0.0, t2, w, acc);
+      edge_layer<true, LOW, NV>(tab, S + v0 * kEU, t2 * (dc * dc), u_sep, 0.0, nullptr, 0.0, t2, w, acc);
     } else {
       const double *am = kind == 2 ? xm : ym, *an = kind == 2 ? xn : yn;  // u edges - centre
       const double *bm = kind == 2 ? ym : xm, *bn = kind == 2 ? yn : xn;  // centre - v edges
@@ -564,7 +630,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
         const double dv = (am[u] - em) - an[fj];
         u_sep[u] = t2 * (dv * dv);
       }
-      edge_layer<false>(tab, nullptr, 0.0, u_sep, bm[fi], bn, en, t2, w, acc);
+      edge_layer<false, LOW, NV>(tab, nullptr, 0.0, u_sep, bm[fi], bn + v0, en, t2, w, acc);
     }
   }
   // through shared memory in two halves (v < 4, v >= 4), so that neighbouring lanes
@@ -572,7 +638,8 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
   const long long ld = d.ld;
   const bool fixed_j = kind == 0 || kind == 3;  // j = 8 fj + v, else 8 v + fj
 #pragma unroll
-  for (int half = 0; half < 2; ++half) {
+  for (int h = 0; h < 2 / PARTS; ++h) {
+    const int half = PARTS == 2 ? v0 / NV : h;
     __syncwarp();
 #pragma unroll
     for (int v = 0; v < kEB / 2; ++v)
@@ -580,7 +647,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
       for (int u = 0; u < kEA; ++u) {
         const int i = (kind == 0 || kind == 2) ? fi * kEA + u : u * kEA + fi;  // b * 4 + a
         const int j = fixed_j ? fj * 4 + v : v * kEB + fj;
-        o[j * kEA * kEA + i] = acc[half * 4 + v][u];
+        o[j * kEA * kEA + i] = acc[h * 4 + v][u];
       }
     __syncwarp();
     for (int q = lane; q < kEPairs / 2; q += 32) {
@@ -597,7 +664,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
 // Persistent: one CTA per SM holds the table in shared memory; item v of the launch
 // goes to warp v / gridDim.x of CTA v % gridDim.x, so that a short launch spreads
 // over the SMs.
-template <typename OutT>
+template <typename OutT, bool LOW, int PARTS>
 __global__ void __launch_bounds__(kEWarps * 32, 1)
     matcov_edge_kernel(const __grid_constant__ EdgeLaunch d, const DevGeometry g,
                        OutT* __restrict__ out) {
@@ -607,8 +674,8 @@ __global__ void __launch_bounds__(kEWarps * 32, 1)
   __syncthreads();
   const int warp = threadIdx.x >> 5;
   double* wsm = reinterpret_cast<double*>(esm + kTabBytes) + warp * kEWarpDoubles;
-  for (int v = blockIdx.x + warp * gridDim.x; v < 4 * d.total_tiles; v += kEWarps * gridDim.x)
-    edge_item<OutT>(d, g, out, esm, wsm, v);
+  for (int v = blockIdx.x + warp * gridDim.x; v < 4 * PARTS * d.total_tiles; v += kEWarps * gridDim.x)
+    edge_item<OutT, LOW, PARTS>(d, g, out, esm, wsm, v);
 }
 
 // Ctt (type 4): truth-sensor auto-covariance from the unprojected positions,
@@ -839,10 +906,22 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
     }
     d.total_tiles = tiles;
     if (tiles == 0) continue;
-    static std::atomic<unsigned long long> configured{0};
-    MOAO_CUDA_TRY(set_smem_limit(matcov_edge_kernel<OutT>, (int)kESmem, configured));
-    const int ctas = std::min(148, 4 * tiles);
-    MOAO_CUDA_TRY(launch_chained(chained, matcov_edge_kernel<OutT>, dim3((unsigned)ctas),
+    static std::atomic<unsigned long long> configured[4];
+    // edge_low where an outer scale puts separations of half a subaperture and a 32nd of the
+    // pupil below the table (Cmm, ms, a branch at each value and edge_low: 39 m, 29 x 29,
+    // 10 layers, L0 = 25 m 1.62 and 1.79, 100 m 1.79 and 1.83, 300 m 1.97 and 1.79; the
+    // direct form before the table 3.03, 2.30 and 2.30). By the geometry alone, so that an
+    // element has the same bits in every window.
+    const bool low = kDphiReach * g.outer > std::max(0.5 * g.pitch, g.diam / 32);
+    // Half tiles (25 values a lane for 45) where the warps then go through fewer values: a
+    // small launch is as long as its longest chain. 8 m, 10 x 10, 3 layers: 49 -> 38 us.
+    const long warps = 148 * kEWarps;
+    const bool half = (8L * tiles + warps - 1) / warps * 25 < (4L * tiles + warps - 1) / warps * 45;
+    const auto kern = half ? (low ? matcov_edge_kernel<OutT, true, 2> : matcov_edge_kernel<OutT, false, 2>)
+                           : (low ? matcov_edge_kernel<OutT, true, 1> : matcov_edge_kernel<OutT, false, 1>);
+    MOAO_CUDA_TRY(set_smem_limit(kern, (int)kESmem, configured[2 * half + low]));
+    const int ctas = (int)std::min(148L, (half ? 8L : 4L) * tiles);
+    MOAO_CUDA_TRY(launch_chained(chained, kern, dim3((unsigned)ctas),
                                  dim3(kEWarps * 32), kESmem, s, d, g, data));
     if (launches) ++*launches;
   }
@@ -893,18 +972,6 @@ void table_pairs(const DevGeometry& g, int2* pairs, int* npairs) {
 
 const DphiRow* dphi_table() {
   static const std::vector<DphiRow> table = [] {
-    // the coefficients of c_Ga and c_Gma
-    static const double Ga[11] = {0, 12.067619015983075, 5.17183672113560444, 0.795667187867016068,
-                                  0.0628158306210802181, 0.00301515986981185091,
-                                  9.72632216068338833e-05, 2.25320204494595251e-06,
-                                  3.93000356676612095e-08, 5.34694362825451923e-10,
-                                  5.83302941264329804e-12};
-    static const double Gma[11] = {-3.74878707653729304, -2.04479295083852408,
-                                   -0.360845814853857083, -0.0313778969438136685,
-                                   -0.001622994669507603, -5.56455315259749673e-05,
-                                   -1.35720808599938951e-06, -2.47515152461894642e-08,
-                                   -3.50257291219662472e-10, -3.95770950530691961e-12,
-                                   -3.65327031259100284e-14};
     auto f = [](long double v, bool asym) {
       const long double x = std::sqrt(v) * (long double)kXlim;
       if (asym) {
@@ -913,14 +980,14 @@ const DphiRow* dphi_table() {
                                       (1.0L + xi * (kA1 + xi * (kA2 + xi * (long double)kA3)));
       }
       const long double c = std::cbrt(x), z = 0.25L * x * x;
-      long double pg = Gma[10], pa = Ga[10];
-      for (int n = 9; n >= 0; --n) pg = pg * z + Gma[n];
-      for (int n = 9; n >= 1; --n) pa = pa * z + Ga[n];
+      long double pg = kGma.c[10], pa = kGa.c[10];
+      for (int n = 9; n >= 0; --n) pg = pg * z + kGma.c[n];
+      for (int n = 9; n >= 1; --n) pa = pa * z + kGa.c[n];
       return -0.5L * (x * c * c * pg + z * pa);
     };
     constexpr int D = 8;  // degree
     std::vector<DphiRow> t(kDphiRows);
-    for (int k = 0; k < kDphiRows; ++k) {
+    for (int k = 0; k + 1 < kDphiRows; ++k) {
       const int e = kDphiLo + k / kDphiSub;
       const long double w = std::ldexp(1.0L, e) / kDphiSub;  // interval width
       const long double mid = std::ldexp(1.0L, e) + w * (k % kDphiSub) + w / 2;
@@ -944,6 +1011,7 @@ const DphiRow* dphi_table() {
         else t[k].f[i - 5] = (float)(mono[i] * scale);
       }
     }
+    t[kDphiRows - 1] = DphiRow{{kK2, 0, 0, 0, 0}, {0, 0, 0, 0}};
     return t;
   }();
   return table.data();

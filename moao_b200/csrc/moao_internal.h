@@ -69,6 +69,7 @@ struct DevGeometry {
   // [3nL, 3nL + nW*nL) sspSizeL, then h [nL]
   double* layer = nullptr;
 
+  double outer = 0;  // largest outer scale of the layers
   const struct DphiRow* dphi = nullptr;  // structure-function table (dphi_table)
 
   // Projection of each WFS onto a layer at altitude h (projectedSubap):
@@ -98,9 +99,10 @@ struct DevGeometry {
 // Piecewise polynomials of the structure function f(x) in v = x^2 / Xlim^2 (matcov.cu):
 // the host table (kDphiRows rows, computed once per process), which the caller keeps
 // in device memory.
-constexpr int kDphiLo = -12, kDphiHi = 6;  // 2^kDphiLo <= v < 2^kDphiHi
+constexpr int kDphiLo = -12, kDphiHi = 6;  // 2^kDphiLo <= v < 2^kDphiHi, and one interval more:
 constexpr int kDphiSub = 16;               // intervals per octave
-constexpr int kDphiRows = (kDphiHi - kDphiLo) * kDphiSub;
+// beyond it, from v = 68 on (the last row), f is its limit in 64 bits
+constexpr int kDphiRows = (kDphiHi - kDphiLo) * kDphiSub + 2;
 struct alignas(8) DphiRow {
   double c[5];  // of 1, y, .. y^4
   float f[4];   // of y^5 .. y^8

@@ -1,8 +1,9 @@
 """Separations of exactly 0.75 L0, where the model's structure function passes from its
 series to its asymptotic form with a jump of 5e-7: a subaperture grid whose pitch divides
 0.75 L0 holds them, and the series applies to them (x > Xlim is false). Covariances of
-the LGS/NGS pairs, the equal-projection pairs and Ctt against the oracle, to 1e-11 of the matrix maximum (the bound of test_gpu_matcov_edge.py; a
-separation on the wrong side is off by 1e-7)."""
+the LGS/NGS pairs, the equal-projection pairs and Ctt against the oracle, to 1e-11 of the
+matrix maximum (the bound of test_gpu_matcov_edge.py; a separation on the wrong side is
+off by 1e-7)."""
 import os
 
 import numpy as np

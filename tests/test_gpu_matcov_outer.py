@@ -1,0 +1,95 @@
+"""Covariances of systems whose outer scales put separations below and above the tabulated
+range of the structure function, on both sides of the rules that choose the kernel:
+whole and half tiles (small and large launches), a branch per value or a form per warp
+(outer scales below and above some 43 subapertures and 2.7 pupils).
+
+Tolerance: 1e-11 of the matrix maximum against the oracle, as in
+test_gpu_matcov_edge.py (values of f within a few units of 2^-53 on both sides, their
+range against the diagonal's (10^2)^(5/3), over at most 7 layers).
+
+An element has the same bits whatever window it is computed in: the forms are chosen by
+the geometry and by the values of a tile. And no outer scale costs much more than
+another: 1.3 times the time of 25 m (with one call for each value outside the table it
+was 1.5 to 2.0; 1.1 now)."""
+import os
+
+import numpy as np
+import pytest
+
+import moao_b200 as M
+import oracle as O
+from moao_b200 import params as P
+
+pytestmark = pytest.mark.gpu
+
+SCALES = {"none outside": [25.0, 25.0, 25.0], "above": [2.0, 5.0, 25.0], "below": [1e4, 1e5, 1e6],
+          "mixed": [25.0, 300.0, 1e3], "spread": [0.3, 60.0, 1e4]}
+
+
+def tomo(tmp_path, nssp, L0, diam=None, nlgs=2, nngs=2):
+    rng = np.random.default_rng(nssp)
+    s = P.make_sys(diam or 0.5 * nssp, 0.14, nssp, nlgs, nngs, 30.0, rng)
+    a = P.make_atm([0.0, 3000.0, 9000.0], [0.5, 0.3, 0.2], 0.13, L0)
+    P.write_system(str(tmp_path), s, a)
+    t = M.Tomo(os.path.join(tmp_path, "sys-params.txt"), os.path.join(tmp_path, "prof-1-atmos-night0.txt"))
+    t.setTarget(0)
+    return t
+
+
+def tile(ctx, t, typ, nr, nc, x0, y0):
+    import torch
+    d = torch.full((nc, nr), 7.0, dtype=torch.float64, device="cuda")
+    M.matcov_tile(d, nr, nc, x0, y0, nr, t, typ, ctx=ctx)
+    ctx.synchronize()
+    return d.T
+
+
+@pytest.mark.parametrize("scales", SCALES)
+@pytest.mark.parametrize("nssp", [6, 13, 20, 25])
+def test_against_the_oracle(tmp_path, ctx, nssp, scales):
+    t = tomo(tmp_path, nssp, SCALES[scales])
+    g = O.Geometry.from_tomo(t)
+    for typ, h, w in ((1, g.nmeas, g.nmeas), (3, g.nmeasts, g.nmeas)):
+        want = O.matcov(g, h, w, 0, 0, typ)
+        got = tile(ctx, t, typ, h, w, 0, 0).cpu().numpy().copy()
+        if typ == 1:
+            want, got = np.tril(want), np.tril(got)
+        err = np.abs(got - want).max() / np.abs(want).max()
+        assert err <= 1e-11, (typ, err)
+
+
+@pytest.mark.parametrize("scales", SCALES)
+def test_windows_have_the_same_bits(tmp_path, ctx, scales):
+    import torch
+    t = tomo(tmp_path, 21, SCALES[scales])
+    nm, nts = t.getNMeas(), t.getNMeasTS()
+    rng = np.random.default_rng(1)
+    for typ, h in ((1, nm), (3, nts), (5, nm)):
+        whole = tile(ctx, t, typ, h, nm, 0, 0)
+        for k in range(6):
+            nr, nc = int(rng.integers(1, (40, h)[k % 2] + 1)), int(rng.integers(1, (40, nm)[k // 2 % 2] + 1))
+            x0, y0 = int(rng.integers(0, h - nr + 1)), int(rng.integers(0, nm - nc + 1))
+            if typ == 5:
+                nc, y0 = nr, x0
+            part = tile(ctx, t, typ, nr, nc, x0, y0)
+            assert torch.equal(part, whole[x0:x0 + nr, y0:y0 + nc]), (typ, nr, nc, x0, y0)
+
+
+def test_no_outer_scale_is_slow(tmp_path, ctx):
+    import torch
+    ms = {}
+    for L0 in (25.0, 5.0, 300.0, 1e3, 1e5):
+        t = tomo(tmp_path, 29, [L0] * 3, diam=39.0, nlgs=3, nngs=1)
+        nm = t.getNMeas()
+        d = torch.empty((nm, nm), dtype=torch.float64, device="cuda")
+        s = torch.cuda.ExternalStream(ctx.stream)
+        best = 1e9
+        for _ in range(20):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(s)
+            M.matcov_tile(d, nm, nm, 0, 0, nm, t, 1, ctx=ctx)
+            b.record(s)
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        ms[L0] = best
+    assert max(ms.values()) <= 1.3 * ms[25.0], ms

@@ -80,6 +80,9 @@ __device__ __forceinline__ double dphi_unit(double x) {
 constexpr double kXlim2 = kXlim * kXlim, kPerXlim2 = 0x1.70e6301e60654p-5;
 static_assert(kXlim2 * kPerXlim2 < 1.0 && kXlim2 * (1.0 + 0x1p-52) * kPerXlim2 >= 1.0,
               "v >= 1 where s > Xlim^2");
+// Rounded by itself (as are the sums that give s): no kernel's compilation may fuse it with
+// what follows, so that they agree to the bit.
+__device__ __forceinline__ double dphi_scaled(double s) { return __dmul_rn(s, kPerXlim2); }
 
 // Values outside the other forms: 0, below kDphiTiny (whose float seeds would lose range),
 // not finite.
@@ -231,7 +234,7 @@ __device__ __forceinline__ double dphi_any(const char* tab, double v) {
 // The same from the rows in global memory (the per-pair and table kernels; not
 // inlined, so that their 9 or 16 points per layer share one body).
 __device__ __noinline__ double dphi_row(const DphiRow* __restrict__ rows, double s) {
-  const double v = s * kPerXlim2;
+  const double v = dphi_scaled(s);
   const int k = dphi_interval(v);
   if ((unsigned)k >= (unsigned)kDphiInf) return dphi_outside(v, k);
   return dphi_one(rows, v);
@@ -455,8 +458,9 @@ struct EdgeLaunch {
 // and unit magnification.
 __device__ __forceinline__ double grid_centre(const DevGeometry& g, int c, double pup,
                                               double rr, double shift) {
-  const double x = g.bornemin + g.pitch / 2. * (2. * c + 1.);
-  return (x + pup) * rr + shift;
+  // fused here, not by choice of a kernel's compilation: its variants agree to the bit
+  const double x = fma(g.pitch / 2., 2. * c + 1., g.bornemin);
+  return fma(x + pup, rr, shift);
 }
 
 // The values of one step of the walk below in a system where many lie below the table:
@@ -518,7 +522,7 @@ __device__ __forceinline__ void edge_layer(const char* tab, const double* S, dou
     }
     EdgeRow r;
 #pragma unroll
-    for (int u = 0; u < kEU; ++u) r.v[u] = (UNIFORM ? S[v * kEU + u] + b : u_sep[u] + b) * kPerXlim2;
+    for (int u = 0; u < kEU; ++u) r.v[u] = dphi_scaled(__dadd_rn(UNIFORM ? S[v * kEU + u] : u_sep[u], b));
     if (LOW) r = edge_low(tab, r);
 #pragma unroll
     for (int u = 0; u < kEU; ++u) cur[u] = LOW ? r.v[u] : dphi_any(tab, r.v[u]);
@@ -605,8 +609,8 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
       const bool yax = k >= ne;
       const int wf = of_m ? m : n;
       const int c = (yax ? k - ne : k) + (of_m ? (yax ? ri0 : ci0) : (yax ? rj0 : cj0));
-      co[lane] = grid_centre(g, c, yax ? g.YPup[wf] : g.XPup[wf], 1. - h * g.gsAlt[wf],
-                             (yax ? g.alphaY[wf] : g.alphaX[wf]) * h);
+      co[lane] = grid_centre(g, c, yax ? g.YPup[wf] : g.XPup[wf], fma(-h, g.gsAlt[wf], 1.),
+                             __dmul_rn(yax ? g.alphaY[wf] : g.alphaX[wf], h));
     }
     __syncwarp();
     // edge k of a WFS's tile is half a projected subaperture below centre k

@@ -75,6 +75,28 @@ def test_windows_have_the_same_bits(tmp_path, ctx, scales):
             assert torch.equal(part, whole[x0:x0 + nr, y0:y0 + nc]), (typ, nr, nc, x0, y0)
 
 
+@pytest.mark.parametrize("nssp", [17, 32])
+def test_windows_of_a_large_field_have_the_same_bits(tmp_path, ctx, nssp):
+    """Layer shifts and cone effects that round at every step: single rows, columns and
+    small windows (half tiles) against the whole matrix (whole tiles)."""
+    import torch
+    s, a = P.config_scaled(nssp, 2, 1, 3, 2)
+    P.write_system(str(tmp_path), s, a)
+    t = M.Tomo(os.path.join(tmp_path, "sys-params.txt"), os.path.join(tmp_path, "prof-1-atmos-night0.txt"))
+    t.setTarget(0)
+    nm, nts = t.getNMeas(), t.getNMeasTS()
+    rng = np.random.default_rng(nssp)
+    for typ, h, w in ((1, nm, nm), (2, nm, nts), (3, nts, nm)):
+        whole = tile(ctx, t, typ, h, w, 0, 0)
+        for k in range(40):
+            nr, nc = (1, w) if k % 2 else (h, 1)
+            if k >= 20:
+                nr, nc = int(rng.integers(1, h // 4)), int(rng.integers(1, w // 4))
+            x0, y0 = int(rng.integers(0, h - nr + 1)), int(rng.integers(0, w - nc + 1))
+            part = tile(ctx, t, typ, nr, nc, x0, y0)
+            assert torch.equal(part, whole[x0:x0 + nr, y0:y0 + nc]), (typ, nr, nc, x0, y0)
+
+
 def test_no_outer_scale_is_slow(tmp_path, ctx):
     import torch
     ms = {}

@@ -108,8 +108,11 @@ moao_status device_geometry(moao_ctx* ctx, const moao_tomo* tp, const DevGeometr
     if (cr[2 * i] >= 0 && cr[2 * i] < N && cr[2 * i + 1] >= 0 && cr[2 * i + 1] < N)
       cell[(size_t)cr[2 * i + 1] * N + cr[2 * i]] = i;
   std::vector<int> ta, tb;
-  auto tiles = [&](int T, std::vector<int>& out) {
-    for (int r0 = 0; r0 < N; r0 += T)
+  GridRows rows;
+  for (int i = 0; i < ngrid; ++i) rows.row.push_back(std::max(0, std::min(N - 1, cr[2 * i + 1])));
+  auto tiles = [&](int T, std::vector<int>& out, std::vector<int>& first) {
+    for (int r0 = 0; r0 < N; r0 += T) {
+      first.push_back((int)out.size() / 2);
       for (int c0 = 0; c0 < N; c0 += T) {
         bool any = false;
         for (int r = r0; r < std::min(N, r0 + T) && !any; ++r)
@@ -119,9 +122,11 @@ moao_status device_geometry(moao_ctx* ctx, const moao_tomo* tp, const DevGeometr
           out.push_back(r0);
         }
       }
+    }
+    first.push_back((int)out.size() / 2);
   };
-  tiles(4, ta);
-  tiles(8, tb);
+  tiles(4, ta, rows.first_a);
+  tiles(8, tb, rows.first_b);
   g.ntiles_a = (int)ta.size() / 2;
   g.ntiles_b = (int)tb.size() / 2;
   g.bornemin = bornemin;
@@ -207,6 +212,8 @@ moao_status device_geometry(moao_ctx* ctx, const moao_tomo* tp, const DevGeometr
     KernelTimer kt(ctx, "matcov_table", (double)ntab / 4);
     MOAO_TRY(build_toeplitz_tables(g, ctx->stream, &ctx->launches));
   }
+  e.rows = std::move(rows);
+  g.rows = &e.rows;
   e.g = g;
   e.version = t.version;
   *out = &e.g;

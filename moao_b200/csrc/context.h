@@ -47,6 +47,7 @@ struct GeomEntry {
   unsigned long long version = ~0ull;
   DevGeometry g;
   DevBuf buf;  // backing store of every array in g
+  GridRows rows;  // g.rows
 };
 
 }  // namespace moao

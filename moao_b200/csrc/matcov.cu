@@ -243,6 +243,7 @@ __device__ __noinline__ double dphi_row(const DphiRow* __restrict__ rows, double
 constexpr double kDphiReach = 0.75 / 64;  // separation at the table's lower end, in outer scales
 static_assert(kDphiLo == -12, "2^-6 of Xlim / 2 pi");
 constexpr int kMaxJobs = 160;
+constexpr long kMaxEdgeTiles = 1L << 27;  // tile pairs of a launch: the warps count eighths
 constexpr int kTileI = 32;
 constexpr int kTileJ = 8;
 
@@ -442,6 +443,8 @@ __constant__ unsigned char c_edge_lane[32] = {
 struct EdgeJob {
   int m, n;        // row WFS, column WFS
   int rb, cb;      // global row / column of the first slope of each WFS
+  int ta0, nta;    // the 4 x 4 tiles of the row WFS, the 8 x 8 tiles of the column WFS that
+  int tb0, ntb;    // hold subapertures of the window
   int tile_base;
 };
 
@@ -556,7 +559,7 @@ __device__ __forceinline__ void edge_item(const EdgeLaunch& d, const DevGeometry
   while (job + 1 < d.njobs && d.jobs[job + 1].tile_base <= tile) ++job;
   const EdgeJob& jb = d.jobs[job];
   const int t = tile - jb.tile_base;
-  const int ta = t % g.ntiles_a, tb = t / g.ntiles_a;
+  const int ta = jb.ta0 + t % jb.nta, tb = jb.tb0 + t / jb.nta;
   const int ci0 = g.tiles_a[2 * ta], ri0 = g.tiles_a[2 * ta + 1];
   const int cj0 = g.tiles_b[2 * tb], rj0 = g.tiles_b[2 * tb + 1];
   const int N = g.nssp_grid, m = jb.m, n = jb.n;
@@ -820,6 +823,14 @@ void subap_range(int base, int N, int w0, int w1, int* lo, int* hi) {
   *hi = h;
 }
 
+// The tiles (of T x T cells, `first` of each row of them) that hold the valid
+// subapertures [i0, i0 + n): whole rows of tiles.
+void tiles_of(const GridRows& g, const std::vector<int>& first, int T, int i0, int n, int* t0, int* nt) {
+  const auto r = std::minmax_element(g.row.begin() + i0, g.row.begin() + i0 + n);
+  *t0 = first[*r.first / T];
+  *nt = first[*r.second / T + 1] - *t0;
+}
+
 template <typename OutT>
 moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, int xoffset,
                         int yoffset, int lda, int type_mat, cudaStream_t s,
@@ -890,25 +901,29 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
         g.ntiles_a > 0 && g.ntiles_b > 0) {
       EdgeJob e{};
       e.m = jb.m; e.n = jb.n; e.rb = jb.rb; e.cb = jb.cb;
+      tiles_of(*g.rows, g.rows->first_a, kEA, jb.i0, jb.ni, &e.ta0, &e.nta);
+      tiles_of(*g.rows, g.rows->first_b, kEB, jb.j0, jb.nj, &e.tb0, &e.ntb);
       edge.push_back(e);
     } else {
       plain.push_back(jb);
     }
   }
   jobs.swap(plain);
-  const int per_job = g.ntiles_a * g.ntiles_b;
-  for (size_t base = 0; base < edge.size(); base += kMaxJobs) {
+  for (size_t base = 0; base < edge.size();) {
     EdgeLaunch d{};
     d.type = type_mat;
     d.r0 = xoffset; d.c0 = yoffset; d.nrows = nrows; d.ncols = ncols; d.ld = lda;
-    int tiles = 0;
-    for (size_t k = base; k < edge.size() && k < base + kMaxJobs; ++k) {
-      EdgeJob e = edge[k];
-      e.tile_base = tiles;
-      tiles += per_job;
+    long tiles = 0;
+    for (; base < edge.size() && d.njobs < kMaxJobs; ++base) {
+      EdgeJob e = edge[base];
+      const long more = (long)e.nta * e.ntb;
+      if (more > kMaxEdgeTiles) return set_error(MOAO_ERR_UNSUPPORTED, "matcov: window too large");
+      if (tiles + more > kMaxEdgeTiles) break;
+      e.tile_base = (int)tiles;
+      tiles += more;
       d.jobs[d.njobs++] = e;
     }
-    d.total_tiles = tiles;
+    d.total_tiles = (int)tiles;
     if (tiles == 0) continue;
     static std::atomic<unsigned long long> configured[4];
     // edge_low where an outer scale puts separations of half a subaperture and a 32nd of the
@@ -920,11 +935,11 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
     // Half tiles (25 values a lane for 45) where the warps then go through fewer values: a
     // small launch is as long as its longest chain. 8 m, 10 x 10, 3 layers: 49 -> 38 us.
     const long warps = 148 * kEWarps;
-    const bool half = (8L * tiles + warps - 1) / warps * 25 < (4L * tiles + warps - 1) / warps * 45;
+    const bool half = (8 * tiles + warps - 1) / warps * 25 < (4 * tiles + warps - 1) / warps * 45;
     const auto kern = half ? (low ? matcov_edge_kernel<OutT, true, 2> : matcov_edge_kernel<OutT, false, 2>)
                            : (low ? matcov_edge_kernel<OutT, true, 1> : matcov_edge_kernel<OutT, false, 1>);
     MOAO_CUDA_TRY(set_smem_limit(kern, (int)kESmem, configured[2 * half + low]));
-    const int ctas = (int)std::min(148L, (half ? 8L : 4L) * tiles);
+    const int ctas = (int)std::min(148L, (half ? 8 : 4) * tiles);
     MOAO_CUDA_TRY(launch_chained(chained, kern, dim3((unsigned)ctas),
                                  dim3(kEWarps * 32), kESmem, s, d, g, data));
     if (launches) ++*launches;

@@ -7,6 +7,7 @@
 #include <atomic>
 #include <cstdint>
 #include <string>
+#include <vector>
 
 #include "moao_b200.h"
 
@@ -94,6 +95,13 @@ struct DevGeometry {
   int* tiles_a = nullptr;       // 4x4-cell tiles holding a valid cell: (col0, row0) pairs
   int* tiles_b = nullptr;       // 8x8-cell tiles likewise
   int ntiles_a = 0, ntiles_b = 0;
+  const struct GridRows* rows = nullptr;  // host: where those tiles' rows begin
+};
+
+// The common grid's rows on the host: of each valid subaperture, and the first tile of
+// each row of 4 x 4 (a) and 8 x 8 (b) cell tiles, with the total behind them.
+struct GridRows {
+  std::vector<int> row, first_a, first_b;
 };
 
 // Piecewise polynomials of the structure function f(x) in v = x^2 / Xlim^2 (matcov.cu):

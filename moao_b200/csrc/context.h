@@ -168,7 +168,7 @@ struct moao_ctx {
     return {&ws_w,  &ws_dinv, &ws_info, &ws_tmp, &ws_host_t, &ws_corner, &mx_a32, &mx_lr,  &mx_lc,    &mx_t32,
             &mx_w1, &mx_w2,   &mx_x,    &mx_r64, &mx_e64, &mx_qa,  &mx_qb,    &mx_ea,
             &mx_fb, &mx_colmax, &mx_norm, &mx_rid, &mx_y, &mx_y2, &mx_zu, &mx_sinv, &mx_exps,
-            &mx_dsl, &cx_qc, &cx_ec, &ws_sync, &cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z, &cf_flag};
+            &mx_dsl, &mx_qr, &mx_qs, &mx_z, &cx_qc, &cx_ec, &ws_sync, &cf_a, &cf_b, &cf_c, &cf_ma, &cf_mb, &cf_mc, &cf_k, &cf_z, &cf_flag};
   }
   // The FP64 residue products' buffers: kept from call to call, but an allocation that
   // would fail beside them takes their room (FP64 calls run without them).

@@ -168,3 +168,22 @@ def test_server_stays_in_its_budget(built, cuda, tmp_path, prec):
                 assert (admitted > 1.2 * foot) == (k == 0)
         out.append(R)
     assert np.linalg.norm(out[0] - out[1]) <= 1e-9 * np.linalg.norm(out[1])
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_a_destroyed_context_leaves_nothing(built, cuda, prec):
+    import torch
+    n, m = 4000, 800
+    C, T, _ = system(n, m)
+    free = []
+    for _ in range(3):
+        ctx = M.Context(0)
+        rec(ctx, n, m, C, T, prec)
+        torch.cuda.synchronize()
+        kept = held(ctx)
+        before = torch.cuda.mem_get_info()[0]
+        ctx.close()
+        free.append(torch.cuda.mem_get_info()[0])
+        # everything counted as held comes back (cudaMalloc rounds each buffer up to 2 MB)
+        assert free[-1] - before >= 0.95 * kept
+    assert free[0] - free[-1] <= 32e6, free

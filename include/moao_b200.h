@@ -234,6 +234,14 @@ moao_status moao_matcov_tile_host(moao_ctx* ctx, const moao_tomo* t, double* h_d
 /* Cmm is overwritten by its lower Cholesky factor (upper triangle left       */
 /* untouched) and Ctm by R, ngal targets of nmeasts x nmeas each, stored      */
 /* nmeas*nmeasts apart.                                                      */
+/* FP64: products over 1,024 terms and more (here and in moao_cee_cvv) are    */
+/* summed exactly from operands of 53 to 57 bits of their row's largest entry */
+/* (after a scaling by the system's own variances). Their error is a few      */
+/* 2^-53 of the rows' magnitudes; unlike an FP64 sum's it is not smaller for  */
+/* an element whose own terms are all far below them. Rows with NaN,          */
+/* infinities or magnitudes beyond 2^900 either way, and calls under stream   */
+/* capture, take FP64 sums. The buffers this takes (about 6 GB at nmeas       */
+/* 29,120) stay on the context and give way to any other allocation of it.    */
 /* ------------------------------------------------------------------------ */
 typedef struct {
   int info;              /* 0, or the 1-based column of a non-positive pivot */
@@ -300,6 +308,7 @@ moao_status moao_dense_gemm(moao_ctx* ctx, int transB, int lowerC, long M, long 
 /* Error covariances.                                                        */
 /* Replaces MOAO_LAPACK::Cee_Cvv  lapack/compute/cee_cvv.cpp:50-125          */
 /*   Cee = Ctt - Ctm R^T - R Ctm^T + R Cmm R^T ;  Cvv = Dx Cee Dx^T           */
+/* FP64 products as described at moao_reconstructor.                         */
 /* Same in-place contract: Cpp (Ctt) and Cpm (Ctm) are destroyed, Tmp is     */
 /* scratch, Cmm is read as a symmetric matrix from its lower triangle.       */
 /* ------------------------------------------------------------------------ */

@@ -80,8 +80,10 @@ struct moao_ctx {
   moao::DevBuf ws_sync;  // barrier word of the diagonal blocks (diag_block)
   int diag_ctas = 96;    // its CTAs: the lookahead's SMs beside other work, not all SMs ever
                          // (a collective's kernels may hold some)
-  bool chained = true;  // chained launches of the small FP64 kernels (off under stream capture)
-  bool crt_f64 = true;  // off where nothing may be allocated (stream capture, no-alloc calls)
+  bool chained = true;  // chained launches of the small FP64 kernels (off in the batch
+                        // engine's captured sub-contexts)
+  bool crt_f64 = true;  // residue products (off there too, and in a serving request that was
+                        // admitted without their buffers)
   // Limits of the residue products that tests lower (0: the defaults in crt_f64.cu):
   // bytes of one operand's residues held at once, tiles of a product per launch.
   size_t cf_operand_bytes = 0;

@@ -16,7 +16,11 @@
 //   combine   X Y^T from its residues, scaled back and added to C (tc_modz_combine).
 // The only roundings are the operands' (elements within 2^4 of their row's
 // largest are exact at 57 bits) and the two of the reconstruction, against K
-// rounded additions per element on the FP64 tensor cores.
+// rounded additions per element on the FP64 tensor cores. The bound is one per row:
+// an element of the result is off by up to 2^(1 - bits) K times the largest entries of
+// its two rows (balanced), where FP64 sums are off by K 2^-53 times the sum of its own
+// terms' absolute values. The two differ where all large entries of a row meet entries
+// 2^-50 of their own row's largest.
 //
 // Measured (B200, against the FP64 tensor cores at 28-31 TF/s): the FP64
 // reconstructor at nmeas 29,120 563 -> 190 ms (lookahead and groups included), its Cee/Cvv chain

@@ -51,7 +51,6 @@ struct moao_isample {
   double* part = nullptr;     // parts x nmap
   int* cell_start = nullptr;  // nmap+1 (CSR over Cvv indices; a warp per cell)
   int* cell_idx = nullptr;    // nidx
-  double* inv_div = nullptr;  // nmap (1/div, or 1 when div == 0)
   double* div = nullptr;      // nmap
   double* dphi = nullptr;     // N*N real: the phase covariance
   double* map = nullptr;      // nmap
@@ -136,8 +135,6 @@ __global__ void __launch_bounds__(kMapThreads)
   for (int c = tid; c < nmap; c += kMapThreads) part[(long)blockIdx.x * nmap + c] = m[c];
 }
 
-// Row ii of the map on the lattice (row a + ii pitch, columns a + jj pitch), forward
-// along j: rows[j * ncov + ii].
 // map = the sum of the partial maps over the hit counts: 32 cells a block, eight
 // threads each.
 __global__ void __launch_bounds__(256)
@@ -260,8 +257,8 @@ __global__ void psf_kernel(const Cplx* __restrict__ spec, double* __restrict__ p
 void free_isample(moao_isample* is) {
   if (!is) return;
   fft2d_free(&is->fft);
-  void* ptrs[] = {is->abs2fi, is->otf, is->cell_start, is->cell_idx, is->inv_div,
-                  is->div, is->dphi, is->map, is->spec, is->rows, is->cell_of, is->part};
+  void* ptrs[] = {is->abs2fi, is->otf, is->cell_start, is->cell_idx, is->div,
+                  is->dphi, is->map, is->spec, is->rows, is->cell_of, is->part};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete is;

@@ -643,7 +643,8 @@ __global__ void __launch_bounds__((4 + epi_warps(MODZ)) * 32, 1)
 // P from its residues z_i (i < 16) by the fractional form of the Chinese
 // remainder theorem: with c_i = (M / m_i)^-1 mod m_i, P / M = sum z_i c_i / m_i
 // modulo 1. The weights c_i / m_i are kept to 80 bits (ten bytes), so ten sums of
-// 16 byte-by-byte products (four dp4a each) and their carries give P / M to
+// 16 byte-by-byte products (four dp4a each) and their carries give P / M (the weights
+// cut off, so from below) to
 // 2^-69, which is 2^-57 of a P of 2^114 (the size of a product of 1,024 terms
 // whose operands' rms is an eighth of their largest). Mixed-radix (Garner)
 // reconstruction takes 120 dependent steps per element instead.
@@ -680,8 +681,7 @@ constexpr FracWeights frac_weights() {
 }
 __constant__ FracWeights c_frac = frac_weights();
 
-// M as the sum of two doubles: the product of the first eight moduli is below
-// 2^64 = 2^8 times an odd 56-bit number, so it is split exactly into 32-bit parts.
+// M, a 126-bit integer, as the sum of two doubles: rounded, and the rest rounded.
 struct ModProduct {
   double hi, lo;
 };

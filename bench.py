@@ -1118,7 +1118,7 @@ def main():
                     "traffic": (ratio * s["work"] / s["launches"]) if ratio else None,
                     "launches": s["launches"], "share": share}
         if fam == "matcov":
-            # HBM framing (bytes stored); the kernel itself is bound by its FP64 pipe
+            # HBM framing (bytes stored); the kernel itself is bound by its table's shared-memory reads
             hbm = float(peaks.get("hbm_gbs", 6650.0))
             bytes_alg = 8.0 * s["work"]
             achieved = bytes_alg / (s["ms"] / 1000.0) / 1e9

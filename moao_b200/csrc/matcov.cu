@@ -827,6 +827,9 @@ void subap_range(int base, int N, int w0, int w1, int* lo, int* hi) {
 // The tiles (of T x T cells, `first` of each row of them) that hold the valid
 // subapertures [i0, i0 + n): whole rows of tiles.
 void tiles_of(const GridRows& g, const std::vector<int>& first, int T, int i0, int n, int* t0, int* nt) {
+  *t0 = 0;
+  *nt = first.back();
+  if (n == (int)g.row.size()) return;
   const auto r = std::minmax_element(g.row.begin() + i0, g.row.begin() + i0 + n);
   *t0 = first[*r.first / T];
   *nt = first[*r.second / T + 1] - *t0;
@@ -927,16 +930,18 @@ moao_status launch_impl(const DevGeometry& g, OutT* data, int nrows, int ncols, 
     d.total_tiles = (int)tiles;
     if (tiles == 0) continue;
     static std::atomic<unsigned long long> configured[4];
-    // edge_low where an outer scale puts separations of half a subaperture and a 32nd of the
-    // pupil below the table (Cmm, ms, a branch at each value and edge_low: 39 m, 29 x 29,
+    // edge_low where an outer scale puts separations of a subaperture and a 32nd of the pupil
+    // below the table (Cmm, ms, a branch at each value and edge_low: 39 m, 29 x 29,
     // 10 layers, L0 = 25 m 1.62 and 1.79, 100 m 1.79 and 1.83, 300 m 1.97 and 1.79; the
     // direct form before the table 3.03, 2.30 and 2.30). By the geometry alone, so that an
     // element has the same bits in every window.
-    const bool low = kDphiReach * g.outer > std::max(0.5 * g.pitch, g.diam / 32);
-    // Half tiles (25 values a lane for 45) where the warps then go through fewer values: a
-    // small launch is as long as its longest chain. 8 m, 10 x 10, 3 layers: 49 -> 38 us.
+    const bool low = kDphiReach * g.outer > std::max(g.pitch, g.diam / 32);
+    // Half tiles (25 values a lane for 45, and 8 % more a value) where the warps then go
+    // through fewer: a small launch is as long as its longest chain. Cmm and Ctm, us, whole
+    // and half: 8 m, 10 x 10, 3 layers 49 + 48 and 40 + 39; 39 m, 10 layers, 10 x 10
+    // 87 + 82 and 66 + 61, 20 x 20 264 + 167 and 270 + 158.
     const long warps = 148 * kEWarps;
-    const bool half = (8 * tiles + warps - 1) / warps * 25 < (4 * tiles + warps - 1) / warps * 45;
+    const bool half = (8 * tiles + warps - 1) / warps * 27 < (4 * tiles + warps - 1) / warps * 45;
     const auto kern = half ? (low ? matcov_edge_kernel<OutT, true, 2> : matcov_edge_kernel<OutT, false, 2>)
                            : (low ? matcov_edge_kernel<OutT, true, 1> : matcov_edge_kernel<OutT, false, 1>);
     MOAO_CUDA_TRY(set_smem_limit(kern, (int)kESmem, configured[2 * half + low]));

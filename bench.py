@@ -875,13 +875,13 @@ def main():
         # sizes from the reference's own Tomo_struct (oracle/_ref): nothing of
         # this repository's library is loaded on this arm
         O = _oracle()
-        if O.RefTomo.available():
-            ri = O.RefTomo(sf, af).info
-            nm, nts = ri.nmeas, ri.nmeasts
-        else:
-            import moao_b200 as M
-            t = M.Tomo(sf, af)
-            nm, nts = t.getNMeas(), t.getNMeasTS()
+        if not O.RefTomo.available():
+            print(json.dumps({"impl": "reference", "unavailable":
+                              "the reference's library (oracle/_ref) is not built: its sources are absent"}),
+                  flush=True)
+            return 0
+        ri = O.RefTomo(sf, af).info
+        nm, nts = ri.nmeas, ri.nmeasts
         vals, walls = [], []
         for i in range(args.warmup + args.steps):
             t0 = time.perf_counter()
